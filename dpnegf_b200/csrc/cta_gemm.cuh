@@ -126,67 +126,67 @@ struct Acc3M {
 NEGF_DEV int acc_row(int i, int e, int wm, int lane) { return wm + 16 * i + (lane >> 2) + ((e & 2) ? 8 : 0); }
 NEGF_DEV int acc_col(int j, int e, int wn, int lane) { return wn + 8 * j + 2 * (lane & 3) + (e & 1); }
 
-// One warp: ksteps x (k=8) slabs of its 32x16 sub-tile (2 x 2 DMMA m16n8k8
-// fragments per real plane).  Fragment reads go through the index functors
-// so the same loop serves the GEMM tiles and the Gauss-Jordan panel update.
+// One warp's operand fragments for a k = 8 step of its 32x16 sub-tile (2 x 2 DMMA m16n8k8
+// fragments per real plane), read through the index functors so the same code serves the GEMM
+// tiles and the Gauss-Jordan panel update.
 // G3 selects the complex product: Gauss/3M (three real MMAs, t1..t3) or the
 // conventional 4M form (four real MMAs into t1 = Re, t2 = Im), whose
 // componentwise error bound is tighter -- used where an iteration amplifies
 // rounding (the lead decimation).
+struct Frag8 {
+  double ar[2][4], ai[2][4], as[2][4], br[2][2], bi[2][2], bs[2][2];  // as/bs: re + im (3M) or -im (4M, as)
+};
+template <bool CONJ_A, bool CONJ_B, bool G3, class AIdx, class BIdx>
+NEGF_DEV void frag8_load(Frag8& f, const cplx* sA, const cplx* sB, int ks, int wm, int wn, int lane, AIdx aidx,
+                         BIdx bidx) {
+  const int gr = lane >> 2, k0 = ks * 8 + (lane & 3);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = wm + 16 * i + gr;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      cplx a = sA[aidx(r + ((e & 1) ? 8 : 0), k0 + ((e & 2) ? 4 : 0))];
+      f.ar[i][e] = a.x;
+      f.ai[i][e] = CONJ_A ? -a.y : a.y;
+      f.as[i][e] = G3 ? f.ar[i][e] + f.ai[i][e] : -f.ai[i][e];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int c = wn + 8 * j + gr;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      cplx b = sB[bidx(k0 + 4 * e, c)];
+      f.br[j][e] = b.x;
+      f.bi[j][e] = CONJ_B ? -b.y : b.y;
+      if (G3) f.bs[j][e] = f.br[j][e] + f.bi[j][e];
+    }
+  }
+}
+template <bool G3>
+NEGF_DEV void frag8_mma(Acc3M& acc, const Frag8& f) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      dmma1688(acc.t1[i][j], f.ar[i], f.br[j]);
+      if (G3) {
+        dmma1688(acc.t2[i][j], f.ai[i], f.bi[j]);
+        dmma1688(acc.t3[i][j], f.as[i], f.bs[j]);
+      } else {
+        dmma1688(acc.t1[i][j], f.as[i], f.bi[j]);
+        dmma1688(acc.t2[i][j], f.ar[i], f.bi[j]);
+        dmma1688(acc.t2[i][j], f.ai[i], f.br[j]);
+      }
+    }
+}
 template <bool CONJ_A, bool CONJ_B, bool G3 = true, class AIdx, class BIdx>
 NEGF_DEV void warp_mma_3m(Acc3M& acc, const cplx* sA, const cplx* sB, int ksteps, int wm, int wn, int lane,
                           AIdx aidx, BIdx bidx) {
-  const int gr = lane >> 2, gc = lane & 3;
   for (int ks = 0; ks < ksteps; ++ks) {
-    const int k0 = ks * 8 + gc;
-    double ar[2][4], ai[2][4], as[2][4], br[2][2], bi[2][2], bs[2][2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = wm + 16 * i + gr;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        cplx a = sA[aidx(r + ((e & 1) ? 8 : 0), k0 + ((e & 2) ? 4 : 0))];
-        ar[i][e] = a.x;
-        ai[i][e] = CONJ_A ? -a.y : a.y;
-        as[i][e] = ar[i][e] + ai[i][e];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int c = wn + 8 * j + gr;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        cplx b = sB[bidx(k0 + 4 * e, c)];
-        br[j][e] = b.x;
-        bi[j][e] = CONJ_B ? -b.y : b.y;
-        bs[j][e] = br[j][e] + bi[j][e];
-      }
-    }
-    if (G3) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          dmma1688(acc.t1[i][j], ar[i], br[j]);
-          dmma1688(acc.t2[i][j], ai[i], bi[j]);
-          dmma1688(acc.t3[i][j], as[i], bs[j]);
-        }
-    } else {
-      double an[2][4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) an[i][e] = -ai[i][e];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          dmma1688(acc.t1[i][j], ar[i], br[j]);
-          dmma1688(acc.t1[i][j], an[i], bi[j]);
-          dmma1688(acc.t2[i][j], ar[i], bi[j]);
-          dmma1688(acc.t2[i][j], ai[i], br[j]);
-        }
-    }
+    Frag8 f;
+    frag8_load<CONJ_A, CONJ_B, G3>(f, sA, sB, ks, wm, wn, lane, aidx, bidx);
+    frag8_mma<G3>(acc, f);
   }
 }
 
@@ -228,15 +228,26 @@ struct EpiStore {
 // is called once for every in-range element.  The output must not alias A or
 // B.  Ends with __syncthreads(), so whatever epi wrote to global memory is
 // visible to every thread of the CTA on return.  k-slabs flow through a
-// GT_STAGES-deep cp.async ring (one barrier per slab).
-// With SKIP, a warp whose 32 x 16 sub-tile lies wholly outside the product
-// skips its MMAs (ragged sizes then execute ~1.07x the useful products instead
-// of up to 16x at n = 16); off by default because the extra live predicate
-// raises register spills in the RGF sweep, which sits at the 255-register cap.
-template <int OPA, int OPB, bool G3, class Epi, bool SKIP = false>
-__device__ __noinline__ void cta_gemm_epi(const GemmArgs g, cplx* smem, const Epi epi) {
+// GT_STAGES-deep cp.async ring with one barrier per slab.  Bound by the DMMA
+// pipe; two forms with the same MMAs in the same order (bitwise equal results):
+//
+// DRIFT = false: the barrier stands at the head of the slab and every tile starts its own ring.
+// DRIFT = true: the slabs of all output tiles form one sequence, so a tile's first slabs load while
+// the tile before it finishes; the slab's barrier stands between the operand reads and the MMAs of
+// its last k = 8 step, which cover its skew and the next slab's first reads; and a warp whose
+// 32 x 16 sub-tile lies outside the product does no MMAs.  Warps w and w + 4 share a tensor core,
+// so the second row of sub-tiles is rotated by two columns: the live warps of a ragged tile then
+// spread over all four.
+// Time of one n^3 product (148 CTAs with their own operands), DRIFT = false -> true: n = 16
+// 3.3 -> 2.5 us, 32 5.4 -> 3.8, 96 53.9 -> 40.5, 115 75.1 -> 72.2, 128 74.1 -> 73.0, 256 545 -> 543
+// (73 % of the DMMA peak); 4M products at 256 666 -> 644.  Inside the 3M sweep at n = 128 and 256,
+// where registers are short, the drifting form is 2-4 % slower, so the sweep takes it for ragged
+// products only (see gemm_ragged); the 4M lead kernels take it always (3.7 % at n = 256).
+template <int OPA, int OPB, bool G3, bool DRIFT, class Epi>
+NEGF_DEV void gemm_body(const GemmArgs& g, const Epi& epi) {
+  cplx* const smem = smem_cplx();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
+  const int wm = (warp >> 2) * 32, wn = ((warp + (DRIFT ? 2 * (warp >> 2) : 0)) & 3) * 16;
   const int nk = (g.K + GT_K - 1) / GT_K;
   typedef typename std::conditional<OPA == OP_C, AIdxOpC, AIdxOp0>::type AI;
   typedef typename std::conditional<OPB == OP_C, BIdxOpC, BIdxOp0>::type BI;
@@ -244,33 +255,92 @@ __device__ __noinline__ void cta_gemm_epi(const GemmArgs g, cplx* smem, const Ep
   auto sA = [&](int s) { return smem + (2 * s) * GT_TILE; };
   auto sB = [&](int s) { return smem + (2 * s + 1) * GT_TILE; };
 
+  if constexpr (!DRIFT) {
+    for (int m0 = 0; m0 < g.M; m0 += GT_M) {
+      for (int n0 = 0; n0 < g.N; n0 += GT_N) {
+        __syncthreads();  // the previous tile's last slab is no longer being read
+#pragma unroll
+        for (int s = 0; s < GT_STAGES - 1; ++s) {
+          if (s < nk) {
+            load_a_tile<OPA>(sA(s), g, m0, s * GT_K, tid);
+            load_b_tile<OPB>(sB(s), g, s * GT_K, n0, tid);
+          }
+          cp_async_commit();
+        }
+        Acc3M acc;
+        acc.zero();
+        for (int kt = 0; kt < nk; ++kt) {
+          cp_async_wait<GT_STAGES - 2>();
+          __syncthreads();
+          const int nx = kt + GT_STAGES - 1;
+          if (nx < nk) {
+            load_a_tile<OPA>(sA(nx % GT_STAGES), g, m0, nx * GT_K, tid);
+            load_b_tile<OPB>(sB(nx % GT_STAGES), g, nx * GT_K, n0, tid);
+          }
+          cp_async_commit();
+          warp_mma_3m<CA, CB, G3>(acc, sA(kt % GT_STAGES), sB(kt % GT_STAGES), GT_K / 8, wm, wn, lane, AI(), BI());
+        }
+        acc_foreach<G3>(acc, wm, wn, lane, [&](int r, int c, cplx v) {
+          int m = m0 + r, n = n0 + c;
+          if (m < g.M && n < g.N) epi(m, n, v);
+        });
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    return;
+  }
+
+  // the next slab to load: its tile corner, k offset and ring stage
+  int lm = 0, ln = 0, lk = 0, lst = 0;
+  int left = ((g.M + GT_M - 1) / GT_M) * ((g.N + GT_N - 1) / GT_N) * nk;
+  auto load_next = [&]() {
+    if (left > 0) {
+      load_a_tile<OPA>(sA(lst), g, lm, lk, tid);
+      load_b_tile<OPB>(sB(lst), g, lk, ln, tid);
+      --left;
+      lst = lst + 1 == GT_STAGES ? 0 : lst + 1;
+      lk += GT_K;
+      if (lk >= g.K) {
+        lk = 0;
+        ln += GT_N;
+        if (ln >= g.N) { ln = 0; lm += GT_M; }
+      }
+    }
+    cp_async_commit();
+  };
+  __syncthreads();  // whatever used the ring's memory before is done with it
+#pragma unroll
+  for (int s = 0; s < GT_STAGES - 1; ++s) load_next();
+  cp_async_wait<GT_STAGES - 2>();
+  __syncthreads();
+  int st = 0;
   for (int m0 = 0; m0 < g.M; m0 += GT_M) {
     for (int n0 = 0; n0 < g.N; n0 += GT_N) {
-      __syncthreads();  // the previous tile's last slab is no longer being read
-#pragma unroll
-      for (int s = 0; s < GT_STAGES - 1; ++s) {
-        if (s < nk) {
-          load_a_tile<OPA>(sA(s), g, m0, s * GT_K, tid);
-          load_b_tile<OPB>(sB(s), g, s * GT_K, n0, tid);
+      if (m0 + wm >= g.M || n0 + wn >= g.N) {  // no output in this warp's sub-tile: keep the ring going
+        for (int k0 = 0; k0 < g.K; k0 += GT_K) {
+          load_next();
+          cp_async_wait<GT_STAGES - 2>();
+          __syncthreads();
+          st = st + 1 == GT_STAGES ? 0 : st + 1;
         }
-        cp_async_commit();
+        continue;
       }
       Acc3M acc;
       acc.zero();
-      const bool live = !SKIP || (m0 + wm < g.M && n0 + wn < g.N);
-      for (int kt = 0; kt < nk; ++kt) {
+      for (int k0 = 0; k0 < g.K; k0 += GT_K) {
+        const cplx *a = sA(st), *b = sB(st);
+        warp_mma_3m<CA, CB, G3>(acc, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
+        load_next();
+        Frag8 f;
+        frag8_load<CA, CB, G3>(f, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
         cp_async_wait<GT_STAGES - 2>();
         __syncthreads();
-        const int nx = kt + GT_STAGES - 1;
-        if (nx < nk) {
-          load_a_tile<OPA>(sA(nx % GT_STAGES), g, m0, nx * GT_K, tid);
-          load_b_tile<OPB>(sB(nx % GT_STAGES), g, nx * GT_K, n0, tid);
-        }
-        cp_async_commit();
-        if (live) warp_mma_3m<CA, CB, G3>(acc, sA(kt % GT_STAGES), sB(kt % GT_STAGES), GT_K / 8, wm, wn, lane, AI(), BI());
+        frag8_mma<G3>(acc, f);
+        st = st + 1 == GT_STAGES ? 0 : st + 1;
       }
       acc_foreach<G3>(acc, wm, wn, lane, [&](int r, int c, cplx v) {
-        int m = m0 + r, n = n0 + c;
+        const int m = m0 + r, n = n0 + c;
         if (m < g.M && n < g.N) epi(m, n, v);
       });
     }
@@ -279,10 +349,34 @@ __device__ __noinline__ void cta_gemm_epi(const GemmArgs g, cplx* smem, const Ep
   __syncthreads();
 }
 
+// Whether the drifting form is the faster one for an M x N product of the sweep: the last row or
+// column of tiles leaves at least half of its warps without output (remainder 1 .. 32 of 64).
+NEGF_DEV bool gemm_ragged(int M, int N) { return ((M - 1) & (GT_M - 1)) < GT_M / 2 || ((N - 1) & (GT_N - 1)) < GT_N / 2; }
+
+// The compiled products.  Arguments go by reference: two non-inlined functions that take the
+// argument structs by value, called from the two arms of a branch, reached one of them with a
+// wrong copy (the checkpointed adjoint then recomputed wrong blocks).
+template <int OPA, int OPB, bool G3, bool DRIFT, class Epi>
+__device__ __noinline__ void cta_gemm_epi(const GemmArgs& gr, const Epi& er) {
+  const GemmArgs g = gr;
+  const Epi epi = er;
+  gemm_body<OPA, OPB, G3, DRIFT>(g, epi);
+}
+template <int OPA, int OPB, bool G3, bool DRIFT>
+__device__ __noinline__ void cta_gemm_std(const GemmArgs& gr) {
+  const GemmArgs g = gr;
+  gemm_body<OPA, OPB, G3, DRIFT>(g, EpiStore{g});
+}
+
 // C = alpha op(A) op(B) + beta D (D may alias C; C must not alias A or B).
-template <int OPA, int OPB, bool G3 = true, bool SKIP = false>
-NEGF_DEV void cta_gemm(const GemmArgs& g, cplx* smem) {
-  cta_gemm_epi<OPA, OPB, G3, EpiStore, SKIP>(g, smem, EpiStore{g});
+template <int OPA, int OPB, bool G3 = true>
+NEGF_DEV void cta_gemm(const GemmArgs& g) {
+  if constexpr (G3) {
+    if (gemm_ragged(g.M, g.N)) cta_gemm_std<OPA, OPB, G3, true>(g);
+    else cta_gemm_std<OPA, OPB, G3, false>(g);
+  } else {
+    cta_gemm_std<OPA, OPB, G3, true>(g);
+  }
 }
 
 }  // namespace negf

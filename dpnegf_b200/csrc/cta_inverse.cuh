@@ -362,12 +362,12 @@ __device__ __noinline__ int cta_inverse_nb(cplx* W, int64_t ldw, int n, cplx* G,
       if (c_lo > 0) {
         GemmArgs g = gemm_args(n, c_lo, kb, W + c_lo, ldw, snap, n, W, ldw);
         if constexpr (TC) cta_gemm_tc_epi<OP_N, OP_N>(g, smem_raw, EpiGJ{W, ldw, pinv, c_lo, c_hi, 0});
-        else cta_gemm_epi<OP_N, OP_N, G3>(g, reinterpret_cast<cplx*>(smem_raw), EpiGJ{W, ldw, pinv, c_lo, c_hi, 0});
+        else cta_gemm_epi<OP_N, OP_N, G3, false>(g, EpiGJ{W, ldw, pinv, c_lo, c_hi, 0});
       }
       if (c_hi < n) {
         GemmArgs g = gemm_args(n, n - c_hi, kb, W + c_lo, ldw, snap + c_hi, n, W + c_hi, ldw);
         if constexpr (TC) cta_gemm_tc_epi<OP_N, OP_N>(g, smem_raw, EpiGJ{W, ldw, pinv, c_lo, c_hi, c_hi});
-        else cta_gemm_epi<OP_N, OP_N, G3>(g, reinterpret_cast<cplx*>(smem_raw), EpiGJ{W, ldw, pinv, c_lo, c_hi, c_hi});
+        else cta_gemm_epi<OP_N, OP_N, G3, false>(g, EpiGJ{W, ldw, pinv, c_lo, c_hi, c_hi});
       }
       pc->mark(PH_INV_UPDATE);
     }
@@ -385,6 +385,228 @@ __device__ __noinline__ int cta_inverse_nb(cplx* W, int64_t ldw, int n, cplx* G,
   return flag;
 }
 
+NEGF_DEV void mbar_init(unsigned long long* b, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(b)), "r"(count) : "memory");
+}
+NEGF_DEV void mbar_inval(unsigned long long* b) {
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_addr(b)) : "memory");
+}
+NEGF_DEV void mbar_arrive(unsigned long long* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(b)) : "memory");
+}
+// Bounded wait for the barrier's first phase; false when the limit (about two seconds) expired.
+NEGF_DEV bool mbar_wait_once(unsigned long long* b) { return tc_bar_wait(smem_addr(b), 0u); }
+
+// Reciprocal of a pivot with one division: conj(a) / |a|^2 on a scaled by the power of two of its
+// larger component (exact, so no overflow or underflow of |a|^2).
+NEGF_DEV cplx crcp_scaled(cplx a) {
+  const int e = max(__double2hiint(a.x) & 0x7ff00000, __double2hiint(a.y) & 0x7ff00000);
+  const double s = __hiloint2double(0x7fe00000 - min(max(e, 0x00100000), 0x7fd00000), 0);  // 2^-exponent
+  const double x = a.x * s, y = a.y * s;
+  const double r = s / fma(x, x, y * y);
+  return cmk(x * r, -y * r);
+}
+
+// Inverse of a block of n <= 64 held in registers, W -> G: blocked Gauss-Jordan with implicit
+// partial pivoting (the in-place transform of the form above, PW columns to a panel).
+//
+// Lane l of warp w owns rows l + 32 a (a < RA) of columns CW w + j.  A warp holds whole columns, so
+// it factorises its panels alone, with reductions and shuffles and no barrier, and publishes each
+// with an mbarrier arrival; every other warp waits for panel t and applies it to its own columns,
+//     x[i][j] = (i a pivot of the panel ? 0 : x[i][j]) + sum_s P[i][s] v_s,   v_s = x[p_s][j],
+// where the pivot rows' entries are exchanged inside the warp.  Every panel has its own slot in
+// shared memory, so the warps need not be in step.  The pivot is the row whose |re| + |im| has the
+// largest leading 32 bits (within 2^-20 of the largest), the lowest lane among equals.
+// Bound by the latency of the panel chain (per column a reduction, a reciprocal and a rank-1 step
+// of PW columns).  Against the blocked form with 8-wide panels in shared memory, every SM inverting
+// its own matrices: n = 16 22.7 -> 7.4 us, 32 47 -> 17, 64 108 -> 57; the block inverse built on it
+// at n = 128 324 -> 219 us, at 256 1278 -> 1072.
+template <int RA, int CW, int PW>
+__device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, cplx* G, int64_t ldg) {
+  constexpr int NM = 32 * RA, NSUB = CW / PW, NPAN = 8 * NSUB;
+  static_assert(NSUB == 1 || NSUB == 2, "one or two panels per warp");
+  cplx* pan = smem_cplx();                      // [NPAN][PW][NM] factorised panels
+  cplx* rows = pan + NPAN * PW * NM;                                  // [8 warps][PW][PW] pivot-row entries
+  unsigned long long* bar = reinterpret_cast<unsigned long long*>(rows + 8 * PW * PW);  // [NPAN] panel published
+  int* piv = reinterpret_cast<int*>(bar + NPAN);                      // [8 CW] logical column -> physical row
+  int* pinv = piv + 8 * CW;                                           // [NM] physical row -> logical column
+  int* flag = pinv + NM;                                              // [0] singular pivot, [1] a panel never came
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  cplx x[RA][CW];
+#pragma unroll
+  for (int a = 0; a < RA; ++a)
+#pragma unroll
+    for (int j = 0; j < CW; ++j) {
+      const int i = lane + 32 * a, c = CW * warp + j;
+      x[a][j] = (i < n && c < n) ? W[(int64_t)i * ldw + c] : cmk(0.0, 0.0);
+    }
+  unsigned used = 0u;  // bit a: row lane + 32 a has served as a pivot (or does not exist)
+#pragma unroll
+  for (int a = 0; a < RA; ++a)
+    if (lane + 32 * a >= n) used |= 1u << a;
+  __syncthreads();  // whatever used this shared memory before is done with it
+  if (tid < NPAN) mbar_init(bar + tid, 1);
+  if (tid < 2) flag[tid] = 0;
+  __syncthreads();
+
+  // Panel g of this warp (g a compile-time index, so that x stays in registers): factorise its
+  // columns and publish them.
+  auto factor = [&](auto g_c) {
+    constexpr int g = decltype(g_c)::value;
+    const int c0 = CW * warp + PW * g, w = min(PW, n - c0);
+    if (w <= 0) return;
+#pragma unroll
+    for (int k = 0; k < PW; ++k) {
+      if (k < w) {
+        unsigned key[RA], best = 0u;
+#pragma unroll
+        for (int a = 0; a < RA; ++a) {
+          key[a] = (used >> a) & 1u ? 0u : 1u + (unsigned)(pivot_key(x[a][g * PW + k]) >> 32);
+          best = max(best, key[a]);
+        }
+        best = __reduce_max_sync(0xffffffffu, best);
+        int p = 0;
+#pragma unroll
+        for (int a = RA - 1; a >= 0; --a) {
+          const unsigned m = __ballot_sync(0xffffffffu, key[a] == best);
+          if (m) p = 32 * a + __ffs(m) - 1;
+        }
+        cplx q[PW];
+#pragma unroll
+        for (int j = 0; j < PW; ++j) {
+          q[j] = x[0][g * PW + j];
+#pragma unroll
+          for (int a = 1; a < RA; ++a)
+            if (a == (p >> 5)) q[j] = x[a][g * PW + j];
+          q[j].x = __shfl_sync(0xffffffffu, q[j].x, p & 31);
+          q[j].y = __shfl_sync(0xffffffffu, q[j].y, p & 31);
+        }
+        const bool sing = pivot_key_singular(pivot_key(q[k]));
+        const cplx d = crcp_scaled(q[k]);
+#pragma unroll
+        for (int j = 0; j < PW; ++j) q[j] = j == k ? d : cmul(q[j], d);
+#pragma unroll
+        for (int a = 0; a < RA; ++a) {
+          const bool pr = lane + 32 * a == p;
+          if (pr) used |= 1u << a;
+          const cplx m = x[a][g * PW + k];
+#pragma unroll
+          for (int j = 0; j < PW; ++j) {
+            const cplx y = j == k ? cmk(0.0, 0.0) : x[a][g * PW + j];
+            const cplx o = cmk(fma(-m.x, q[j].x, fma(m.y, q[j].y, y.x)), fma(-m.x, q[j].y, fma(-m.y, q[j].x, y.y)));
+            x[a][g * PW + j] = cmk(pr ? q[j].x : o.x, pr ? q[j].y : o.y);
+          }
+        }
+        if (lane == 0) {
+          piv[c0 + k] = p;
+          pinv[p] = c0 + k;
+          if (sing) flag[0] = 1;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < PW; ++k)
+#pragma unroll
+      for (int a = 0; a < RA; ++a) pan[(c0 + k) * NM + lane + 32 * a] = x[a][g * PW + k];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar + c0 / PW);
+  };
+
+  // Apply the published panel at column c0 to column group g of this warp.
+  cplx* rv = rows + warp * PW * PW;
+  auto apply = [&](auto g_c, int c0) {
+    constexpr int g = decltype(g_c)::value;
+    const int w = min(PW, n - c0);
+    bool gone[RA];  // rows that are pivots of the panel
+#pragma unroll
+    for (int a = 0; a < RA; ++a) gone[a] = false;
+#pragma unroll
+    for (int s = 0; s < PW; ++s) {
+      const int p = s < w ? piv[c0 + s] : -1;
+#pragma unroll
+      for (int a = 0; a < RA; ++a) {
+        const bool is = lane + 32 * a == p;
+        gone[a] |= is;
+#pragma unroll
+        for (int j = 0; j < PW; ++j)
+          if (is) rv[s * PW + j] = x[a][g * PW + j];
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < RA; ++a) {
+      if (gone[a]) used |= 1u << a;
+#pragma unroll
+      for (int j = 0; j < PW; ++j) {
+        x[a][g * PW + j].x = gone[a] ? 0.0 : x[a][g * PW + j].x;
+        x[a][g * PW + j].y = gone[a] ? 0.0 : x[a][g * PW + j].y;
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < PW; ++s) {
+      if (s < w) {
+        cplx m[RA];
+#pragma unroll
+        for (int a = 0; a < RA; ++a) m[a] = pan[(c0 + s) * NM + lane + 32 * a];
+#pragma unroll
+        for (int j = 0; j < PW; ++j) {
+          const cplx v = rv[s * PW + j];
+#pragma unroll
+          for (int a = 0; a < RA; ++a) x[a][g * PW + j] = cfma(m[a], v, x[a][g * PW + j]);
+        }
+      }
+    }
+    __syncwarp();  // rv is rewritten by the next call
+  };
+
+  constexpr std::integral_constant<int, 0> G0{};
+  constexpr std::integral_constant<int, NSUB - 1> GL{};
+  bool lost = false;
+  if (warp == 0) factor(G0);
+  for (int w0 = 0; w0 < 8 && CW * w0 < n; ++w0) {
+    const int c0 = CW * w0, c1 = c0 + PW;
+    if (warp != w0) {
+      lost |= !mbar_wait_once(bar + c0 / PW);
+      __syncwarp();
+      if (__any_sync(0xffffffffu, lost)) break;
+      apply(G0, c0);
+      if (NSUB == 1 && warp == w0 + 1) factor(G0);
+    }
+    if constexpr (NSUB == 2) {
+      apply(GL, c0);
+      if (c1 < n) {
+        if (warp == w0) {
+          factor(GL);
+          apply(G0, c1);
+        } else {
+          lost |= !mbar_wait_once(bar + c1 / PW);
+          __syncwarp();
+          if (__any_sync(0xffffffffu, lost)) break;
+          apply(G0, c1);
+          if (warp == w0 + 1) factor(G0);
+          apply(GL, c1);
+        }
+      }
+    }
+  }
+  if (lost) flag[1] = 1;
+  __syncthreads();
+  // G[i][j] = W[p(i)][p^-1(j)]
+  if (!flag[1]) {
+#pragma unroll
+    for (int a = 0; a < RA; ++a)
+#pragma unroll
+      for (int j = 0; j < CW; ++j) {
+        const int i = lane + 32 * a, c = CW * warp + j;
+        if (i < n && c < n) G[(int64_t)pinv[i] * ldg + piv[c]] = x[a][j];
+      }
+  }
+  const int f = flag[0] | flag[1];
+  if (tid < NPAN) mbar_inval(bar + tid);
+  __syncthreads();
+  return f;
+}
+
 // G3: complex products of the rank updates (Gauss/3M or conventional 4M);
 // TC: outer update on the tensor-core 3xTF32 GEMM.  ob: outer block width,
 // a multiple of 32 up to INV_OB_MAX (narrower blocks move work from the
@@ -393,12 +615,25 @@ __device__ __noinline__ int cta_inverse_nb(cplx* W, int64_t ldw, int n, cplx* G,
 template <bool G3 = true, bool TC = false>
 NEGF_DEV int cta_inverse(cplx* W, int64_t ldw, int n, cplx* G, int64_t ldg, char* smem_raw, PhaseClock* pc,
                          cplx* snap, int ob = INV_OB) {
+  // Up to n = 64 the block fits the CTA's registers.  The mixed sweep keeps the panel form: its
+  // FP32-accurate products amplify every rounding of the leaves, so its results would move.
+  if constexpr (!TC) {
+    if (n <= 64) {
+      const int f = n <= 16   ? cta_inverse_reg<1, 2, 2>(W, ldw, n, G, ldg)
+                    : n <= 32 ? cta_inverse_reg<1, 4, 4>(W, ldw, n, G, ldg)
+                              : cta_inverse_reg<2, 8, 4>(W, ldw, n, G, ldg);
+      pc->mark(PH_INV_PANEL);
+      return f;
+    }
+  }
   // Narrow panels for small blocks (the block inverse's 64-wide leaves): a column step's
   // latency chain is shorter (16-wide measured 22 % faster than 32-wide at n = 64, 8 % at
   // n = 128, where the rank-16 updates start to cost more; 8-wide another 4-9 % for n <= 64).
   // One register row per thread up to n = 256.
   if (n > 64 && n <= 256) return cta_inverse_nb<32, 1, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
-  if (n <= 64) return cta_inverse_nb<INV_SMALL_NB, 1, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
+  if constexpr (TC) {
+    if (n <= 64) return cta_inverse_nb<INV_SMALL_NB, 1, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
+  }
   return cta_inverse_nb<16, 2, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
 }
 

@@ -82,7 +82,7 @@ NEGF_DEV void lu_gemm_sub(const LuCtx& c, int M, int N, int K, const cplx* A, in
   GemmArgs g = gemm_args(M, N, K, A, lda, B, ldb, C, ldc);
   g.alpha = cmk(-1.0, 0.0);
   g.D = C; g.ldd = ldc; g.beta = cmk(1.0, 0.0); g.use_d = true;
-  cta_gemm<OP_N, OP_N, false, true>(g, reinterpret_cast<cplx*>(c.smem));  // 4M products (see lopez_sancho.cu)
+  cta_gemm<OP_N, OP_N, false>(g);  // 4M products (see lopez_sancho.cu)
   c.mark(PH_INV_UPDATE);
 }
 

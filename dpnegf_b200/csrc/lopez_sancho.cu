@@ -228,7 +228,7 @@ NEGF_DEV void ls_item(const NegfLsProblem& P, const NegfLsItem& it, cplx* slot, 
 }
 
 __global__ void __launch_bounds__(CTA_THREADS, 1) ls_kernel(const NegfLsProblem P) {
-  extern __shared__ __align__(16) char smem[];
+  char* const smem = negf_smem;
   __shared__ int s_item;
   __shared__ double red[CTA_THREADS / 32];
   unsigned* queue = reinterpret_cast<unsigned*>(P.scratch);

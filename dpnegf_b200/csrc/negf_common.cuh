@@ -37,6 +37,10 @@ NEGF_DEV cplx crcp(cplx a) {
 NEGF_DEV double cabs1(cplx a) { return fabs(a.x) + fabs(a.y); }
 NEGF_DEV bool cfinite(cplx a) { return isfinite(a.x) && isfinite(a.y); }
 
+// The CTA's dynamic shared memory, shared by the CTA-wide building blocks one after another.
+extern __shared__ __align__(1024) char negf_smem[];
+NEGF_DEV cplx* smem_cplx() { return reinterpret_cast<cplx*>(negf_smem); }
+
 // ---------------------------------------------------------------------------
 // cp.async (16-byte, L2-only) with zero fill when the source is out of range.
 NEGF_DEV void cp_async16(void* smem_dst, const void* gmem_src, bool valid) {

@@ -43,7 +43,7 @@ inline size_t gamma_part_bytes(const NegfGammaSum& p) {
 inline int64_t gamma_split_len(int64_t K, int split) { return ((K + split - 1) / split + 15) / 16 * 16; }
 
 __global__ void __launch_bounds__(CTA_THREADS, 1) gamma_stack_kernel(const NegfGammaSum P, cplx* Tst, cplx* Gst) {
-  extern __shared__ __align__(16) char smem_raw[];
+  char* const smem_raw = negf_smem;
   cplx* smem = reinterpret_cast<cplx*>(smem_raw);
   const int64_t K = (int64_t)P.n_items * P.k;
   for (int i = blockIdx.x; i < P.n_items; i += gridDim.x) {
@@ -70,7 +70,7 @@ struct EpiRealOut {
 __global__ void __launch_bounds__(CTA_THREADS, 1) gamma_reduce_kernel(const NegfGammaSum P, const cplx* Tst,
                                                                       const cplx* Gst, double* part,
                                                                       int64_t klen) {
-  extern __shared__ __align__(16) char smem_raw[];
+  char* const smem_raw = negf_smem;
   cplx* smem = reinterpret_cast<cplx*>(smem_raw);
   const int64_t K = (int64_t)P.n_items * P.k;
   const int m0 = blockIdx.y * GT_M, n0 = blockIdx.x * GT_N;
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gamma_reduce_kernel(const Negf
     return;
   }
   GemmArgs g = gemm_args(M, N, Kz, Tst + (int64_t)m0 * K + k0, K, Gst + (int64_t)n0 * K + k0, K, nullptr, 0);
-  cta_gemm_epi<OP_N, OP_C, true, EpiRealOut, true>(g, smem, EpiRealOut{out, P.n, m0, n0});
+  cta_gemm_epi<OP_N, OP_C, true, true>(g, EpiRealOut{out, P.n, m0, n0});
 }
 
 // Stage 3: out = sum of the partial outputs in range order.
@@ -240,7 +240,7 @@ NEGF_DEV void la_item(const NegfLeadAdjProblem& P, int idx, cplx* slot, char* sm
 }
 
 __global__ void __launch_bounds__(CTA_THREADS, 1) lead_adjoint_kernel(const NegfLeadAdjProblem P) {
-  extern __shared__ __align__(16) char smem[];
+  char* const smem = negf_smem;
   __shared__ double red[CTA_THREADS / 32];
   cplx* slot = reinterpret_cast<cplx*>(P.scratch) + (size_t)blockIdx.x * la_slot_elems(P);
   const size_t mn = (size_t)la_max_n(P.lead);

@@ -211,13 +211,13 @@ NEGF_DEV void gemm(cplx* smem, int M, int N, int K, const cplx* A, int64_t lda, 
   g.alpha = alpha;
   if (D) { g.D = D; g.ldd = ldd; g.beta = beta; g.use_d = true; }
   if constexpr (MX) cta_gemm_tc<OPA, OPB>(g, reinterpret_cast<char*>(smem));
-  else cta_gemm<OPA, OPB>(g, smem);
+  else cta_gemm<OPA, OPB>(g);
 }
 
 template <int OPA, int OPB, bool MX, class Epi>
 NEGF_DEV void gemm_epi(const GemmArgs& g, cplx* smem, const Epi& e) {
   if constexpr (MX) cta_gemm_tc_epi<OPA, OPB>(g, reinterpret_cast<char*>(smem), e);
-  else cta_gemm_epi<OPA, OPB, true>(g, smem, e);
+  else cta_gemm_epi<OPA, OPB, true, true>(g, e);
 }
 
 // Recursive 2x2 block inverse (inv_mode 1): G = W^-1, W destroyed.  With
@@ -998,7 +998,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
 
 template <bool MX, int FEAT>
 __global__ void __launch_bounds__(CTA_THREADS, 1) rgf_kernel(const NegfRgfProblem P) {
-  extern __shared__ __align__(1024) char smem[];
+  char* const smem = negf_smem;
   __shared__ int s_item;
   __shared__ double red[CTA_THREADS / 32];
   unsigned* queue = reinterpret_cast<unsigned*>(P.scratch);

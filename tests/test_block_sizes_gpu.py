@@ -1,0 +1,62 @@
+"""The sweep at block sizes where its kernels change form: the in-register inverse (row and column
+edges of its 16, 32 and 64-wide layouts), the block inverse just above it, and ragged GEMM tiles."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ETA = 1e-3
+# The blocks are well conditioned (eta and the retarded self-energies bound |G| by O(10)), each entry
+# of a Green's-function block is a sum of at most K n products, so a backward-stable sweep leaves
+# K n eps cond ~ 4 * 130 * 2.2e-16 * 1e2 ~ 1e-11 relative to the block's norm.
+TOL = 1e-10
+
+
+def _device(dims, seed):
+    rng = np.random.default_rng(seed)
+    c = lambda m, n, s: (rng.normal(size=(m, n)) + 1j * rng.normal(size=(m, n))) * s
+    herm = lambda x: (x + x.conj().T) / 2
+    hd = [herm(c(n, n, 0.5 / np.sqrt(n))) + np.diag(rng.uniform(-2, 2, n)) for n in dims]
+    sd = [np.eye(n) + herm(c(n, n, 0.02 / np.sqrt(n))) for n in dims]
+    hu = [c(a, b, 0.5 / np.sqrt(max(a, b))) for a, b in zip(dims, dims[1:])]
+    su = [c(a, b, 0.01 / np.sqrt(max(a, b))) for a, b in zip(dims, dims[1:])]
+    se = []
+    for n in (dims[0], dims[-1]):
+        x = c(n, n, 0.5 / np.sqrt(n))
+        se.append(herm(c(n, n, 0.3 / np.sqrt(n))) - 1j * (x @ x.conj().T + 0.2 * np.eye(n)))
+    return hd, hu, [u.conj().T for u in hu], sd, su, [s.conj().T for s in su], se
+
+
+@pytest.mark.parametrize("n", [1, 2, 5, 8, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 95, 97, 130])
+def test_blocks_match_oracle(n):
+    from dpnegf_b200.recursive_green_cal import recursive_gf
+    dims = [n, max(1, n - 1), n + 1]
+    hd, hu, hl, sd, su, sl, (seL, seR) = _device(dims, 100 + n)
+    B = 3
+    E = np.linspace(-0.7, 0.9, B)
+    t = lambda x: torch.as_tensor(np.ascontiguousarray(x), dtype=torch.complex128, device="cuda")
+    ts = lambda xs: [t(x) for x in xs]
+    rep = lambda s: t(s).expand(B, -1, -1)
+    got = recursive_gf(torch.as_tensor(E).cuda(), ts(hl), ts(hd), ts(hu), ts(sd), ts(su), ts(sl), rep(seL), rep(seR),
+                       eta=ETA, need_gr_lc=True)
+    A = np.zeros((sum(dims), sum(dims)), complex)
+    off = np.concatenate([[0], np.cumsum(dims)])
+    for e in range(B):
+        z = E[e] + 1j * ETA
+        A[:] = 0
+        for q in range(3):
+            A[off[q]:off[q + 1], off[q]:off[q + 1]] = z * sd[q] - hd[q]
+        for q in range(2):
+            A[off[q]:off[q + 1], off[q + 1]:off[q + 2]] = z * su[q] - hu[q]
+            A[off[q + 1]:off[q + 2], off[q]:off[q + 1]] = z * sl[q] - hl[q]
+        A[:dims[0], :dims[0]] -= seL
+        A[-dims[2]:, -dims[2]:] -= seR
+        G = np.linalg.inv(A)
+        blk = lambda i, j: G[off[i]:off[i + 1], off[j]:off[j + 1]]
+        pairs = [(got[0][e], blk(0, 2))] + [(got[1][q][e], blk(q, 2)) for q in range(3)]
+        pairs += [(got[2][q][e], blk(q, q)) for q in range(3)]
+        pairs += [(got[3][q][e], blk(q + 1, q)) for q in range(2)] + [(got[4][q][e], blk(q, q + 1)) for q in range(2)]
+        for x, y in pairs:
+            x = x.cpu().numpy()
+            assert np.linalg.norm(x - y) <= TOL * max(np.linalg.norm(y), 1e-3 * np.linalg.norm(G)), (n, e)
