@@ -43,6 +43,7 @@ MIXED = 1 << 13
 REFINE = 1 << 14
 GREATER = 1 << 15
 ADJ_DOS = 1 << 16
+KEEP_LG = 1 << 17
 PHASES = ("form", "gemm_fwd", "inv_stage", "inv_panel", "inv_update", "inv_gather", "gemm_bwd", "lesser",
           "dos", "trans", "other", "refine")
 

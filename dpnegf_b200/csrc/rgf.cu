@@ -37,6 +37,9 @@ int negf_rgf_run(const NegfRgfProblem* p, void* stream) {
   if ((p->flags & NEGF_REFINE) && (p->col_slab <= 0 || !(p->flags & NEGF_TRANS))) return NEGF_ERR_ARGUMENT;
   if ((p->flags & NEGF_ADJ_DOS) && !(p->flags & NEGF_ADJOINT)) return NEGF_ERR_ARGUMENT;
   if (p->ckpt < 0) return NEGF_ERR_ARGUMENT;
+  if ((p->flags & NEGF_KEEP_LG) &&
+      ((p->flags & (NEGF_MIXED | NEGF_LESSER | NEGF_GREATER | NEGF_ADJ_DOS)) || p->ckpt > 0))
+    return NEGF_ERR_ARGUMENT;
   if (p->ckpt > 0 && (p->flags & NEGF_ADJOINT) &&
       ((p->flags & (NEGF_OUT_GR_LEFT | NEGF_LESSER | NEGF_GREATER | NEGF_REFINE)) || p->ckpt_blocks <= 0))
     return NEGF_ERR_ARGUMENT;

@@ -71,6 +71,7 @@ int negf_rgf_static_slots(const NegfRgfProblem* p) {
   if (!p || p->n_slots <= 0 || p->max_n <= 0) return NEGF_ERR_ARGUMENT;
   if (p->max_n > NEGF_MAX_BLOCK) return NEGF_ERR_UNSUPPORTED;
   NegfRgfProblem q = *p;
+  q.flags &= ~NEGF_KEEP_LG;  // slots are scarcer than products here
   q.n_slots = 1;
   const size_t one = negf_rgf_scratch_bytes(&q);
   if (one == 0) return NEGF_ERR_ARGUMENT;
@@ -87,6 +88,7 @@ int negf_rgf_run_static(const NegfRgfProblem* p, void* stream) {
   const int slots = negf_rgf_static_slots(p);
   if (slots <= 0) return slots;
   NegfRgfProblem q = *p;
+  q.flags &= ~NEGF_KEEP_LG;
   q.n_slots = slots;
   void* addr = nullptr;
   const int st = static_scratch_address(&addr);

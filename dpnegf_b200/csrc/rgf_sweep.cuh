@@ -48,6 +48,7 @@ struct SlotBufs {
   cplx* yslab;    // refinement: forward-substituted residual y_q of every block
   cplx* gipslab;  // greater gip_q storage when gip_left is not an output
   cplx* Pd;       // greater: gpd_{q+1} when gpd is not an output
+  cplx* lgslab;   // NEGF_KEEP_LG: L_q g_q of every block, from the forward sweep
   cplx* gdslab;   // density gradient: z-tangent dg_q/dz of every block
   cplx *D0, *D1;  // density gradient: dG_qq/dz of the current / next block
   cplx *W, *T1, *Lz, *Uz, *gU, *Gd, *Gl, *Gu, *Gt0, *Gt1, *tA, *tB, *tC, *tD;
@@ -72,6 +73,7 @@ __host__ __device__ inline size_t rgf_slot_elems(const NegfRgfProblem& p) {
   if (p.flags & (NEGF_ADJOINT | NEGF_REFINE)) e += (size_t)p.col_slab;
   if (p.flags & NEGF_REFINE) e += (size_t)p.col_slab;
   if (p.flags & NEGF_GREATER) e += (size_t)p.max_g_slab + mn2;
+  if (p.flags & NEGF_KEEP_LG) e += (size_t)p.max_g_slab;  // sum n_q n_{q+1} <= sum n_q^2
   if ((p.flags & NEGF_ADJOINT) && (p.flags & NEGF_ADJ_DOS)) e += rgf_g_elems(p) + 2 * mn2;
   return (e + 15) & ~(size_t)15;  // keep slots 256-byte aligned
 }
@@ -94,6 +96,7 @@ NEGF_DEV SlotBufs slot_bufs(const NegfRgfProblem& p, int slot) {
   s.yslab = nullptr;
   s.gipslab = nullptr;
   s.Pd = nullptr;
+  s.lgslab = nullptr;
   s.gdslab = s.D0 = s.D1 = nullptr;
   if (!(p.flags & NEGF_OUT_GR_LEFT)) { s.gslab = b; b += rgf_g_elems(p); }
   if (p.flags & NEGF_LESSER) { s.ginslab = b; b += p.max_g_slab; }
@@ -104,6 +107,7 @@ NEGF_DEV SlotBufs slot_bufs(const NegfRgfProblem& p, int slot) {
     s.gipslab = b; b += p.max_g_slab;
     s.Pd = b; b += mn2;
   }
+  if (p.flags & NEGF_KEEP_LG) { s.lgslab = b; b += p.max_g_slab; }
   if ((p.flags & NEGF_ADJOINT) && (p.flags & NEGF_ADJ_DOS)) {
     s.gdslab = b; b += rgf_g_elems(p);
     s.D0 = b; b += mn2;
@@ -345,13 +349,13 @@ struct EpiGrad {
 
 // One forward step of an item: g_q = (-D_q - L_{q-1} g_{q-1} U_{q-1})^-1 into gq from gprev
 // (null for q = 0), and with dgq its z-tangent dg_q from dgprev.  Uses the slot's W, T1, Lz, Uz
-// and tA..tE; leaves L_{q-1}, U_{q-1} in Lz, Uz and L_{q-1} g_{q-1} in T1 for the lesser and
-// greater steps.  Inlined into the sweep; the checkpointed adjoint recomputes its segments
+// and tA..tE; leaves L_{q-1}, U_{q-1} in Lz, Uz for the lesser and greater steps, and
+// L_{q-1} g_{q-1} in lg (T1 when null; the tangent reads it from T1).  Inlined into the sweep; the checkpointed adjoint recomputes its segments
 // through the non-inlined copy below.  Returns the singular-pivot flag.
 template <bool MX>
 NEGF_DEV int forward_block_body(const NegfRgfProblem& P, const NegfItem& it, const SlotBufs& sb,
                                 char* smem_raw, double* red, PhaseClock& pc, int q,
-                                const cplx* gprev, cplx* gq, const cplx* dgprev, cplx* dgq) {
+                                const cplx* gprev, cplx* gq, const cplx* dgprev, cplx* dgq, cplx* lg = nullptr) {
   cplx* smem = reinterpret_cast<cplx*>(smem_raw);
   const NegfDevice dv = P.devices[it.dev];
   const NegfBlock* blk = P.blocks + dv.blk0;
@@ -372,8 +376,9 @@ NEGF_DEV int forward_block_body(const NegfRgfProblem& P, const NegfItem& it, con
     form_shift(sb.Uz, hs, bp.hu, bp.su, z, np, nq, smem);  // U_{q-1}: n_{q-1} x n_q
     __syncthreads();
     pc.mark(PH_FORM);
-    gemm<OP_N, OP_N, MX>(smem, nq, np, np, sb.Lz, np, gprev, np, sb.T1, np);
-    gemm<OP_N, OP_N, MX>(smem, nq, nq, np, sb.T1, np, sb.Uz, nq, sb.W, nq, MONE, sb.W, nq);
+    cplx* t1 = !MX && lg ? lg : sb.T1;
+    gemm<OP_N, OP_N, MX>(smem, nq, np, np, sb.Lz, np, gprev, np, t1, np);
+    gemm<OP_N, OP_N, MX>(smem, nq, nq, np, t1, np, sb.Uz, nq, sb.W, nq, MONE, sb.W, nq);
     pc.mark(PH_GEMM_FWD);
   } else {
     __syncthreads();
@@ -527,7 +532,8 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
   // ------------------------------------------------------------ forward sweep
   for (int q = 0; q < K; ++q) {
     bad |= forward_block_body<MX>(P, it, sb, smem_raw, red, pc, q, q > 0 ? gptr(q - 1) : nullptr, gptr(q),
-                                  dosg && q > 0 ? dgptr(q - 1) : nullptr, dosg ? dgptr(q) : nullptr);
+                                  dosg && q > 0 ? dgptr(q - 1) : nullptr, dosg ? dgptr(q) : nullptr,
+                                  sb.lgslab && q > 0 ? sb.lgslab + blk[q - 1].gu : nullptr);
     const NegfBlock& b = blk[q];
     const int nq = b.n;
     if (lesser) {
@@ -658,12 +664,22 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
                                    want_dg ? dgptr(r - 1) : nullptr, want_dg ? dgptr(r) : nullptr);
     seg_lo = c;
   };
-  for (int q = K - 2; q >= 0; --q) {
+  // Only the products that something asked for are formed.  T(E), g_trans, gr_lc and the spectral
+  // diagonals need g U and the last column alone; G_qq and what is read from it need grl as well, and
+  // gru only as an output, for lesser / greater / tangents, or for the DOS of a non-orthogonal basis.
+  // With L g kept from the forward sweep, grl is one product (G_{q+1,q+1} (L g)) and L is not needed.
+  // The mixed kernel forms them all: it holds every feature in one instantiation, and the extra live
+  // conditions there cost 5 % of its sweep.
+  const bool keep_lg = !MX && sb.lgslab != nullptr;
+  const bool need_full = lesser || greater || adj;
+  const bool need_G = MX || need_full || want_dos || (fl & (NEGF_OUT_GRD | NEGF_OUT_GRL | NEGF_OUT_GRU | NEGF_ORB_GDIAG)) != 0;
+  for (int q = (need_G || need_gt) ? K - 2 : -1; q >= 0; --q) {
     if (ck && q < seg_lo) load_segment(seg_lo - ck, dosg);
     const NegfBlock& b = blk[q];
     const int nq = b.n, nn = b.n_next;
     const int64_t szu = (int64_t)nq * nn;
-    form_shift(sb.Lz, hs, b.hl, b.sl, z, nn, nq, smem);  // L_q: n_{q+1} x n_q
+    const bool need_gru = MX || lesser || greater || dosg || (fl & NEGF_OUT_GRU) != 0 || (want_dos && b.slT >= 0);
+    if (need_G && !keep_lg) form_shift(sb.Lz, hs, b.hl, b.sl, z, nn, nq, smem);  // L_q: n_{q+1} x n_q
     form_shift(sb.Uz, hs, b.hu, b.su, z, nq, nn, smem);  // U_q: n_q x n_{q+1}
     __syncthreads();
     pc.mark(PH_FORM);
@@ -672,10 +688,16 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     cplx* gru = (fl & NEGF_OUT_GRU) ? out + b.o_gru + row * szu : sb.Gu;
     cplx* grd = (fl & NEGF_OUT_GRD) ? out + b.o_grd + row * sq(q) : (adj ? sb.grdslab + b.g : sb.Gd);
     gemm<OP_N, OP_N, MX>(smem, nq, nn, nq, g, nq, sb.Uz, nn, sb.gU, nn);         // gU = g U
-    gemm<OP_N, OP_N, MX>(smem, nn, nq, nn, Gnext, nn, sb.Lz, nq, sb.T1, nq);     // G_{q+1,q+1} L
-    gemm<OP_N, OP_N, MX>(smem, nn, nq, nq, sb.T1, nq, g, nq, grl, nq);           // grl
-    gemm<OP_N, OP_N, MX>(smem, nq, nn, nn, sb.gU, nn, Gnext, nn, gru, nn);       // gru
-    gemm<OP_N, OP_N, MX>(smem, nq, nq, nn, sb.gU, nn, grl, nq, grd, nq, ONE, g, nq);  // grd
+    if (need_G) {
+      if (keep_lg) {
+        gemm<OP_N, OP_N, MX>(smem, nn, nq, nn, Gnext, nn, sb.lgslab + b.gu, nq, grl, nq);  // grl = G_{q+1,q+1} (L g)
+      } else {
+        gemm<OP_N, OP_N, MX>(smem, nn, nq, nn, Gnext, nn, sb.Lz, nq, sb.T1, nq);           // G_{q+1,q+1} L
+        gemm<OP_N, OP_N, MX>(smem, nn, nq, nq, sb.T1, nq, g, nq, grl, nq);                 // grl
+      }
+      if (need_gru) gemm<OP_N, OP_N, MX>(smem, nq, nn, nn, sb.gU, nn, Gnext, nn, gru, nn);  // gru
+      gemm<OP_N, OP_N, MX>(smem, nq, nq, nn, sb.gU, nn, grl, nq, grd, nq, ONE, g, nq);      // grd
+    }
     if (need_gt) {
       cplx* gtn = (fl & NEGF_OUT_GR_LC) ? out + b.o_grlc + row * (int64_t)nq * nN
                                           : (sb.colslab ? sb.colslab + b.gc : (tog ? sb.Gt1 : sb.Gt0));
@@ -774,7 +796,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       }
       pc.mark(PH_DOS);
     }
-    Gnext = grd;
+    if (need_G) Gnext = grd;
   }
   if (dosg && seL && it.gse_l) {  // Dnext = dG_11/dz
     acc_se(it.gse_l, it.nse_l, 0, Dnext, blk[0].n, 0, min(blk[0].n, it.nse_l));

@@ -114,6 +114,7 @@ class Geometry:
             dv["g_slab"] = g
             devs.append(dv)
             self.max_g_slab = max(self.max_g_slab, g)
+            self.max_blocks = max(getattr(self, "max_blocks", 0), K)
             self.col_slab = max(getattr(self, "col_slab", 0), gc)
             self.u_slab = max(getattr(self, "u_slab", 0), gu)
         if self.max_n > _lib.NEGF_MAX_BLOCK:
@@ -486,8 +487,23 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     if inverse not in ("gj", "block"):
         raise ValueError(f"inverse must be 'gj' or 'block', not {inverse!r}")
     prob.inv_mode = 1 if inverse == "block" else 0
+    # L g kept for the backward sweep: one block product of eight less, while its slab leaves the
+    # scratch within a quarter of the GPU's memory
+    if precision == "fp64" and not (lesser or greater or ckpt or adjoint_w_dos is not None) and geom.max_blocks > 1 \
+            and flags & (_lib.OUT_GRD | _lib.OUT_GRL | _lib.OUT_GRU | _lib.DOS | _lib.ORB_DOS | _lib.ORB_GDIAG
+                         | _lib.ADJOINT):
+        prob.flags = flags | _lib.KEEP_LG
+        if lib.negf_rgf_scratch_bytes(ctypes.byref(prob)) > torch.cuda.get_device_properties(dev).total_memory // 4:
+            prob.flags = flags
     need = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
-    scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
+    try:
+        scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
+    except torch.cuda.OutOfMemoryError:
+        if prob.flags == flags:
+            raise
+        prob.flags = flags
+        need = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
+        scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
     prob.scratch = scratch.data_ptr()
     prob.scratch_bytes = scratch.numel()
     grad_t = None

@@ -71,6 +71,11 @@ extern "C" {
 #define NEGF_GREATER (1u << 15)    /* greater sweep from s_out: gip_left, gpd, gpl, gpu
                                       (recursive_green_cal.py:143-161, :267-289) */
 
+#define NEGF_KEEP_LG (1u << 17)    /* keep L_q g_q of the forward sweep for the backward sweep (one block product
+                                      less per block, max_g_slab more elements per slot; uses NegfBlock.gu).
+                                      FP64 retarded sweep and T adjoint only: not with MIXED, LESSER, GREATER,
+                                      ADJ_DOS or ckpt > 0.  The static-scratch entry point ignores it */
+
 /* Phase indices of NegfRgfProblem.phase_cycles (clock64 cycles per slot). */
 #define NEGF_PHASES 12 /* form, gemm_fwd, inv_stage, inv_panel, inv_update, inv_gather,
                           gemm_bwd, lesser, dos, trans, other, refine */
@@ -87,7 +92,7 @@ typedef struct NegfBlock {
   int64_t orb0;   /* first orbital of block q within its device */
   int64_t g;      /* offset of g_q inside one item's g slab (prefix sum of n^2) */
   int64_t gc;     /* NEGF_ADJOINT: offset of G_qN in the per-slot column slab (prefix of n_q n_N) */
-  int64_t gu;     /* NEGF_ADJOINT: offset of the coupling gradients of block q (prefix of n_q n_{q+1}) */
+  int64_t gu;     /* NEGF_ADJOINT, NEGF_KEEP_LG: offset of the coupling blocks of block q (prefix of n_q n_{q+1}) */
   /* block outputs: offset of batch row 0 in out; row b adds b * (block size).
      -1 when not produced. */
   int64_t o_grd, o_grl, o_gru, o_grlc, o_grleft;

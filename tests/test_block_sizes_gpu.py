@@ -60,3 +60,33 @@ def test_blocks_match_oracle(n):
         for x, y in pairs:
             x = x.cpu().numpy()
             assert np.linalg.norm(x - y) <= TOL * max(np.linalg.norm(y), 1e-3 * np.linalg.norm(G)), (n, e)
+
+
+@pytest.mark.parametrize("overlap", [True, False])
+@pytest.mark.parametrize("dims", [[20, 24, 16, 24], [70, 66, 90]])
+def test_every_output_selection_agrees(dims, overlap):
+    """The sweep forms only the products its outputs need: each output alone equals the same output
+    of a sweep that returns everything (the same products in another association at most: TOL)."""
+    from dpnegf_b200 import rgf_plan
+    hd, hu, hl, sd, su, sl, (seL, seR) = _device(dims, 7)
+    if not overlap:
+        su, sl, sd = [0 * x for x in su], [0 * x for x in sl], [np.eye(n) for n in dims]
+    t = lambda x: torch.as_tensor(np.ascontiguousarray(x), dtype=torch.complex128, device="cuda")
+    ts = lambda xs: [t(x) for x in xs]
+    geom = rgf_plan.Geometry([rgf_plan.DeviceBlocks(ts(hd), ts(hu), ts(hl), ts(sd), ts(su), ts(sl))])
+    B = 4
+    E = [torch.linspace(-0.7, 0.9, B, dtype=torch.float64).cuda()]
+    L, R = [t(seL).expand(B, -1, -1)], [t(seR).expand(B, -1, -1)]
+    run = lambda **kw: rgf_plan.run(geom, E, L, R, eta=ETA, **kw)
+    tags = ("g_trans", "grd", "grl", "gru", "gr_lc")
+    full = run(outputs=tags, trans=True, dos=True, orb_dos=True, orb_g=True, orb_ar=True,
+               s_in=[[torch.zeros(B, n, n, dtype=torch.complex128, device="cuda") for n in dims]])
+    same = lambda x, y: float((x - y).abs().max()) <= TOL * float(y.abs().max())
+    for key in ("trans", "dos", "orb_dos", "orb_g", "orb_ar"):
+        assert same(getattr(run(outputs=(), **{key: True}), key), getattr(full, key)), key
+    both = run(outputs=(), trans=True, dos=True)
+    assert same(both.trans, full.trans) and same(both.dos, full.dos)
+    for tag in tags:
+        got, want = run(outputs=(tag,)).blocks[0][tag], full.blocks[0][tag]
+        for x, y in [(got, want)] if tag == "g_trans" else zip(got, want):
+            assert same(x, y), tag
