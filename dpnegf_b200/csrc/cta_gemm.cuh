@@ -13,7 +13,7 @@
 #include <type_traits>
 #include "negf_common.cuh"
 
-namespace negf {
+namespace NEGF_NS {
 
 #ifndef NEGF_GT_K
 #define NEGF_GT_K 16
@@ -67,13 +67,13 @@ template <int OP>
 NEGF_DEV int b_idx(int k, int n) { return OP == OP_C ? n * PITCH_MK + k : k * PITCH_KN + n; }
 
 // Stage the (m0,k0) tile of op(A) into sA.
-template <int OP>
+template <int OP, int TM = GT_M>
 NEGF_DEV void load_a_tile(cplx* sA, const GemmArgs& g, int m0, int k0, int tid) {
 #pragma unroll
-  for (int s = 0; s < GT_LOADS; ++s) {
+  for (int s = 0; s < GT_LOADS * TM / GT_M; ++s) {
     int e = tid + s * CTA_THREADS;
     if (OP == OP_C) {  // stored X is K x M: tile rows k, cols m
-      int r = e >> 6, c = e & 63;
+      int r = e / TM, c = e % TM;
       int k = k0 + r, m = m0 + c;
       bool v = (k < g.K) && (m < g.M);
       const cplx* src = v ? g.A + (int64_t)k * g.lda + m : g.A;
@@ -136,12 +136,12 @@ NEGF_DEV int acc_col(int j, int e, int wn, int lane) { return wn + 8 * j + 2 * (
 struct Frag8 {
   double ar[2][4], ai[2][4], as[2][4], br[2][2], bi[2][2], bs[2][2];  // as/bs: re + im (3M) or -im (4M, as)
 };
-template <bool CONJ_A, bool CONJ_B, bool G3, class AIdx, class BIdx>
+template <bool CONJ_A, bool CONJ_B, bool G3, int MI = 2, class AIdx, class BIdx>
 NEGF_DEV void frag8_load(Frag8& f, const cplx* sA, const cplx* sB, int ks, int wm, int wn, int lane, AIdx aidx,
                          BIdx bidx) {
   const int gr = lane >> 2, k0 = ks * 8 + (lane & 3);
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < MI; ++i) {
     const int r = wm + 16 * i + gr;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -163,10 +163,10 @@ NEGF_DEV void frag8_load(Frag8& f, const cplx* sA, const cplx* sB, int ks, int w
     }
   }
 }
-template <bool G3>
+template <bool G3, int MI = 2>
 NEGF_DEV void frag8_mma(Acc3M& acc, const Frag8& f) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       dmma1688(acc.t1[i][j], f.ar[i], f.br[j]);
@@ -199,10 +199,10 @@ NEGF_DEV cplx acc_value(const Acc3M& acc, int i, int j, int e) {
 }
 
 // Visit every accumulator element of this warp: f(row, col, value).
-template <bool G3, class F>
+template <bool G3, int MI = 2, class F>
 NEGF_DEV void acc_foreach(const Acc3M& acc, int wm, int wn, int lane, F f) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -243,11 +243,11 @@ struct EpiStore {
 // (73 % of the DMMA peak); 4M products at 256 666 -> 644.  Inside the 3M sweep at n = 128 and 256,
 // where registers are short, the drifting form is 2-4 % slower, so the sweep takes it for ragged
 // products only (see gemm_ragged); the 4M lead kernels take it always (3.7 % at n = 256).
-template <int OPA, int OPB, bool G3, bool DRIFT, class Epi>
+template <int OPA, int OPB, bool G3, bool DRIFT, int MI = 2, class Epi>
 NEGF_DEV void gemm_body(const GemmArgs& g, const Epi& epi) {
   cplx* const smem = smem_cplx();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp >> 2) * 32, wn = ((warp + (DRIFT ? 2 * (warp >> 2) : 0)) & 3) * 16;
+  const int wm = (warp >> 2) * 16 * MI, wn = ((warp + (DRIFT ? 2 * (warp >> 2) : 0)) & 3) * 16;
   const int nk = (g.K + GT_K - 1) / GT_K;
   typedef typename std::conditional<OPA == OP_C, AIdxOpC, AIdxOp0>::type AI;
   typedef typename std::conditional<OPB == OP_C, BIdxOpC, BIdxOp0>::type BI;
@@ -291,6 +291,67 @@ NEGF_DEV void gemm_body(const GemmArgs& g, const Epi& epi) {
     return;
   }
 
+#ifdef NEGF_TEAM
+  // Output tiles of TM rows, dealt round the team.  The next slab to load: its tile, k offset, stage.
+  constexpr int TM = 32 * MI;
+  const int tn = (g.N + GT_N - 1) / GT_N, tiles = ((g.M + TM - 1) / TM) * tn;
+  int lt = team_rank(), lk = 0, lst = 0;
+  auto load_next = [&]() {
+    if (lt < tiles) {
+      load_a_tile<OPA, TM>(sA(lst), g, (lt / tn) * TM, lk, tid);
+      load_b_tile<OPB>(sB(lst), g, lk, (lt % tn) * GT_N, tid);
+      lst = lst + 1 == GT_STAGES ? 0 : lst + 1;
+      lk += GT_K;
+      if (lk >= g.K) { lk = 0; lt += team_size(); }
+    }
+    cp_async_commit();
+  };
+  __syncthreads();  // whatever used the ring's memory before is done with it
+  if (nk > 0) {
+#pragma unroll
+    for (int s = 0; s < GT_STAGES - 1; ++s) load_next();
+  }
+  cp_async_wait<GT_STAGES - 2>();
+  __syncthreads();
+  int st = 0;
+  for (int t = team_rank(); t < tiles; t += team_size()) {
+    const int m0 = (t / tn) * TM, n0 = (t % tn) * GT_N;
+    if (m0 + wm >= g.M || n0 + wn >= g.N) {  // no output in this warp's sub-tile: keep the ring going
+      for (int k0 = 0; k0 < g.K; k0 += GT_K) {
+        load_next();
+        cp_async_wait<GT_STAGES - 2>();
+        __syncthreads();
+        st = st + 1 == GT_STAGES ? 0 : st + 1;
+      }
+      continue;
+    }
+    Acc3M acc;
+    acc.zero();
+    for (int k0 = 0; k0 < g.K; k0 += GT_K) {
+      const cplx *a = sA(st), *b = sB(st);
+#pragma unroll
+      for (int ks = 0; ks < GT_K / 8 - 1; ++ks) {
+        Frag8 f;
+        frag8_load<CA, CB, G3, MI>(f, a, b, ks, wm, wn, lane, AI(), BI());
+        frag8_mma<G3, MI>(acc, f);
+      }
+      load_next();
+      Frag8 f;
+      frag8_load<CA, CB, G3, MI>(f, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
+      cp_async_wait<GT_STAGES - 2>();
+      __syncthreads();
+      frag8_mma<G3, MI>(acc, f);
+      st = st + 1 == GT_STAGES ? 0 : st + 1;
+    }
+    acc_foreach<G3, MI>(acc, wm, wn, lane, [&](int r, int c, cplx v) {
+      const int m = m0 + r, n = n0 + c;
+      if (m < g.M && n < g.N) epi(m, n, v);
+    });
+  }
+  cp_async_wait<0>();
+  team_sync();
+}
+#else
   // the next slab to load: its tile corner, k offset and ring stage
   int lm = 0, ln = 0, lk = 0, lst = 0;
   int left = ((g.M + GT_M - 1) / GT_M) * ((g.N + GT_N - 1) / GT_N) * nk;
@@ -348,35 +409,60 @@ NEGF_DEV void gemm_body(const GemmArgs& g, const Epi& epi) {
   cp_async_wait<0>();
   __syncthreads();
 }
+#endif
 
 // Whether the drifting form is the faster one for an M x N product of the sweep: the last row or
 // column of tiles leaves at least half of its warps without output (remainder 1 .. 32 of 64).
 NEGF_DEV bool gemm_ragged(int M, int N) { return ((M - 1) & (GT_M - 1)) < GT_M / 2 || ((N - 1) & (GT_N - 1)) < GT_N / 2; }
 
-// The compiled products.  Arguments go by reference: two non-inlined functions that take the
-// argument structs by value, called from the two arms of a branch, reached one of them with a
-// wrong copy (the checkpointed adjoint then recomputed wrong blocks).
-template <int OPA, int OPB, bool G3, bool DRIFT, class Epi>
-__device__ __noinline__ void cta_gemm_epi(const GemmArgs& gr, const Epi& er) {
+// The compiled products (arguments by reference: one copy per call instead of two).
+template <int OPA, int OPB, bool G3, bool DRIFT, int MI, class Epi>
+__device__ __noinline__ void cta_gemm_fn(const GemmArgs& gr, const Epi& er) {
   const GemmArgs g = gr;
   const Epi epi = er;
-  gemm_body<OPA, OPB, G3, DRIFT>(g, epi);
+  gemm_body<OPA, OPB, G3, DRIFT, MI>(g, epi);
 }
-template <int OPA, int OPB, bool G3, bool DRIFT>
+template <int OPA, int OPB, bool G3, bool DRIFT, int MI>
 __device__ __noinline__ void cta_gemm_std(const GemmArgs& gr) {
   const GemmArgs g = gr;
-  gemm_body<OPA, OPB, G3, DRIFT>(g, EpiStore{g});
+  gemm_body<OPA, OPB, G3, DRIFT, MI>(g, EpiStore{g});
+}
+
+#ifdef NEGF_TEAM
+// Tiles of 32 rows instead of 64 where they even out what the team's CTAs get: the longest share,
+// in units of 32-row tiles, is compared (a 64 x 64 product on two CTAs is one 32-row tile each).
+NEGF_DEV bool team_half_tiles(int M, int N) {
+  const int tn = (N + GT_N - 1) / GT_N, sz = team_size();
+  const int full = (((M + 63) / 64) * tn + sz - 1) / sz, half = (((M + 31) / 32) * tn + sz - 1) / sz;
+  return half < 2 * full;
+}
+#endif
+
+// The product with a caller's epilogue.
+template <int OPA, int OPB, bool G3, bool DRIFT, class Epi>
+NEGF_DEV void cta_gemm_epi(const GemmArgs& g, const Epi& e) {
+#ifdef NEGF_TEAM
+  if (team_half_tiles(g.M, g.N)) cta_gemm_fn<OPA, OPB, G3, true, 1>(g, e);
+  else cta_gemm_fn<OPA, OPB, G3, true, 2>(g, e);
+#else
+  cta_gemm_fn<OPA, OPB, G3, DRIFT, 2>(g, e);
+#endif
 }
 
 // C = alpha op(A) op(B) + beta D (D may alias C; C must not alias A or B).
 template <int OPA, int OPB, bool G3 = true>
 NEGF_DEV void cta_gemm(const GemmArgs& g) {
+#ifdef NEGF_TEAM
+  if (team_half_tiles(g.M, g.N)) cta_gemm_std<OPA, OPB, G3, true, 1>(g);
+  else cta_gemm_std<OPA, OPB, G3, true, 2>(g);
+#else
   if constexpr (G3) {
-    if (gemm_ragged(g.M, g.N)) cta_gemm_std<OPA, OPB, G3, true>(g);
-    else cta_gemm_std<OPA, OPB, G3, false>(g);
+    if (gemm_ragged(g.M, g.N)) cta_gemm_std<OPA, OPB, G3, true, 2>(g);
+    else cta_gemm_std<OPA, OPB, G3, false, 2>(g);
   } else {
-    cta_gemm_std<OPA, OPB, G3, true>(g);
+    cta_gemm_std<OPA, OPB, G3, true, 2>(g);
   }
+#endif
 }
 
-}  // namespace negf
+}  // namespace NEGF_NS

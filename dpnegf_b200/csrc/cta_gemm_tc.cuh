@@ -38,7 +38,7 @@
 #pragma once
 #include "cta_gemm.cuh"
 
-namespace negf {
+namespace NEGF_NS {
 
 constexpr int TC_M = 128, TC_N = 256, TC_KC = 8;
 constexpr int TC_PLANE_A = TC_M * TC_KC * 4;                   // bytes of one A plane
@@ -371,4 +371,4 @@ NEGF_DEV void cta_gemm_tc(const GemmArgs& g, char* smem) {
   cta_gemm_tc_epi<OPA, OPB>(g, smem, EpiStore{g});
 }
 
-}  // namespace negf
+}  // namespace NEGF_NS

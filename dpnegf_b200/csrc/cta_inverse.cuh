@@ -30,7 +30,7 @@
 #pragma once
 #include "cta_gemm_tc.cuh"
 
-namespace negf {
+namespace NEGF_NS {
 
 #ifndef NEGF_INV_SMALL_NB
 #define NEGF_INV_SMALL_NB 8
@@ -591,8 +591,8 @@ __device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, c
   }
   if (lost) flag[1] = 1;
   __syncthreads();
-  // G[i][j] = W[p(i)][p^-1(j)]
-  if (!flag[1]) {
+  // G[i][j] = W[p(i)][p^-1(j)] (every CTA of a team holds the same result; one stores it)
+  if (!flag[1] && team_rank() == 0) {
 #pragma unroll
     for (int a = 0; a < RA; ++a)
 #pragma unroll
@@ -603,7 +603,7 @@ __device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, c
   }
   const int f = flag[0] | flag[1];
   if (tid < NPAN) mbar_inval(bar + tid);
-  __syncthreads();
+  team_sync();
   return f;
 }
 
@@ -612,6 +612,19 @@ __device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, c
 // a multiple of 32 up to INV_OB_MAX (narrower blocks move work from the
 // panels' rank-NB updates to the outer GEMM; ob >= n leaves no outer update).
 // With ob < n the snapshot needs ob x n complex elements.
+template <bool G3 = true, bool TC = false>
+NEGF_DEV int cta_inverse_pivoted(cplx* W, int64_t ldw, int n, cplx* G, int64_t ldg, char* smem_raw, PhaseClock* pc,
+                                 cplx* snap, int ob) {
+  // Narrow panels for small blocks (the mixed block inverse's 64-wide leaves): a column step's
+  // latency chain is shorter (16-wide measured 22 % faster than 32-wide at n = 64, 8 % at
+  // n = 128, where the rank-16 updates start to cost more; 8-wide another 4-9 % for n <= 64).
+  // One register row per thread up to n = 256.
+  if (n > 64 && n <= 256) return cta_inverse_nb<32, 1, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
+  if constexpr (TC) {
+    if (n <= 64) return cta_inverse_nb<INV_SMALL_NB, 1, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
+  }
+  return cta_inverse_nb<16, 2, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
+}
 template <bool G3 = true, bool TC = false>
 NEGF_DEV int cta_inverse(cplx* W, int64_t ldw, int n, cplx* G, int64_t ldg, char* smem_raw, PhaseClock* pc,
                          cplx* snap, int ob = INV_OB) {
@@ -626,15 +639,11 @@ NEGF_DEV int cta_inverse(cplx* W, int64_t ldw, int n, cplx* G, int64_t ldg, char
       return f;
     }
   }
-  // Narrow panels for small blocks (the block inverse's 64-wide leaves): a column step's
-  // latency chain is shorter (16-wide measured 22 % faster than 32-wide at n = 64, 8 % at
-  // n = 128, where the rank-16 updates start to cost more; 8-wide another 4-9 % for n <= 64).
-  // One register row per thread up to n = 256.
-  if (n > 64 && n <= 256) return cta_inverse_nb<32, 1, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
-  if constexpr (TC) {
-    if (n <= 64) return cta_inverse_nb<INV_SMALL_NB, 1, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
-  }
-  return cta_inverse_nb<16, 2, G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
+#ifdef NEGF_TEAM
+  return 1;  // not reached: a team's larger blocks go through the block inverse or one CTA's pivoted form
+#else
+  return cta_inverse_pivoted<G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);
+#endif
 }
 
-}  // namespace negf
+}  // namespace NEGF_NS

@@ -4,25 +4,31 @@
 // form passes of the first kernel version were load-latency bound at
 // ~25 GB/s per SM).  Here every thread stages its elements of 2048-element
 // chunks with cp.async, two chunks in flight (128 KB per SM), and consumes
-// exactly the elements it staged, so no barrier is needed inside the loop.
+// exactly the elements it staged, so no barrier is needed inside the loop (the
+// reads are ordered behind the wait by lds_after_wait).
 #pragma once
 #include "negf_common.cuh"
 
-namespace negf {
+namespace NEGF_NS {
 
 constexpr int STREAM_CHUNK = 2048;
 constexpr int STREAM_SMEM_BYTES = 4 * STREAM_CHUNK * (int)sizeof(cplx);
 
 // out[e] = alpha * (X[e] - z * Y[e]) for e < count; a null X or Y is zero.
-// Ends with __syncthreads().
+// The chunks go round the team's CTAs.  Ends with team_sync().
+// The roundings of z Y are spelled out, so that results do not depend on how the compiler contracts
+// an instantiation: the products with Re z, the large ones, are fused into the sums.  The mixed sweep
+// amplifies every rounding of its inputs and keeps the imaginary part it has always had (MX).
+template <bool MX = false>
 NEGF_DEV void cta_shift_form(cplx* out, const cplx* X, const cplx* Y, cplx z, cplx alpha, int count,
                              cplx* smem) {
   const int tid = threadIdx.x;
   cplx* sx[2] = {smem, smem + STREAM_CHUNK};
   cplx* sy[2] = {smem + 2 * STREAM_CHUNK, smem + 3 * STREAM_CHUNK};
-  const int nch = (count + STREAM_CHUNK - 1) / STREAM_CHUNK;
+  const int all = (count + STREAM_CHUNK - 1) / STREAM_CHUNK;
+  const int nch = (all - team_rank() + team_size() - 1) / team_size();  // this CTA's chunks
   auto issue = [&](int c) {
-    const int base = c * STREAM_CHUNK;
+    const int base = (team_rank() + c * team_size()) * STREAM_CHUNK;
 #pragma unroll
     for (int s = 0; s < STREAM_CHUNK / 256; ++s) {
       const int k = tid + s * 256, e = base + k;
@@ -37,19 +43,21 @@ NEGF_DEV void cta_shift_form(cplx* out, const cplx* X, const cplx* Y, cplx z, cp
     if (c + 1 < nch) issue(c + 1);
     else cp_async_commit();
     cp_async_wait<1>();
-    const int base = c * STREAM_CHUNK;
+    const int base = (team_rank() + c * team_size()) * STREAM_CHUNK;
 #pragma unroll
     for (int s = 0; s < STREAM_CHUNK / 256; ++s) {
       const int k = tid + s * 256, e = base + k;
       if (e < count) {
-        cplx x = X ? sx[c & 1][k] : cmk(0.0, 0.0);
-        cplx y = Y ? sy[c & 1][k] : cmk(0.0, 0.0);
-        out[e] = cmul(alpha, csub(x, cmul(z, y)));
+        cplx x = X ? lds_after_wait(sx[c & 1] + k) : cmk(0.0, 0.0);
+        cplx y = Y ? lds_after_wait(sy[c & 1] + k) : cmk(0.0, 0.0);
+        const double re = __fma_rn(z.x, y.x, -__dmul_rn(z.y, y.y));
+        const double im = MX ? __fma_rn(z.y, y.x, __dmul_rn(z.x, y.y)) : __fma_rn(z.x, y.y, __dmul_rn(z.y, y.x));
+        out[e] = cmul(alpha, csub(x, cmk(re, im)));
       }
     }
   }
   cp_async_wait<0>();
-  __syncthreads();
+  team_sync();
 }
 
-}  // namespace negf
+}  // namespace NEGF_NS

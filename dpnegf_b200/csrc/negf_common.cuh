@@ -9,7 +9,53 @@
 
 #define NEGF_DEV __device__ __forceinline__
 
-namespace negf {
+// The CTA building blocks and the sweep compile twice: one CTA per work item (namespace negf), and,
+// with NEGF_TEAM, a thread-block cluster per item (namespace negf_team), whose CTAs split the output
+// tiles and the elementwise passes and repeat the small serial parts.
+#ifdef NEGF_TEAM
+#define NEGF_NS negf_team
+#else
+#define NEGF_NS negf
+#endif
+
+namespace NEGF_NS {
+
+constexpr int TEAM_THREADS_PER_CTA = 256;
+#ifdef NEGF_TEAM
+NEGF_DEV int team_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return (int)r;
+}
+NEGF_DEV int team_size() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(r));
+  return (int)r;
+}
+// Barrier over every thread of the team; global writes before it are visible to the team after it.
+NEGF_DEV void team_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// The 8 bytes at `p` (this CTA's shared memory) as CTA `rank` of the team has them.
+NEGF_DEV unsigned long long team_peek(const unsigned long long* p, int rank) {
+  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
+  unsigned long long v;
+  asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.u64 %0, [r];\n\t}\n"
+               : "=l"(v)
+               : "r"(a), "r"(rank)
+               : "memory");
+  return v;
+}
+#else
+NEGF_DEV constexpr int team_rank() { return 0; }
+NEGF_DEV constexpr int team_size() { return 1; }
+NEGF_DEV void team_sync() { __syncthreads(); }
+#endif
+NEGF_DEV int team_tid() { return team_rank() * TEAM_THREADS_PER_CTA + (int)threadIdx.x; }
+NEGF_DEV int team_threads() { return team_size() * TEAM_THREADS_PER_CTA; }
+NEGF_DEV int team_warp() { return team_tid() >> 5; }
+NEGF_DEV int team_warps() { return team_threads() >> 5; }
 
 typedef double2 cplx;
 
@@ -42,22 +88,35 @@ extern __shared__ __align__(1024) char negf_smem[];
 NEGF_DEV cplx* smem_cplx() { return reinterpret_cast<cplx*>(negf_smem); }
 
 // ---------------------------------------------------------------------------
-// cp.async (16-byte, L2-only) with zero fill when the source is out of range.
+// cp.async (16-byte, L2-only) with zero fill when the source is out of range.  The copy writes
+// shared memory behind the compiler's back: the memory clobbers here and on the wait keep reads of
+// the staged entries between them, also where a thread consumes its own copies without a barrier.
 NEGF_DEV void cp_async16(void* smem_dst, const void* gmem_src, bool valid) {
   unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
   int n = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem_src), "r"(n));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem_src), "r"(n) : "memory");
 }
 // Global load that the compiler may not sink below later volatile asm (the
 // DMMAs): used to put a read-modify-write's reads in flight before the math.
 NEGF_DEV cplx ldg_early(const cplx* p) {
   cplx v;
-  asm volatile("ld.global.cg.v2.f64 {%0,%1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  asm volatile("ld.global.cg.v2.f64 {%0,%1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
   return v;
 }
-NEGF_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+// Shared-memory read that stays behind the wait for a copy of the same thread.  A plain load is not
+// ordered against cp.async.wait_group without a barrier in between: some instantiations of the sweep
+// read the streamed entries before they had arrived.
+NEGF_DEV cplx lds_after_wait(const cplx* p) {
+  cplx v;
+  asm volatile("ld.shared.v2.f64 {%0,%1}, [%2];\n"
+               : "=d"(v.x), "=d"(v.y)
+               : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p)))
+               : "memory");
+  return v;
+}
+NEGF_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
-NEGF_DEV void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+NEGF_DEV void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // ---------------------------------------------------------------------------
 // FP64 tensor-core MMA, D(8x8) += A(8x4, row) * B(4x8, col).
@@ -107,4 +166,4 @@ struct PhaseClock {
   }
 };
 
-}  // namespace negf
+}  // namespace NEGF_NS

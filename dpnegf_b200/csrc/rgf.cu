@@ -2,7 +2,26 @@
 // in rgf_sweep.cuh, the mixed-precision kernel in rgf_mx.cu.
 #include "rgf_sweep.cuh"
 
+namespace negf_team {
+int rgf_launch_team(int feat, const NegfRgfProblem& p, size_t smem, int slots, int cl, cudaStream_t s);
+int rgf_team_fit(int feat, size_t smem, int cl);
+}
+
 namespace negf {
+
+// CTAs per work slot.  A launch with fewer slots than half the SMs leaves the others idle, so each
+// item gets a cluster of 2, 4 or 8 CTAs while all slots still run at once and the block products
+// have a 32 x 64 output piece for every CTA.
+static int team_ctas(int feat, const NegfRgfProblem& p, size_t smem, int slots) {
+  int dev = 0, sms = 0;
+  if (p.max_n <= 32 || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  const int pieces = ((p.max_n + 31) / 32) * ((p.max_n + 63) / 64);
+  for (int cl = 8; cl > 1; cl /= 2)
+    if (cl <= pieces && slots * cl <= sms && negf_team::rgf_team_fit(feat, smem, cl) >= slots) return cl;
+  return 1;
+}
 
 int rgf_launch_fp64(int feat, const NegfRgfProblem& p, size_t smem, int grid, cudaStream_t s) {
   if (feat == FEAT_ADJOINT) return rgf_launch_impl<false, FEAT_ADJOINT>(p, smem, grid, s);
@@ -59,7 +78,11 @@ int negf_rgf_run(const NegfRgfProblem* p, void* stream) {
                    : (p->flags & (NEGF_LESSER | NEGF_GREATER)) ? negf::FEAT_LESSER : negf::FEAT_RETARDED;
   if (cudaMemsetAsync(p->scratch, 0, negf::RGF_SCRATCH_HEADER, s) != cudaSuccess) return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
-  if (!mixed) return negf::rgf_launch_fp64(feat, *p, smem, grid, s);
+  if (!mixed) {
+    const int cl = negf::team_ctas(feat, *p, smem, grid);
+    if (cl > 1) return negf_team::rgf_launch_team(feat, *p, smem, grid, cl, s);
+    return negf::rgf_launch_fp64(feat, *p, smem, grid, s);
+  }
   return negf::rgf_launch_mx(*p, smem, grid, s);  // one mixed instantiation with every feature
 }
 

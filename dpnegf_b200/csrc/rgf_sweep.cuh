@@ -36,7 +36,7 @@
 #include "cta_inverse.cuh"
 #include "cta_stream.cuh"
 
-namespace negf {
+namespace NEGF_NS {
 
 constexpr int RGF_NBUF = 18;  // per-slot max_n^2 work buffers (see SlotBufs)
 
@@ -117,29 +117,31 @@ NEGF_DEV SlotBufs slot_bufs(const NegfRgfProblem& p, int slot) {
 }
 
 // Out = X - z Y  ([m x n]); a missing X or Y (offset -1) is a zero block.
+template <bool MX>
 NEGF_DEV void form_shift(cplx* out, const cplx* hs, int64_t ox, int64_t oy, cplx z, int m, int n, cplx* smem) {
-  cta_shift_form(out, ox >= 0 ? hs + ox : nullptr, oy >= 0 ? hs + oy : nullptr, z, cmk(1.0, 0.0), m * n, smem);
+  cta_shift_form<MX>(out, ox >= 0 ? hs + ox : nullptr, oy >= 0 ? hs + oy : nullptr, z, cmk(1.0, 0.0), m * n, smem);
 }
 
 // W = z S - H - (Sigma_L in the top-left corner) - (Sigma_R in the bottom-right
 // corner); the corner rule is recursive_green_cal.py:411-428.
+template <bool MX>
 NEGF_DEV void form_a0(cplx* W, const cplx* hs, const NegfBlock& b, cplx z, const cplx* seL, int nsl,
                       const cplx* seR, int nsr, cplx* smem) {
-  const int n = b.n, tid = threadIdx.x;
-  cta_shift_form(W, hs + b.hd, hs + b.sd, z, cmk(-1.0, 0.0), n * n, smem);
+  const int n = b.n, tid = team_tid();
+  cta_shift_form<MX>(W, hs + b.hd, hs + b.sd, z, cmk(-1.0, 0.0), n * n, smem);
   const int cl = seL ? min(n, nsl) : 0;
   const int cr = seR ? min(n, nsr) : 0;
-  for (int e = tid; e < cl * cl; e += CTA_THREADS) {
+  for (int e = tid; e < cl * cl; e += team_threads()) {
     int i = e / cl, j = e % cl;
     W[(int64_t)i * n + j] = csub(W[(int64_t)i * n + j], seL[(int64_t)i * nsl + j]);
   }
-  __syncthreads();  // a block can carry both corners (K = 1)
-  for (int e = tid; e < cr * cr; e += CTA_THREADS) {
+  team_sync();  // a block can carry both corners (K = 1)
+  for (int e = tid; e < cr * cr; e += team_threads()) {
     int i = e / cr, j = e % cr;
     int64_t w = (int64_t)(n - cr + i) * n + (n - cr + j);
     W[w] = csub(W[w], seR[(int64_t)(nsr - cr + i) * nsr + (nsr - cr + j)]);
   }
-  __syncthreads();
+  team_sync();
 }
 
 NEGF_DEV void copy_mat(cplx* dst, const cplx* src, int m, int n, cplx* smem) {
@@ -151,8 +153,8 @@ NEGF_DEV void copy_mat(cplx* dst, const cplx* src, int m, int n, cplx* smem) {
 // the row values are also summed into dsum (lane 0 of each warp).
 NEGF_DEV void diag_im_acc(double* dst, double& dsum, const cplx* A, const cplx* BT, int rows, int inner,
                           bool init) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = warp; i < rows; i += CTA_THREADS / 32) {
+  const int lane = threadIdx.x & 31, warp = team_warp();
+  for (int i = warp; i < rows; i += team_warps()) {
     double acc = 0.0;
 #pragma unroll 4
     for (int j = lane; j < inner; j += 32) {
@@ -171,7 +173,7 @@ NEGF_DEV void diag_im_acc(double* dst, double& dsum, const cplx* A, const cplx* 
 
 // Gamma = i (Sigma - Sigma^H) on the c x c corner of Sigma (ns x ns) at (r0, r0).
 NEGF_DEV void form_gamma(cplx* out, const cplx* se, int ns, int r0, int c) {
-  for (int e = threadIdx.x; e < c * c; e += CTA_THREADS) {
+  for (int e = team_tid(); e < c * c; e += team_threads()) {
     int i = e / c, k = e % c;
     cplx a = se[(int64_t)(r0 + i) * ns + r0 + k], b = se[(int64_t)(r0 + k) * ns + r0 + i];
     cplx d = csub(a, cconj(b));
@@ -204,6 +206,38 @@ NEGF_DEV double cta_sum(double v, double* red) {
   __syncthreads();
   return s;
 }
+
+#ifdef NEGF_TEAM
+static __shared__ unsigned long long team_slot;  // what the team's other CTAs may read of this one
+
+// v of every CTA's thread 0, folded in rank order by every thread: each sees the same bits.
+template <class F>
+NEGF_DEV double team_fold(double v, F f) {
+  if (threadIdx.x == 0) team_slot = (unsigned long long)__double_as_longlong(v);
+  team_sync();
+  double s = __longlong_as_double((long long)team_peek(&team_slot, 0));
+  for (int r = 1; r < team_size(); ++r) s = f(s, __longlong_as_double((long long)team_peek(&team_slot, r)));
+  team_sync();
+  return s;
+}
+NEGF_DEV double team_max(double v, double* red) {
+  return team_fold(cta_max(v, red), [](double x, double y) { return fmax(x, y); });
+}
+NEGF_DEV double team_sum(double v, double* red) {
+  return team_fold(cta_sum(v, red), [](double x, double y) { return x + y; });
+}
+// rank 0's value of v (uniform in that CTA)
+NEGF_DEV int team_from_first(int v) {
+  if (threadIdx.x == 0) team_slot = (unsigned long long)(unsigned)v;
+  team_sync();
+  const int f = (int)(unsigned)team_peek(&team_slot, 0);
+  team_sync();
+  return f;
+}
+#else
+NEGF_DEV double team_max(double v, double* red) { return cta_max(v, red); }
+NEGF_DEV double team_sum(double v, double* red) { return cta_sum(v, red); }
+#endif
 
 // C = alpha op(A) op(B) (+ beta D) on the FP64 DMMA GEMM, or on the tcgen05
 // 3xTF32 GEMM when MX.
@@ -257,11 +291,11 @@ __device__ __noinline__ int cta_inverse_blk(cplx* W, int64_t ldw, int n, cplx* G
     gemm<OP_N, OP_N, MX>(smem, h, m, m, W11, ldw, G22, ldg, G12, ldg, MONE);                  // G12 = -T Y
     gemm<OP_N, OP_N, MX>(smem, h, h, m, G12, ldg, G21, ldg, G11, ldg, MONE, G11, ldg);       // X + T Y U
     gemm<OP_N, OP_N, MX>(smem, m, h, m, G22, ldg, G21, ldg, W21, ldw, MONE);                  // -Y U
-    for (int e = threadIdx.x; e < m * h; e += CTA_THREADS) {
+    for (int e = team_tid(); e < m * h; e += team_threads()) {
       const int i = e / h, j = e % h;
       G21[(int64_t)i * ldg + j] = W21[(int64_t)i * ldw + j];
     }
-    __syncthreads();
+    team_sync();
     pc.mark(PH_INV_UPDATE);
     (void)ONE;
     return bad;
@@ -273,14 +307,15 @@ __device__ __noinline__ int cta_inverse_blk(cplx* W, int64_t ldw, int n, cplx* G
 // r = A y - v; true when max|r| <= tol n max|A| max|y| (a backward-stable
 // inverse leaves about n u there) and everything is finite.  Whole CTA (the
 // decision is uniform); y lives in smem.
-NEGF_DEV bool inv_probe(const cplx* A, const cplx* G, int n, double tol, cplx* smem, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// A team shares the rows: y goes through yg (n elements of global memory, else unused).
+NEGF_DEV bool inv_probe(const cplx* A, const cplx* G, int n, double tol, cplx* smem, double* red, cplx* yg) {
+  const int lane = threadIdx.x & 31, warp = team_warp();
   auto v = [](int j) {
     const unsigned h = (unsigned)(j + 1) * 2654435761u;
     return cmk((h & 0x10000u) ? 1.0 : -1.0, (h & 0x20000u) ? 1.0 : -1.0);
   };
   cplx* y = smem;
-  for (int i = warp; i < n; i += CTA_THREADS / 32) {
+  for (int i = warp; i < n; i += team_warps()) {
     cplx acc = cmk(0.0, 0.0);
     for (int j = lane; j < n; j += 32) acc = cfma(G[(int64_t)i * n + j], v(j), acc);
 #pragma unroll
@@ -288,11 +323,19 @@ NEGF_DEV bool inv_probe(const cplx* A, const cplx* G, int n, double tol, cplx* s
       acc.x += __shfl_xor_sync(0xffffffffu, acc.x, off);
       acc.y += __shfl_xor_sync(0xffffffffu, acc.y, off);
     }
+#ifdef NEGF_TEAM
+    if (lane == 0) yg[i] = acc;
+  }
+  team_sync();
+  for (int i = threadIdx.x; i < n; i += CTA_THREADS) y[i] = yg[i];
+  __syncthreads();
+#else
     if (lane == 0) y[i] = acc;
   }
   __syncthreads();
+#endif
   double rmax = 0.0, amax = 0.0, ymax = 0.0;
-  for (int i = warp; i < n; i += CTA_THREADS / 32) {
+  for (int i = warp; i < n; i += team_warps()) {
     cplx acc = cmk(0.0, 0.0);
     double am = 0.0;
     for (int j = lane; j < n; j += 32) {
@@ -311,9 +354,9 @@ NEGF_DEV bool inv_probe(const cplx* A, const cplx* G, int n, double tol, cplx* s
     amax = fmax(amax, am);
     ymax = fmax(ymax, cabs1(y[i]));
   }
-  rmax = cta_max(rmax, red);
-  amax = cta_max(amax, red);
-  ymax = cta_max(ymax, red);
+  rmax = team_max(rmax, red);
+  amax = team_max(amax, red);
+  ymax = team_max(ymax, red);
   return rmax <= tol * (double)n * amax * ymax;
 }
 
@@ -368,20 +411,20 @@ NEGF_DEV int forward_block_body(const NegfRgfProblem& P, const NegfItem& it, con
   int bad = 0;
   const NegfBlock& b = blk[q];
   const int nq = b.n;
-  form_a0(sb.W, hs, b, z, q == 0 ? seL : nullptr, it.nse_l, q == K - 1 ? seR : nullptr, it.nse_r, smem);
+  form_a0<MX>(sb.W, hs, b, z, q == 0 ? seL : nullptr, it.nse_l, q == K - 1 ? seR : nullptr, it.nse_r, smem);
   if (q > 0) {
     const NegfBlock& bp = blk[q - 1];
     const int np = bp.n;
-    form_shift(sb.Lz, hs, bp.hl, bp.sl, z, nq, np, smem);  // L_{q-1}: n_q x n_{q-1}
-    form_shift(sb.Uz, hs, bp.hu, bp.su, z, np, nq, smem);  // U_{q-1}: n_{q-1} x n_q
-    __syncthreads();
+    form_shift<MX>(sb.Lz, hs, bp.hl, bp.sl, z, nq, np, smem);  // L_{q-1}: n_q x n_{q-1}
+    form_shift<MX>(sb.Uz, hs, bp.hu, bp.su, z, np, nq, smem);  // U_{q-1}: n_{q-1} x n_q
+    team_sync();
     pc.mark(PH_FORM);
     cplx* t1 = !MX && lg ? lg : sb.T1;
     gemm<OP_N, OP_N, MX>(smem, nq, np, np, sb.Lz, np, gprev, np, t1, np);
     gemm<OP_N, OP_N, MX>(smem, nq, nq, np, t1, np, sb.Uz, nq, sb.W, nq, MONE, sb.W, nq);
     pc.mark(PH_GEMM_FWD);
   } else {
-    __syncthreads();
+    team_sync();
     pc.mark(PH_FORM);
   }
   bool gj = P.inv_mode != 1;
@@ -389,16 +432,29 @@ NEGF_DEV int forward_block_body(const NegfRgfProblem& P, const NegfItem& it, con
     // block inverse on a copy of W; a failed residual probe (or a singular leaf) falls
     // back to the pivoted Gauss-Jordan on the saved W
     copy_mat(sb.tD, sb.W, nq, nq, smem);
-    const int bb = cta_inverse_blk<3, MX>(sb.W, nq, nq, gq, nq, smem, pc, sb.tE);
-    if (bb || !inv_probe(sb.tD, gq, nq, MX ? 1e-4 : 1e-10, smem, red)) {
+    int bb = cta_inverse_blk<3, MX>(sb.W, nq, nq, gq, nq, smem, pc, sb.tE);
+#ifdef NEGF_TEAM
+    bb = team_max((double)bb, red) != 0.0;  // one decision for the team, whatever a CTA met
+#endif
+    if (bb || !inv_probe(sb.tD, gq, nq, MX ? 1e-4 : 1e-10, smem, red, sb.tE)) {
       copy_mat(sb.W, sb.tD, nq, nq, smem);
       gj = true;
     }
     pc.mark(PH_INV_GATHER);
   }
+#ifdef NEGF_TEAM
+  if (gj && nq > 64) {  // the pivoted form works in place on one CTA; one outer block, so it calls no team product
+    int f = 0;
+    if (team_rank() == 0) f = cta_inverse_pivoted<true, MX>(sb.W, nq, nq, gq, nq, smem_raw, &pc, sb.tE, INV_OB_MAX);
+    bad |= team_from_first(f);
+  } else if (gj) {
+    bad |= cta_inverse<true, MX>(sb.W, nq, nq, gq, nq, smem_raw, &pc, sb.tE, INV_OB_MAX);
+  }
+#else
   if (gj)
     bad |= cta_inverse<true, MX>(sb.W, nq, nq, gq, nq, smem_raw, &pc, sb.tE,  // tE: pivot-row snapshot
                                  P.inv_ob > 0 ? P.inv_ob : INV_OB);
+#endif
   if (dgq) {
     // dg_q/dz = -g_q Kd g_q with Kd = S_q - (L dg_{q-1} - sl g_{q-1}) U + (L g_{q-1}) su
     // (d/dz of g_q^-1 = zS_q - H_q - Sigma - L g U, dL/dz = -sl, dU/dz = -su; sb.T1 = L g_{q-1})
@@ -461,7 +517,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
   cplx *gHd = nullptr, *gSd = nullptr, *gHu = nullptr, *gSu = nullptr, *gHl = nullptr, *gSl = nullptr;
   if (adj) {
     const int64_t u_slab = (P.grad_slab - 2 * dv.g_slab) / 4;
-    cplx* gslot = reinterpret_cast<cplx*>(P.grad) + (size_t)blockIdx.x * P.grad_slab;
+    cplx* gslot = reinterpret_cast<cplx*>(P.grad) + (size_t)(blockIdx.x / team_size()) * P.grad_slab;
     gHd = gslot;
     gSd = gslot + dv.g_slab;
     gHu = gslot + 2 * dv.g_slab;
@@ -471,9 +527,9 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     // the per-item self-energy gradients are sums of the T and density terms
     cplx* gl = reinterpret_cast<cplx*>(it.gse_l);
     cplx* gr = reinterpret_cast<cplx*>(it.gse_r);
-    if (gl) for (int e = threadIdx.x; e < it.nse_l * it.nse_l; e += CTA_THREADS) gl[e] = cmk(0.0, 0.0);
-    if (gr) for (int e = threadIdx.x; e < it.nse_r * it.nse_r; e += CTA_THREADS) gr[e] = cmk(0.0, 0.0);
-    __syncthreads();
+    if (gl) for (int e = team_tid(); e < it.nse_l * it.nse_l; e += team_threads()) gl[e] = cmk(0.0, 0.0);
+    if (gr) for (int e = team_tid(); e < it.nse_r * it.nse_r; e += team_threads()) gr[e] = cmk(0.0, 0.0);
+    team_sync();
   }
   // Density-gradient weight: DOS = -(2/pi) Im Tr[G S], and with Y = G S G = -dG/dz the
   // torch-convention gradients of w_d DOS are i c conj(Y_qp)^T for H and Sigma and
@@ -482,7 +538,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
   const cplx zc_d = cconj(z);
   // gradient block [r x s] += from the tangent Yd = dG/dz and G, both stored [s x r]
   auto acc_hs = [&](cplx* gH, cplx* gS, const cplx* Yd, const cplx* Gm, int r, int s_) {
-    for (int e = threadIdx.x; e < r * s_; e += CTA_THREADS) {
+    for (int e = team_tid(); e < r * s_; e += team_threads()) {
       const int i = e / s_, j = e % s_;
       const cplx y = cconj(Yd[(int64_t)j * r + i]), gg = cconj(Gm[(int64_t)j * r + i]);
       gH[e] = cadd(gH[e], cmk(cd * y.y, -cd * y.x));  // -i c y
@@ -493,7 +549,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
   // self-energy corner [c x c] at (os, os) of gse (ns x ns) from Yd (n x n) at (oy, oy)
   auto acc_se = [&](double* gse_raw, int ns, int os, const cplx* Yd, int n, int oy, int c) {
     cplx* gse = reinterpret_cast<cplx*>(gse_raw);
-    for (int e = threadIdx.x; e < c * c; e += CTA_THREADS) {
+    for (int e = team_tid(); e < c * c; e += team_threads()) {
       const int i = e / c, j = e % c;
       const cplx y = cconj(Yd[(int64_t)(oy + j) * n + oy + i]);
       cplx* d = gse + (int64_t)(os + i) * ns + os + j;
@@ -546,8 +602,8 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
         else gemm<OP_N, OP_N, MX>(smem, nq, nq, np, sb.T1, np, sb.Uz, nq, sb.tA, nq);
       } else {
         if (s) copy_mat(sb.tA, s, nq, nq, smem);
-        else for (int e = threadIdx.x; e < nq * nq; e += CTA_THREADS) sb.tA[e] = cmk(0.0, 0.0);
-        __syncthreads();
+        else for (int e = team_tid(); e < nq * nq; e += team_threads()) sb.tA[e] = cmk(0.0, 0.0);
+        team_sync();
       }
       gemm<OP_N, OP_N, MX>(smem, nq, nq, nq, gptr(q), nq, sb.tA, nq, sb.tB, nq);
       gemm<OP_N, OP_C, MX>(smem, nq, nq, nq, sb.tB, nq, gptr(q), nq, ginptr(q), nq);
@@ -563,8 +619,8 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
         else gemm<OP_N, OP_K, MX>(smem, nq, nq, np, sb.T1, np, sb.Uz, nq, sb.tA, nq);
       } else {
         if (s) copy_mat(sb.tA, s, nq, nq, smem);
-        else for (int e = threadIdx.x; e < nq * nq; e += CTA_THREADS) sb.tA[e] = cmk(0.0, 0.0);
-        __syncthreads();
+        else for (int e = team_tid(); e < nq * nq; e += team_threads()) sb.tA[e] = cmk(0.0, 0.0);
+        team_sync();
       }
       gemm<OP_N, OP_N, MX>(smem, nq, nq, nq, gptr(q), nq, sb.tA, nq, sb.tB, nq);
       gemm<OP_N, OP_K, MX>(smem, nq, nq, nq, sb.tB, nq, gptr(q), nq, gipptr(q), nq);
@@ -581,8 +637,8 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
   // diag(G_qN Gamma_R G_qN^H) of block q from gt = G_qN (nq x nN); Gamma_R corner in sb.Nu
   auto spectral_diag = [&](double* dst, const cplx* gtq, int nq) {
     gemm<OP_N, OP_N, MX>(smem, nq, crA, crA, gtq + (nN - crA), nN, sb.Nu, crA, sb.W, crA);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = warp; i < nq; i += CTA_THREADS / 32) {
+    const int lane = threadIdx.x & 31, warp = team_warp();
+    for (int i = warp; i < nq; i += team_warps()) {
       double acc = 0.0;
       for (int l = lane; l < crA; l += 32) {
         cplx y = sb.W[(int64_t)i * crA + l], g = gtq[(int64_t)i * nN + (nN - crA) + l];
@@ -592,10 +648,10 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
       if (lane == 0) dst[i] = acc;
     }
-    __syncthreads();
+    team_sync();
   };
   auto gdiag = [&](cplx* dst, const cplx* G, int nq) {
-    for (int i = threadIdx.x; i < nq; i += CTA_THREADS) dst[i] = G[(int64_t)i * nq + i];
+    for (int i = team_tid(); i < nq; i += team_threads()) dst[i] = G[(int64_t)i * nq + i];
   };
   const bool want_dos = (fl & (NEGF_ORB_DOS | NEGF_DOS)) != 0;
   double* orb = (fl & NEGF_ORB_DOS) ? P.orb_dos + it.orb : nullptr;
@@ -631,17 +687,17 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       Pnext = d;
     }
   }
-  __syncthreads();
+  team_sync();
   pc.mark(PH_FORM);
   if (want_dos) {
     diag_im_acc(orb ? orb + blk[K - 1].orb0 : nullptr, dsum, gptr(K - 1), hs + blk[K - 1].sdT, nN, nN, true);
-    __syncthreads();
+    team_sync();
     pc.mark(PH_DOS);
   }
   if (orbg) gdiag(orbg + blk[K - 1].orb0, gptr(K - 1), nN);
   if (orbar) {
     form_gamma(sb.Nu, seR, it.nse_r, it.nse_r - crA, crA);
-    __syncthreads();
+    team_sync();
     spectral_diag(orbar + blk[K - 1].orb0, gt, nN);
   }
   const cplx* Dnext = nullptr;  // dG_{q+1,q+1}/dz
@@ -653,7 +709,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       const int crd = min(nN, it.nse_r);
       acc_se(it.gse_r, it.nse_r, it.nse_r - crd, Dnext, nN, nN - crd, crd);
     }
-    __syncthreads();
+    team_sync();
   }
   int tog = 0;
   int seg_lo = ck ? ((K - 1) / ck) * ck : 0;  // checkpoint of the segment whose g_q are in the slab
@@ -679,9 +735,9 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     const int nq = b.n, nn = b.n_next;
     const int64_t szu = (int64_t)nq * nn;
     const bool need_gru = MX || lesser || greater || dosg || (fl & NEGF_OUT_GRU) != 0 || (want_dos && b.slT >= 0);
-    if (need_G && !keep_lg) form_shift(sb.Lz, hs, b.hl, b.sl, z, nn, nq, smem);  // L_q: n_{q+1} x n_q
-    form_shift(sb.Uz, hs, b.hu, b.su, z, nq, nn, smem);  // U_q: n_q x n_{q+1}
-    __syncthreads();
+    if (need_G && !keep_lg) form_shift<MX>(sb.Lz, hs, b.hl, b.sl, z, nn, nq, smem);  // L_q: n_{q+1} x n_q
+    form_shift<MX>(sb.Uz, hs, b.hu, b.su, z, nq, nn, smem);  // U_q: n_q x n_{q+1}
+    team_sync();
     pc.mark(PH_FORM);
     const cplx* g = gptr(q);
     cplx* grl = (fl & NEGF_OUT_GRL) ? out + b.o_grl + row * szu : sb.Gl;
@@ -724,7 +780,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       acc_hs(gHd + b.g, gSd + b.g, Dcur, grd, nq, nq);         // (q, q)
       acc_hs(gHu + b.gu, gSu + b.gu, sb.tC, grl, nq, nn);      // (q, q+1): Y_{q+1,q}, G_{q+1,q}
       acc_hs(gHl + b.gu, gSl + b.gu, sb.tD, gru, nn, nq);      // (q+1, q): Y_{q,q+1}, G_{q,q+1}
-      __syncthreads();
+      team_sync();
       Dnext = Dcur;
       dtog ^= 1;
     }
@@ -748,12 +804,12 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       gemm<OP_N, OP_N, MX>(smem, nq, nq, nq, sb.tE, nq, gin, nq, gnd, nq, ONE, sb.tC, nq);
       if (b.o_gnu >= 0) {
         cplx* gnu = out + b.o_gnu + row * szu;
-        for (int e = threadIdx.x; e < nq * nn; e += CTA_THREADS) {
+        for (int e = team_tid(); e < nq * nn; e += team_threads()) {
           int i = e / nn, j = e % nn;  // gnu[i][j] = conj(gnl[j][i])
           gnu[e] = cconj(gnl[(int64_t)j * nq + i]);
         }
       }
-      __syncthreads();
+      team_sync();
       Nnext = gnd;
       pc.mark(PH_LESSER);
     }
@@ -774,25 +830,25 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       gemm<OP_N, OP_N, MX>(smem, nq, nq, nq, sb.tE, nq, gip, nq, gpd, nq, ONE, sb.tC, nq);
       if (b.o_gpu >= 0) {
         cplx* gpu = out + b.o_gpu + row * szu;
-        for (int e = threadIdx.x; e < nq * nn; e += CTA_THREADS) {
+        for (int e = team_tid(); e < nq * nn; e += team_threads()) {
           int i = e / nn, j = e % nn;  // gpu[i][j] = conj(gpl[j][i])
           gpu[e] = cconj(gpl[(int64_t)j * nq + i]);
         }
       }
-      __syncthreads();
+      team_sync();
       Pnext = gpd;
       pc.mark(PH_LESSER);
     }
     if (want_dos) {
       diag_im_acc(orb ? orb + b.orb0 : nullptr, dsum, grd, hs + b.sdT, nq, nq, true);
-      __syncthreads();
+      team_sync();
       if (b.slT >= 0) {
         diag_im_acc(orb ? orb + b.orb0 : nullptr, dsum, gru, hs + b.slT, nq, nn, false);
-        __syncthreads();
+        team_sync();
       }
       if (b.suT >= 0) {
         diag_im_acc(orb ? orb + blk[q + 1].orb0 : nullptr, dsum, grl, hs + b.suT, nn, nq, false);
-        __syncthreads();
+        team_sync();
       }
       pc.mark(PH_DOS);
     }
@@ -800,15 +856,15 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
   }
   if (dosg && seL && it.gse_l) {  // Dnext = dG_11/dz
     acc_se(it.gse_l, it.nse_l, 0, Dnext, blk[0].n, 0, min(blk[0].n, it.nse_l));
-    __syncthreads();
+    team_sync();
   }
   if (fl & NEGF_OUT_GTRANS) {
     cplx* d = out + dv.o_gtrans + row * (int64_t)blk[0].n * nN;
     copy_mat(d, gt, blk[0].n, nN, smem);
-    __syncthreads();
+    team_sync();
   }
   double dos_total = 0.0;
-  if (fl & NEGF_DOS) dos_total = 2.0 * cta_sum(dsum, red);
+  if (fl & NEGF_DOS) dos_total = 2.0 * team_sum(dsum, red);
   pc.mark(PH_DOS);
 
   // ------------------------------------------------------------ refinement
@@ -829,28 +885,28 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     };
     if (!(fl & NEGF_OUT_GR_LC)) copy_mat(colx(K - 1), gptr(K - 1), nN, nN, smem);  // X_N apart from g_N
     auto add_into = [&](cplx* x, const cplx* d, int64_t cnt) {
-      for (int64_t e = threadIdx.x; e < cnt; e += CTA_THREADS) x[e] = cadd(x[e], d[e]);
-      __syncthreads();
+      for (int64_t e = team_tid(); e < cnt; e += team_threads()) x[e] = cadd(x[e], d[e]);
+      team_sync();
     };
     for (int step = 0; step < steps; ++step) {
       for (int q = 0; q < K; ++q) {
         const NegfBlock& b = blk[q];
         const int nq = b.n;
         cplx* yq = sb.yslab + b.gc;
-        form_a0(sb.W, hs, b, z, q == 0 ? seL : nullptr, it.nse_l, q == K - 1 ? seR : nullptr, it.nse_r, smem);
+        form_a0<MX>(sb.W, hs, b, z, q == 0 ? seL : nullptr, it.nse_l, q == K - 1 ? seR : nullptr, it.nse_r, smem);
         gemm<OP_N, OP_N, false>(smem, nq, nN, nq, sb.W, nq, colx(q), nN, yq, nN, MONE);  // -A_qq X_q
         if (q == K - 1) {
-          for (int i = threadIdx.x; i < nN; i += CTA_THREADS) yq[(int64_t)i * nN + i].x += 1.0;
-          __syncthreads();
+          for (int i = team_tid(); i < nN; i += team_threads()) yq[(int64_t)i * nN + i].x += 1.0;
+          team_sync();
         }
         if (q > 0) {
           const int np = blk[q - 1].n;
-          form_shift(sb.Lz, hs, blk[q - 1].hl, blk[q - 1].sl, z, nq, np, smem);
+          form_shift<MX>(sb.Lz, hs, blk[q - 1].hl, blk[q - 1].sl, z, nq, np, smem);
           gemm<OP_N, OP_N, false>(smem, nq, nN, np, sb.Lz, np, colx(q - 1), nN, yq, nN, ONE, yq, nN);
         }
         if (q < K - 1) {
           const int nn = b.n_next;
-          form_shift(sb.Uz, hs, b.hu, b.su, z, nq, nn, smem);
+          form_shift<MX>(sb.Uz, hs, b.hu, b.su, z, nq, nn, smem);
           gemm<OP_N, OP_N, false>(smem, nq, nN, nn, sb.Uz, nn, colx(q + 1), nN, yq, nN, ONE, yq, nN);
         }
         if (q > 0) {
@@ -866,7 +922,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       for (int q = K - 2; q >= 0; --q) {
         const NegfBlock& b = blk[q];
         const int nq = b.n, nn = b.n_next;
-        form_shift(sb.Uz, hs, b.hu, b.su, z, nq, nn, smem);
+        form_shift<MX>(sb.Uz, hs, b.hu, b.su, z, nq, nn, smem);
         gemm<OP_N, OP_N, MX>(smem, nq, nN, nn, sb.Uz, nn, dx, nN, sb.T1, nN, ONE, sb.yslab + b.gc, nN);
         gemm<OP_N, OP_N, MX>(smem, nq, nN, nq, gptr(q), nq, sb.T1, nN, dn, nN);
         add_into(colx(q), dn, (int64_t)nq * nN);
@@ -875,12 +931,12 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
       if (step + 1 < steps) {  // dx holds dX_0
         const cplx* x0 = colx(0);
         double dmax = 0.0, xmax = 0.0;
-        for (int64_t e = threadIdx.x; e < (int64_t)blk[0].n * nN; e += CTA_THREADS) {
+        for (int64_t e = team_tid(); e < (int64_t)blk[0].n * nN; e += team_threads()) {
           dmax = fmax(dmax, cabs1(dx[e]));
           xmax = fmax(xmax, cabs1(x0[e]));
         }
-        dmax = cta_max(dmax, red);
-        xmax = cta_max(xmax, red);
+        dmax = team_max(dmax, red);
+        xmax = team_max(xmax, red);
         if (!(dmax > REFINE_TOL * xmax)) break;  // uniform: every thread sees the same maxima
       }
     }
@@ -896,18 +952,18 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     const cplx* Gc = gt + (nN - cr);  // G_1N[0:cl, nN-cr:nN], row stride nN
     form_gamma(sb.tA, seL, it.nse_l, 0, cl);
     form_gamma(sb.tB, seR, it.nse_r, it.nse_r - cr, cr);
-    __syncthreads();
+    team_sync();
     // FP64 on both paths: per energy (not per block), and the mixed path's
     // refined G_1N must not meet FP32-level products here
     gemm<OP_N, OP_N, false>(smem, cl, cr, cl, sb.tA, cl, Gc, nN, sb.tC, cr);   // Gamma_L G
     gemm<OP_N, OP_N, false>(smem, cl, cr, cr, sb.tC, cr, sb.tB, cr, sb.tD, cr);  // ... Gamma_R
     double part = 0.0;
-    for (int e = threadIdx.x; e < cl * cr; e += CTA_THREADS) {
+    for (int e = team_tid(); e < cl * cr; e += team_threads()) {
       int i = e / cr, l = e % cr;
       cplx a = sb.tD[e], gg = Gc[(int64_t)i * nN + l];
       part += a.x * gg.x + a.y * gg.y;  // Re(a conj(g))
     }
-    tval = cta_sum(part, red);
+    tval = team_sum(part, red);
   }
   // ------------------------------------------------------------ adjoint
   // d(c T)/dX_pq = 2c W_qp^H with W_qp = G_qN M G_1p, M = Gamma_R G_1N^H Gamma_L
@@ -928,7 +984,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     if (gseL) {
       gemm<OP_N, OP_N, MX>(smem, cl, cl, cr, Gc, nN, sb.T1, cl, sb.Nd, cl);
       const int ns = it.nse_l;
-      for (int e = threadIdx.x; e < ns * ns; e += CTA_THREADS) {
+      for (int e = team_tid(); e < ns * ns; e += team_threads()) {
         int i = e / ns, j = e % ns;
         cplx v = cmk(0.0, 0.0);
         if (i < cl && j < cl) {
@@ -941,7 +997,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     if (gseR) {
       gemm<OP_C, OP_N, MX>(smem, cr, cr, cl, Gc, nN, sb.tC, cr, sb.Nl, cr);  // Gc^H (Gamma_L Gc)
       const int ns = it.nse_r, o = ns - cr;
-      for (int e = threadIdx.x; e < ns * ns; e += CTA_THREADS) {
+      for (int e = team_tid(); e < ns * ns; e += team_threads()) {
         int i = e / ns, j = e % ns;
         cplx v = cmk(0.0, 0.0);
         if (i >= o && j >= o) {
@@ -951,7 +1007,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
         gseR[e] = cadd(gseR[e], v);
       }
     }
-    __syncthreads();
+    team_sync();
     auto colp = [&](int q) -> const cplx* {
       if (q == K - 1) return gptr(K - 1);
       return (fl & NEGF_OUT_GR_LC) ? out + blk[q].o_grlc + row * (int64_t)blk[q].n * nN : sb.colslab + blk[q].gc;
@@ -995,7 +1051,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
           gemm_epi<OP_N, OP_N, MX>(g, smem, e);
         }
         // P_{p+1} = P_p g_p U_p
-        form_shift(sb.Uz, hs, blk[p].hu, blk[p].su, z, np, nn, smem);
+        form_shift<MX>(sb.Uz, hs, blk[p].hu, blk[p].su, z, np, nn, smem);
         gemm<OP_N, OP_N, MX>(smem, np, nn, np, gptr(p), np, sb.Uz, nn, sb.gU, nn);
         if (p == 0) copy_mat(Pn, sb.gU, cl, nn, smem);
         else gemm<OP_N, OP_N, MX>(smem, cl, nn, np, Pc, np, sb.gU, nn, Pn, nn);
@@ -1005,7 +1061,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     pc.mark(PH_GEMM_BWD);
   }
 
-  if (threadIdx.x == 0) {
+  if (team_tid() == 0) {
     if (fl & NEGF_TRANS) P.trans[it.out] = tval;
     if (fl & NEGF_DOS) P.dos[it.out] = dos_total;
     int st = NEGF_OK;
@@ -1014,33 +1070,37 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
     else if (!isfinite(tval) || !isfinite(dos_total)) st = NEGF_ERR_NONFINITE;
     P.status[it.out] = st;
   }
-  __syncthreads();
+  team_sync();
   pc.mark(PH_TRANS);
 }
 
 template <bool MX, int FEAT>
 __global__ void __launch_bounds__(CTA_THREADS, 1) rgf_kernel(const NegfRgfProblem P) {
   char* const smem = negf_smem;
-  __shared__ int s_item;
+  __shared__ unsigned long long s_item;
   __shared__ double red[CTA_THREADS / 32];
   unsigned* queue = reinterpret_cast<unsigned*>(P.scratch);
-  const SlotBufs sb = slot_bufs(P, blockIdx.x);
+  const SlotBufs sb = slot_bufs(P, blockIdx.x / team_size());
   PhaseClock pc;
   pc.start(P.phase_cycles != nullptr);
   if constexpr (MX) tc_tmem_alloc();
   for (;;) {
-    if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
-    __syncthreads();
-    const int idx = s_item;
-    __syncthreads();
+    if (team_tid() == 0) s_item = atomicAdd(queue, 1u);
+    team_sync();
+#ifdef NEGF_TEAM
+    const int idx = (int)team_peek(&s_item, 0);
+#else
+    const int idx = (int)s_item;
+#endif
+    team_sync();
     pc.mark(PH_OTHER);
     if (idx >= P.n_items) break;
     const NegfItem it = P.items[idx];
     rgf_item<MX, FEAT>(P, it, sb, smem, red, pc);
   }
   if constexpr (MX) tc_tmem_free();
-  if (pc.on)
-    for (int i = 0; i < NPH; ++i) P.phase_cycles[(size_t)blockIdx.x * NPH + i] = pc.c[i];
+  if (pc.on && team_rank() == 0)
+    for (int i = 0; i < NPH; ++i) P.phase_cycles[(size_t)(blockIdx.x / team_size()) * NPH + i] = pc.c[i];
 }
 
 // Dynamic shared memory: the union of the GEMM ring, the inverse panel and the
@@ -1053,6 +1113,12 @@ inline size_t rgf_smem_bytes(int max_n, bool mixed) {
 static_assert(CTA_THREADS == 256, "cta_stream.cuh assumes 256-thread CTAs");
 
 
+#ifdef NEGF_TEAM
+// One team of `cl` CTAs per work slot (rgf_team.cu).
+int rgf_launch_team(int feat, const NegfRgfProblem& p, size_t smem, int slots, int cl, cudaStream_t s);
+// Teams of `cl` CTAs that fit the GPU at once; 0 when it cannot run them.
+int rgf_team_fit(int feat, size_t smem, int cl);
+#else
 // Set the shared-memory limit of one instantiation and launch it (grid CTAs).  The FP64 sweep
 // is compiled per feature set (rgf.cu); the mixed-precision sweep is one instantiation with
 // every feature (rgf_mx.cu).
@@ -1066,5 +1132,6 @@ inline int rgf_launch_impl(const NegfRgfProblem& p, size_t smem, int grid, cudaS
 }
 int rgf_launch_fp64(int feat, const NegfRgfProblem& p, size_t smem, int grid, cudaStream_t s);  // rgf.cu
 int rgf_launch_mx(const NegfRgfProblem& p, size_t smem, int grid, cudaStream_t s);                // rgf_mx.cu
+#endif
 
-}  // namespace negf
+}  // namespace NEGF_NS

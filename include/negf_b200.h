@@ -147,7 +147,8 @@ typedef struct NegfRgfProblem {
   double* orb_ar;           /* per-orbital diag(G_qN Gamma_R G_qN^H), offset NegfItem.orb (NEGF_ORB_AR) */
   int32_t* status;          /* [n_items] per-item status (always written) */
   uint32_t flags;
-  int32_t n_slots;          /* concurrent work slots = CTAs launched */
+  int32_t n_slots;          /* concurrent work slots; each runs on one CTA, or (FP64) on a cluster of 2, 4 or
+                               8 CTAs when the slots in use leave that many SMs free */
   void* scratch;            /* >= negf_rgf_scratch_bytes(problem) bytes, 256-aligned */
   size_t scratch_bytes;
   unsigned long long* phase_cycles; /* optional [n_slots x NEGF_PHASES] SM-cycle counters; NULL = off */
