@@ -224,6 +224,24 @@ struct EpiStore {
   }
 };
 
+// The same with the addend of a warp's sub-tile fetched before the first store, so that its reads are
+// in flight together and not one behind another's store (same values).  For 4M products only: their
+// two accumulator planes leave the registers for it; with three the main loop would lose more.
+struct EpiAdd {
+  typedef cplx Addend;
+  GemmArgs g;
+  NEGF_DEV cplx fetch(int m, int n) const { return g.D[(int64_t)m * g.ldd + n]; }
+  NEGF_DEV void store(int m, int n, cplx v, cplx d) const {
+    g.C[(int64_t)m * g.ldc + n] = cfma(g.beta, d, cmul(g.alpha, v));
+  }
+};
+template <class Epi>
+struct EpiTraits {
+  template <class T> static char test(typename T::Addend*);
+  template <class T> static long test(...);
+  static constexpr bool two_phase = sizeof(test<Epi>(nullptr)) == 1;
+};
+
 // acc = op(A) op(B) over the whole M x N output by the whole CTA; epi(m, n, acc)
 // is called once for every in-range element.  The output must not alias A or
 // B.  Ends with __syncthreads(), so whatever epi wrote to global memory is
@@ -291,7 +309,68 @@ NEGF_DEV void gemm_body(const GemmArgs& g, const Epi& epi) {
     return;
   }
 
-#ifdef NEGF_TEAM
+#ifndef NEGF_TEAM
+  if constexpr (G3) {  // nested tile loops: 2.5 % faster than the general form below in the sweep at n = 96
+    // the next slab to load: its tile corner, k offset and ring stage
+    int lm = 0, ln = 0, lk = 0, lst = 0;
+    int left = ((g.M + GT_M - 1) / GT_M) * ((g.N + GT_N - 1) / GT_N) * nk;
+    auto load_next = [&]() {
+      if (left > 0) {
+        load_a_tile<OPA>(sA(lst), g, lm, lk, tid);
+        load_b_tile<OPB>(sB(lst), g, lk, ln, tid);
+        --left;
+        lst = lst + 1 == GT_STAGES ? 0 : lst + 1;
+        lk += GT_K;
+        if (lk >= g.K) {
+          lk = 0;
+          ln += GT_N;
+          if (ln >= g.N) { ln = 0; lm += GT_M; }
+        }
+      }
+      cp_async_commit();
+    };
+    __syncthreads();  // whatever used the ring's memory before is done with it
+#pragma unroll
+    for (int s = 0; s < GT_STAGES - 1; ++s) load_next();
+    cp_async_wait<GT_STAGES - 2>();
+    __syncthreads();
+    int st = 0;
+    for (int m0 = 0; m0 < g.M; m0 += GT_M) {
+      for (int n0 = 0; n0 < g.N; n0 += GT_N) {
+        if (m0 + wm >= g.M || n0 + wn >= g.N) {  // no output in this warp's sub-tile: keep the ring going
+          for (int k0 = 0; k0 < g.K; k0 += GT_K) {
+            load_next();
+            cp_async_wait<GT_STAGES - 2>();
+            __syncthreads();
+            st = st + 1 == GT_STAGES ? 0 : st + 1;
+          }
+          continue;
+        }
+        Acc3M acc;
+        acc.zero();
+        for (int k0 = 0; k0 < g.K; k0 += GT_K) {
+          const cplx *a = sA(st), *b = sB(st);
+          warp_mma_3m<CA, CB, G3>(acc, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
+          load_next();
+          Frag8 f;
+          frag8_load<CA, CB, G3>(f, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
+          cp_async_wait<GT_STAGES - 2>();
+          __syncthreads();
+          frag8_mma<G3>(acc, f);
+          st = st + 1 == GT_STAGES ? 0 : st + 1;
+        }
+        acc_foreach<G3>(acc, wm, wn, lane, [&](int r, int c, cplx v) {
+          const int m = m0 + r, n = n0 + c;
+          if (m < g.M && n < g.N) epi(m, n, v);
+        });
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    return;
+  }
+#endif
+
   // Output tiles of TM rows, dealt round the team.  The next slab to load: its tile, k offset, stage.
   constexpr int TM = 32 * MI;
   const int tn = (g.N + GT_N - 1) / GT_N, tiles = ((g.M + TM - 1) / TM) * tn;
@@ -343,73 +422,36 @@ NEGF_DEV void gemm_body(const GemmArgs& g, const Epi& epi) {
       frag8_mma<G3, MI>(acc, f);
       st = st + 1 == GT_STAGES ? 0 : st + 1;
     }
-    acc_foreach<G3, MI>(acc, wm, wn, lane, [&](int r, int c, cplx v) {
-      const int m = m0 + r, n = n0 + c;
-      if (m < g.M && n < g.N) epi(m, n, v);
-    });
-  }
-  cp_async_wait<0>();
-  team_sync();
-}
-#else
-  // the next slab to load: its tile corner, k offset and ring stage
-  int lm = 0, ln = 0, lk = 0, lst = 0;
-  int left = ((g.M + GT_M - 1) / GT_M) * ((g.N + GT_N - 1) / GT_N) * nk;
-  auto load_next = [&]() {
-    if (left > 0) {
-      load_a_tile<OPA>(sA(lst), g, lm, lk, tid);
-      load_b_tile<OPB>(sB(lst), g, lk, ln, tid);
-      --left;
-      lst = lst + 1 == GT_STAGES ? 0 : lst + 1;
-      lk += GT_K;
-      if (lk >= g.K) {
-        lk = 0;
-        ln += GT_N;
-        if (ln >= g.N) { ln = 0; lm += GT_M; }
-      }
-    }
-    cp_async_commit();
-  };
-  __syncthreads();  // whatever used the ring's memory before is done with it
+    if constexpr (EpiTraits<Epi>::two_phase) {
+      cplx d[MI][2][4];
 #pragma unroll
-  for (int s = 0; s < GT_STAGES - 1; ++s) load_next();
-  cp_async_wait<GT_STAGES - 2>();
-  __syncthreads();
-  int st = 0;
-  for (int m0 = 0; m0 < g.M; m0 += GT_M) {
-    for (int n0 = 0; n0 < g.N; n0 += GT_N) {
-      if (m0 + wm >= g.M || n0 + wn >= g.N) {  // no output in this warp's sub-tile: keep the ring going
-        for (int k0 = 0; k0 < g.K; k0 += GT_K) {
-          load_next();
-          cp_async_wait<GT_STAGES - 2>();
-          __syncthreads();
-          st = st + 1 == GT_STAGES ? 0 : st + 1;
-        }
-        continue;
-      }
-      Acc3M acc;
-      acc.zero();
-      for (int k0 = 0; k0 < g.K; k0 += GT_K) {
-        const cplx *a = sA(st), *b = sB(st);
-        warp_mma_3m<CA, CB, G3>(acc, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
-        load_next();
-        Frag8 f;
-        frag8_load<CA, CB, G3>(f, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
-        cp_async_wait<GT_STAGES - 2>();
-        __syncthreads();
-        frag8_mma<G3>(acc, f);
-        st = st + 1 == GT_STAGES ? 0 : st + 1;
-      }
-      acc_foreach<G3>(acc, wm, wn, lane, [&](int r, int c, cplx v) {
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int m = m0 + acc_row(i, e, wm, lane), n = n0 + acc_col(j, e, wn, lane);
+            d[i][j][e] = m < g.M && n < g.N ? epi.fetch(m, n) : cmk(0.0, 0.0);
+          }
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int m = m0 + acc_row(i, e, wm, lane), n = n0 + acc_col(j, e, wn, lane);
+            if (m < g.M && n < g.N) epi.store(m, n, acc_value<G3>(acc, i, j, e), d[i][j][e]);
+          }
+    } else {
+      acc_foreach<G3, MI>(acc, wm, wn, lane, [&](int r, int c, cplx v) {
         const int m = m0 + r, n = n0 + c;
         if (m < g.M && n < g.N) epi(m, n, v);
       });
     }
   }
   cp_async_wait<0>();
-  __syncthreads();
+  team_sync();
 }
-#endif
 
 // Whether the drifting form is the faster one for an M x N product of the sweep: the last row or
 // column of tiles leaves at least half of its warps without output (remainder 1 .. 32 of 64).
@@ -426,6 +468,12 @@ template <int OPA, int OPB, bool G3, bool DRIFT, int MI>
 __device__ __noinline__ void cta_gemm_std(const GemmArgs& gr) {
   const GemmArgs g = gr;
   gemm_body<OPA, OPB, G3, DRIFT, MI>(g, EpiStore{g});
+}
+
+template <int OPA, int OPB, int MI>
+__device__ __noinline__ void cta_gemm_add(const GemmArgs& gr) {  // 4M, with an addend
+  const GemmArgs g = gr;
+  gemm_body<OPA, OPB, false, true, MI>(g, EpiAdd{g});
 }
 
 #ifdef NEGF_TEAM
@@ -453,16 +501,27 @@ NEGF_DEV void cta_gemm_epi(const GemmArgs& g, const Epi& e) {
 template <int OPA, int OPB, bool G3 = true>
 NEGF_DEV void cta_gemm(const GemmArgs& g) {
 #ifdef NEGF_TEAM
-  if (team_half_tiles(g.M, g.N)) cta_gemm_std<OPA, OPB, G3, true, 1>(g);
-  else cta_gemm_std<OPA, OPB, G3, true, 2>(g);
+  const bool half = team_half_tiles(g.M, g.N);
 #else
+  // 4M products with few rows (the small updates of the lead LU): 16-row sub-tiles keep all eight
+  // warps, or at 16 rows no idle halves of four, on the tensor cores
+  const bool half = !G3 && g.M <= GT_M / 2;
+#endif
   if constexpr (G3) {
+#ifdef NEGF_TEAM
+    if (half) cta_gemm_std<OPA, OPB, G3, true, 1>(g);
+    else cta_gemm_std<OPA, OPB, G3, true, 2>(g);
+#else
     if (gemm_ragged(g.M, g.N)) cta_gemm_std<OPA, OPB, G3, true, 2>(g);
     else cta_gemm_std<OPA, OPB, G3, false, 2>(g);
-  } else {
-    cta_gemm_std<OPA, OPB, G3, true, 2>(g);
-  }
 #endif
+  } else if (g.use_d) {
+    if (half) cta_gemm_add<OPA, OPB, 1>(g);
+    else cta_gemm_add<OPA, OPB, 2>(g);
+  } else {
+    if (half) cta_gemm_std<OPA, OPB, G3, true, 1>(g);
+    else cta_gemm_std<OPA, OPB, G3, true, 2>(g);
+  }
 }
 
 }  // namespace NEGF_NS

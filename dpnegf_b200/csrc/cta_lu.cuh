@@ -25,7 +25,7 @@
 #pragma once
 #include "cta_inverse.cuh"  // pivot search helpers, the CTA GEMM
 
-namespace negf {
+namespace NEGF_NS {
 
 // 1/a as conj(a) / |a|^2 (one division; pivots here are far from the
 // over/underflow range of |a|^2).
@@ -39,7 +39,8 @@ constexpr int LU_TB = 16;  // diagonal blocks of the triangular solves (register
 template <int NB>
 struct LuLayout {
   static constexpr int PP = NB + 1;  // panel pitch (complex entries)
-  __host__ __device__ static size_t panel_bytes(int n) { return (size_t)n * PP * sizeof(double2); }
+  // the panel and the rows that trade places (two columns in flight)
+  __host__ __device__ static size_t panel_bytes(int n) { return ((size_t)n * PP + 4 * NB) * sizeof(double2); }
   // the small arrays sit above both the panel and the GEMM ring (the GEMM reuses the panel area)
   __host__ __device__ static size_t small_offset(int n) {
     size_t a = panel_bytes(n), g = (size_t)GEMM_SMEM_BYTES;
@@ -104,53 +105,113 @@ NEGF_DEV void lu_laswp(const LuCtx& c, cplx* col0, int64_t ld, int ncols, int ka
   c.mark(PH_INV_STAGE);
 }
 
-// Unblocked LU with row swaps of rows r0..n-1, columns r0..r0+w-1 (w <= NB) in shared memory.
-template <int NB>
-NEGF_DEV void lu_panel(const LuCtx& c, int r0, int w) {
+// Unblocked LU with row swaps of rows r0..n-1, columns r0..r0+w-1 (w <= NB).  Thread t holds the
+// not yet eliminated entries of rows t + 256 a in registers, the current column first: a step's
+// rank-1 update writes one place to the left, so that no register index depends on the column.  The
+// multipliers go to shared memory, where the row swaps reach them.  Two barriers per column, for
+// the pivot candidates of the warps and for the two rows that trade places (with the panel in shared
+// memory and every operand read from it, a column took 3000-3400 cycles; now about 1200).
+template <int NB, int RT, int WID>
+NEGF_DEV void lu_panel_steps(const LuCtx& c, cplx (&x)[RT][NB], cplx* P, cplx* rows, int r0, int m, int j0, int j1) {
   constexpr int PP = LuLayout<NB>::PP;
   constexpr int NWARP = CTA_THREADS / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int m = c.n - r0;
-  cplx* P = reinterpret_cast<cplx*>(c.smem);
-  cplx* Wp = c.W + (int64_t)r0 * c.ldw + r0;
-  for (int e = tid; e < m * NB; e += CTA_THREADS) {
-    const int r = e / NB, k = e % NB;
-    P[r * PP + k] = k < w ? Wp[(int64_t)r * c.ldw + k] : cmk(0.0, 0.0);
-  }
-  __syncthreads();
-  for (int j = 0; j < w; ++j) {
-    long long bv = -1;
-    int bi = m;
-    for (int r = j + tid; r < m; r += CTA_THREADS) argmax_merge_key(bv, bi, pivot_key(P[r * PP + j]), r);
-    warp_argmax_key(bv, bi);
-    if (lane == 0) { c.red_v[warp] = bv; c.red_i[warp] = bi; }
+  for (int j = j0; j < j1; ++j) {
+    unsigned hi = 0u, lo = 0u;
+    int bi = 0x7fffffff;
+#pragma unroll
+    for (int a = 0; a < RT; ++a) {
+      const int r = tid + CTA_THREADS * a;
+      if (r >= j && r < m) {
+        const unsigned long long k = (unsigned long long)pivot_key(x[a][0]);
+        const unsigned kh = (unsigned)(k >> 32), kl = (unsigned)k;
+        if (bi == 0x7fffffff || kh > hi || (kh == hi && kl > lo)) { hi = kh; lo = kl; bi = r; }
+      }
+    }
+    const bool any = bi != 0x7fffffff;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    bi = (int)__reduce_min_sync(0xffffffffu, (unsigned)(any && hi == mh && lo == ml ? bi : 0x7fffffff));
+    if (lane == 0) {
+      c.red_v[warp] = bi == 0x7fffffff ? -1LL : (long long)(((unsigned long long)mh << 32) | ml);
+      c.red_i[warp] = bi;
+    }
     __syncthreads();
-    bv = c.red_v[0];
+    long long bv = c.red_v[0];
     bi = c.red_i[0];
 #pragma unroll
     for (int k = 1; k < NWARP; ++k) argmax_merge_key(bv, bi, c.red_v[k], c.red_i[k]);
-    if (bi != j)
-      for (int k = tid; k < NB; k += CTA_THREADS) {
-        const cplx t = P[j * PP + k];
-        P[j * PP + k] = P[bi * PP + k];
-        P[bi * PP + k] = t;
+    // the pivot row and row j meet in shared memory, their multipliers trade places there
+    cplx *prow = rows + (j & 1) * 2 * NB, *jrow = prow + NB;
+#pragma unroll
+    for (int a = 0; a < RT; ++a) {
+      const int r = tid + CTA_THREADS * a;
+      if (r == bi) {
+#pragma unroll
+        for (int k = 0; k < WID; ++k) prow[k] = x[a][k];
       }
+      if (r == j && bi != j) {
+#pragma unroll
+        for (int k = 0; k < WID; ++k) jrow[k] = x[a][k];
+      }
+    }
+    if (bi != j && tid < j) {
+      const cplx t = P[j * PP + tid];
+      P[j * PP + tid] = P[bi * PP + tid];
+      P[bi * PP + tid] = t;
+    }
     if (tid == 0) {
       c.ipiv[r0 + j] = r0 + bi;
       if (pivot_key_singular(bv)) *c.flag = 1;
     }
     __syncthreads();
-    const cplx d = crcp_fast(P[j * PP + j]);
-    for (int r = j + 1 + tid; r < m; r += CTA_THREADS) {
-      const cplx l = cmul(P[r * PP + j], d);
-      P[r * PP + j] = l;
-      for (int k = j + 1; k < w; ++k) P[r * PP + k] = csub(P[r * PP + k], cmul(l, P[j * PP + k]));
+    const cplx d = crcp_fast(prow[0]);
+    if (tid < NB - j) P[j * PP + j + tid] = prow[tid];  // row j of U
+#pragma unroll
+    for (int a = 0; a < RT; ++a) {
+      const int r = tid + CTA_THREADS * a;
+      if (r > j && r < m) {
+        if (r == bi) {
+#pragma unroll
+          for (int k = 0; k < WID; ++k) x[a][k] = jrow[k];
+        }
+        const cplx l = cmul(x[a][0], d);
+        P[r * PP + j] = l;
+#pragma unroll
+        for (int k = 1; k < WID; ++k) x[a][k - 1] = csub(x[a][k], cmul(l, prow[k]));
+      }
     }
-    __syncthreads();
   }
-  for (int e = tid; e < m * w; e += CTA_THREADS) {
-    const int r = e / w, k = e % w;
-    Wp[(int64_t)r * c.ldw + k] = P[r * PP + k];
+}
+template <int NB>
+NEGF_DEV void lu_panel(const LuCtx& c, int r0, int w) {
+  constexpr int PP = LuLayout<NB>::PP, RT = NB == 32 ? 1 : 2;  // NB = 32 for n <= 256
+  const int tid = threadIdx.x;
+  const int m = c.n - r0;
+  cplx* P = smem_cplx();
+  cplx* rows = P + (size_t)c.n * PP;  // [2][2][NB]
+  cplx* Wp = c.W + (int64_t)r0 * c.ldw + r0;
+  for (int e = tid; e < m * NB; e += CTA_THREADS) {
+    const int r = e / NB, k = e % NB;
+    cp_async16(P + r * PP + k, k < w ? Wp + (int64_t)r * c.ldw + k : c.W, k < w);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  cplx x[RT][NB];
+#pragma unroll
+  for (int a = 0; a < RT; ++a) {
+    const int r = tid + CTA_THREADS * a;
+#pragma unroll
+    for (int k = 0; k < NB; ++k) x[a][k] = r < m ? P[r * PP + k] : cmk(0.0, 0.0);
+  }
+  __syncthreads();
+  lu_panel_steps<NB, RT, NB>(c, x, P, rows, r0, m, 0, min(w, NB / 2));
+  lu_panel_steps<NB, RT, NB / 2>(c, x, P, rows, r0, m, NB / 2, w);
+  __syncthreads();
+  for (int e = tid; e < m * NB; e += CTA_THREADS) {
+    const int r = e / NB, k = e % NB;
+    if (k < w) Wp[(int64_t)r * c.ldw + k] = P[r * PP + k];
   }
   __syncthreads();
   c.mark(PH_INV_PANEL);
@@ -158,8 +219,11 @@ NEGF_DEV void lu_panel(const LuCtx& c, int r0, int w) {
 
 // C (h x N, row stride ldc) <- L^-1 C with L the unit-lower triangle of W at (r0, r0), h <= LU_TB:
 // L staged in shared memory, each thread solves whole columns in registers.
-NEGF_DEV void lu_trsm_lower_leaf(const LuCtx& c, int r0, int h, cplx* C, int64_t ldc, int N) {
+// FULL: h = LU_TB, without the 120 uniform branches of a ragged block.
+template <bool FULL>
+NEGF_DEV void lu_trsm_lower_leaf(const LuCtx& c, int r0, int hr, cplx* C, int64_t ldc, int N) {
   constexpr int TP = LU_TB + 1;
+  const int h = FULL ? LU_TB : hr;
   cplx* Ls = reinterpret_cast<cplx*>(c.smem);
   for (int e = threadIdx.x; e < h * h; e += CTA_THREADS) {
     const int i = e / h, j = e % h;
@@ -187,8 +251,10 @@ NEGF_DEV void lu_trsm_lower_leaf(const LuCtx& c, int r0, int h, cplx* C, int64_t
 }
 
 // C <- U^-1 C with U the upper triangle (non-unit) of W at (r0, r0), h <= LU_TB.
-NEGF_DEV void lu_trsm_upper_leaf(const LuCtx& c, int r0, int h, cplx* C, int64_t ldc, int N) {
+template <bool FULL>
+NEGF_DEV void lu_trsm_upper_leaf(const LuCtx& c, int r0, int hr, cplx* C, int64_t ldc, int N) {
   constexpr int TP = LU_TB + 1;
+  const int h = FULL ? LU_TB : hr;
   cplx* Us = reinterpret_cast<cplx*>(c.smem);
   for (int e = threadIdx.x; e < h * h; e += CTA_THREADS) {
     const int i = e / h, j = e % h;
@@ -224,10 +290,12 @@ NEGF_DEV int lu_split(int h, int unit) { return ((h / 2 + unit - 1) / unit) * un
 // C <- L^-1 C, L the unit-lower triangle of W at (r0, r0) of size h: halves down to LU_TB.
 template <int LV>
 __device__ __noinline__ void lu_trsm_lower(const LuCtx c, int r0, int h, cplx* C, int64_t ldc, int N) {
-  if constexpr (LV == 0) {
-    lu_trsm_lower_leaf(c, r0, h, C, ldc, N);
-  } else {
-    if (h <= LU_TB) { lu_trsm_lower_leaf(c, r0, h, C, ldc, N); return; }
+  if (h <= LU_TB) {
+    if (h == LU_TB) lu_trsm_lower_leaf<true>(c, r0, h, C, ldc, N);
+    else lu_trsm_lower_leaf<false>(c, r0, h, C, ldc, N);
+    return;
+  }
+  if constexpr (LV > 0) {
     const int h1 = lu_split(h, LU_TB);
     lu_trsm_lower<LV - 1>(c, r0, h1, C, ldc, N);
     lu_gemm_sub(c, h - h1, N, h1, c.W + (int64_t)(r0 + h1) * c.ldw + r0, c.ldw, C, ldc, C + (int64_t)h1 * ldc, ldc);
@@ -238,10 +306,12 @@ __device__ __noinline__ void lu_trsm_lower(const LuCtx c, int r0, int h, cplx* C
 // C <- U^-1 C, U the upper triangle of W at (r0, r0) of size h.
 template <int LV>
 __device__ __noinline__ void lu_trsm_upper(const LuCtx c, int r0, int h, cplx* C, int64_t ldc, int N) {
-  if constexpr (LV == 0) {
-    lu_trsm_upper_leaf(c, r0, h, C, ldc, N);
-  } else {
-    if (h <= LU_TB) { lu_trsm_upper_leaf(c, r0, h, C, ldc, N); return; }
+  if (h <= LU_TB) {
+    if (h == LU_TB) lu_trsm_upper_leaf<true>(c, r0, h, C, ldc, N);
+    else lu_trsm_upper_leaf<false>(c, r0, h, C, ldc, N);
+    return;
+  }
+  if constexpr (LV > 0) {
     const int h1 = lu_split(h, LU_TB);
     lu_trsm_upper<LV - 1>(c, r0 + h1, h - h1, C + (int64_t)h1 * ldc, ldc, N);
     lu_gemm_sub(c, h1, N, h - h1, c.W + (int64_t)r0 * c.ldw + r0 + h1, c.ldw, C + (int64_t)h1 * ldc, ldc, C, ldc);
@@ -338,4 +408,4 @@ NEGF_DEV void cta_lu_trsolve(cplx* W, int64_t ldw, int n, cplx* B, int64_t ldb, 
   else cta_lu_trsolve_nb<16>(W, ldw, n, B, ldb, nb, smem_raw, pc);
 }
 
-}  // namespace negf
+}  // namespace NEGF_NS

@@ -18,7 +18,8 @@ constexpr int STREAM_SMEM_BYTES = 4 * STREAM_CHUNK * (int)sizeof(cplx);
 // The chunks go round the team's CTAs.  Ends with team_sync().
 // The roundings of z Y are spelled out, so that results do not depend on how the compiler contracts
 // an instantiation: the products with Re z, the large ones, are fused into the sums.  The mixed sweep
-// amplifies every rounding of its inputs and keeps the imaginary part it has always had (MX).
+// and the lead decimation amplify every rounding of their inputs and keep the imaginary part they
+// have always had (MX).
 template <bool MX = false>
 NEGF_DEV void cta_shift_form(cplx* out, const cplx* X, const cplx* Y, cplx z, cplx alpha, int count,
                              cplx* smem) {

@@ -5,7 +5,7 @@
 #include "cta_lu.cuh"
 #include "cta_stream.cuh"
 
-namespace negf {
+namespace NEGF_NS {
 
 // out[i][j] = conj(X[j][i]) - z conj(Y[j][i])   (n x n), i.e. X^H - z Y^H
 NEGF_DEV void form_herm_shift(cplx* out, const cplx* X, const cplx* Y, cplx z, int n) {
@@ -76,4 +76,4 @@ inline size_t lead_smem_bytes(int max_n) {
   return m > c ? m : c;
 }
 
-}  // namespace negf
+}  // namespace NEGF_NS

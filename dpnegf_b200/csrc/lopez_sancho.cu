@@ -27,7 +27,7 @@
 #include "../../include/negf_b200.h"
 #include "lead_forms.cuh"
 
-namespace negf {
+namespace NEGF_NS {
 
 constexpr int LS_NBUF = 14;  // max_n^2 buffers per slot (see ls_item)
 constexpr size_t LS_SCRATCH_HEADER = 256;
@@ -110,19 +110,20 @@ NEGF_DEV void ls_item(const NegfLsProblem& P, const NegfLsItem& it, cplx* slot, 
 
   // alpha = h10 - z s10 = h01^H - z s01^H ; beta = h01 - z s01 ; eps = eps_s = H
   form_herm_shift(AB, h01, s01, z, n);
-  cta_shift_form(AB + n2, h01, s01, z, ONE, (int)n2, smem);
-  cta_shift_form(eps, H, nullptr, cmk(0.0, 0.0), ONE, (int)n2, smem);
-  cta_shift_form(epss, H, nullptr, cmk(0.0, 0.0), ONE, (int)n2, smem);
+  cta_shift_form<true>(AB + n2, h01, s01, z, ONE, (int)n2, smem);
+  cta_shift_form<true>(eps, H, nullptr, cmk(0.0, 0.0), ONE, (int)n2, smem);
+  cta_shift_form<true>(epss, H, nullptr, cmk(0.0, 0.0), ONE, (int)n2, smem);
 
   int it_n = 0;
   bool converged = false;
   for (int iter = 1; iter <= P.max_iter + 1; ++iter) {
     it_n = iter;
     // A = zS - eps;  [Xa Xb] = A^-1 [alpha beta]
-    cta_shift_form(A, eps, S, z, cmk(-1.0, 0.0), (int)n2, smem);
+    cta_shift_form<true>(A, eps, S, z, cmk(-1.0, 0.0), (int)n2, smem);
     bad |= cta_lu_factor(A, n, n, smem_raw);
     {  // the right-hand sides [alpha beta] in the pivoted row order
       const int* perm = cta_lu_perm(smem_raw, n);
+#pragma unroll 4
       for (int e = threadIdx.x; e < n2; e += CTA_THREADS) {
         const int i = e / n, j = e % n;
         const int64_t src = (int64_t)perm[i] * n + j;
@@ -136,6 +137,7 @@ NEGF_DEV void ls_item(const NegfLsProblem& P, const NegfLsItem& it, cplx* slot, 
     gemm_ls<OP_N, OP_N>(smem, n2c, n2c, n, AB, n, Xab, n2c, Pm, n2c);
     // eps = eps + alpha Xb + beta Xa;  eps_s += beta Xa;  alpha <- alpha Xa;  beta <- beta Xb
     double m = 0.0;
+#pragma unroll 4
     for (int e = threadIdx.x; e < n2; e += CTA_THREADS) {
       const int64_t i = e / n, j = e % n;
       const cplx aXa = Pm[i * n2c + j], aXb = Pm[i * n2c + n + j];
@@ -177,7 +179,7 @@ NEGF_DEV void ls_item(const NegfLsProblem& P, const NegfLsItem& it, cplx* slot, 
   } else {
     cplx* gs = it.gs ? reinterpret_cast<cplx*>(it.gs) : gsb;
     // g_s = (zS - eps_s)^-1
-    cta_shift_form(A, epss, S, z, cmk(-1.0, 0.0), (int)n2, smem);
+    cta_shift_form<true>(A, epss, S, z, cmk(-1.0, 0.0), (int)n2, smem);
     bad |= lu_inverse(A, gs);
     // residual: (zS - H - (z s01 - h01) g_s (z s10 - h10)) g_s - I
     // z s01 - h01
@@ -210,7 +212,7 @@ NEGF_DEV void ls_item(const NegfLsProblem& P, const NegfLsItem& it, cplx* slot, 
         coupling_sigma(gs, sig);
       } else {
         // bulk form: Sigma = (E S - H) - g_s^-1
-        cta_shift_form(A, gs, nullptr, cmk(0.0, 0.0), ONE, (int)n2, smem);
+        cta_shift_form<true>(A, gs, nullptr, cmk(0.0, 0.0), ONE, (int)n2, smem);
         bad |= lu_inverse(A, Ya);
 #pragma unroll 4
         for (int e = threadIdx.x; e < n2; e += CTA_THREADS) sig[e] = csub(csub(cmul(E, S[e]), H[e]), Ya[e]);
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) ls_kernel(const NegfLsProblem 
 
 size_t ls_smem_bytes(int max_n) { return lead_smem_bytes(max_n); }
 
-}  // namespace negf
+}  // namespace NEGF_NS
 
 extern "C" {
 

@@ -15,7 +15,7 @@
 #include "../../include/negf_b200.h"
 #include "lead_forms.cuh"
 
-namespace negf {
+namespace NEGF_NS {
 
 // ---------------------------------------------------------------------------------------------
 // Weighted G Gamma G^H sum.  Stage 1 (one CTA per energy): T_i = w_i G_i[:, c0:] Gamma_i and a
@@ -186,7 +186,7 @@ NEGF_DEV void la_item(const NegfLeadAdjProblem& P, int idx, cplx* slot, char* sm
   }
 
   // ---- Lambda by doubling
-  cta_shift_form(tau, H01, S01, z, MONE, (int)n2, smem);                // z S01 - H01
+  cta_shift_form<true>(tau, H01, S01, z, MONE, (int)n2, smem);                // z S01 - H01
   form_eS_minus_h_herm(taup, H01, S01, z, n, n);                        // z S01^H - H01^H
   gemm_ls<OP_N, OP_N, true>(smem, n, n, n, g, n, tau, n, Pm, n);              // P = g tau
   gemm_ls<OP_N, OP_N, true>(smem, n, n, n, taup, n, g, n, Qm, n);             // Q = tau' g
@@ -275,7 +275,7 @@ static int sm_count_or(int fallback) {
   return n > 0 ? n : fallback;
 }
 
-}  // namespace negf
+}  // namespace NEGF_NS
 
 extern "C" {
 
