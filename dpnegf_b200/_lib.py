@@ -67,6 +67,8 @@ LS_ITEM_DTYPE = np.dtype([("lead", "<i4"), ("mode", "<i4"), ("e_re", "<f8"), ("e
                           ("sigma", "<u8"), ("gs", "<u8"), ("out", "<i8")])
 LS_DECIMATE = 0
 LS_SIGMA_FROM_GS = 1
+PACK_DTYPE = np.dtype([("src", "<u8"), ("dst", "<i8"), ("row_stride", "<i8"), ("col_stride", "<i8"), ("rows", "<i4"),
+                       ("cols", "<i4"), ("conj", "<i4"), ("pad", "<i4")])
 LEADADJ_ITEM_DTYPE = np.dtype([("e_re", "<f8"), ("e_im", "<f8"), ("gs", "<u8"), ("gsig", "<u8")])
 
 
@@ -186,6 +188,9 @@ def load():
     lib.negf_rgf_scratch_bytes.argtypes = [ctypes.POINTER(NegfRgfProblem)]
     lib.negf_rgf_run.restype = ctypes.c_int
     lib.negf_rgf_run.argtypes = [ctypes.POINTER(NegfRgfProblem), ctypes.c_void_p]
+    lib.negf_pack_run.restype = ctypes.c_int
+    lib.negf_pack_run.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p,
+                                  ctypes.c_void_p]
     lib.negf_sm_count.restype = ctypes.c_int
     lib.negf_sm_count.argtypes = []
     lib.negf_version.restype = ctypes.c_char_p

@@ -107,6 +107,7 @@ size_t negf_abi_struct_size(int which) {
     case 7: return sizeof(NegfGammaSum);
     case 8: return sizeof(NegfLeadAdjItem);
     case 9: return sizeof(NegfLeadAdjProblem);
+    case 10: return sizeof(NegfPackPiece);
     default: return 0;
   }
 }

@@ -46,7 +46,7 @@ class Geometry:
         self.device = dev
         self.devices = devices
         blocks, devs, copies = [], [], []
-        offdiag = []  # (block index, field, arena offset, numel) of H/S coupling blocks
+        offdiag = []  # (block index, field, piece index, arena offset, numel) of H/S coupling blocks
         cursor = 0
 
         def put(t):
@@ -88,10 +88,10 @@ class Geometry:
                         if tuple(t.shape[-2:]) != shape:
                             raise ValueError(f"{name}[{q}] has shape {tuple(t.shape)}, expected {shape}")
                         b[name] = put(t)
-                        offdiag.append((len(blocks), name, int(b[name]), t.numel()))
+                        offdiag.append((len(blocks), name, len(copies) - 1, int(b[name]), t.numel()))
                     for name, t in (("suT", d.su[q].mT), ("slT", d.sl[q].mT)):
                         b[name] = put(t)
-                        offdiag.append((len(blocks), name, int(b[name]), t.numel()))
+                        offdiag.append((len(blocks), name, len(copies) - 1, int(b[name]), t.numel()))
                 b["orb0"] = orb
                 b["g"] = g
                 b["gc"] = gc
@@ -119,21 +119,49 @@ class Geometry:
             self.u_slab = max(getattr(self, "u_slab", 0), gu)
         if self.max_n > _lib.NEGF_MAX_BLOCK:
             raise ValueError(f"block size {self.max_n} exceeds the supported maximum {_lib.NEGF_MAX_BLOCK}")
-        # one host->device copy per block straight into the arena
         self.hs = torch.empty(max(cursor, 1), dtype=C128, device=dev)
-        for off, t in copies:
-            src = t.detach()
-            if src.dtype != C128:
-                src = src.to(C128)
-            self.hs[off:off + src.numel()].view(src.shape).copy_(src, non_blocking=True)
+        nonzero = self._pack(copies) if dev.type == "cuda" else None
+        if nonzero is None:  # one copy per block straight into the arena
+            for off, t in copies:
+                src = t.detach()
+                if src.dtype != C128:
+                    src = src.to(C128)
+                self.hs[off:off + src.numel()].view(src.shape).copy_(src, non_blocking=True)
         self.blocks = np.array(blocks, dtype=_lib.BLOCK_DTYPE)
         self.devs = np.array(devs, dtype=_lib.DEVICE_DTYPE)
         if detect_zero_offdiag and offdiag:
             # zero coupling blocks (orthogonal basis: su = sl = 0) are skipped by the kernel
-            amax = torch.stack([self.hs[o:o + n].abs().amax() for _, _, o, n in offdiag])
-            for (bi, name, _, _), z in zip(offdiag, (amax == 0).tolist()):
+            if nonzero is not None:
+                flags = nonzero.cpu().numpy()
+                zero = [not flags[piece] for _, _, piece, _, _ in offdiag]
+            else:
+                zero = (torch.stack([self.hs[o:o + n].abs().amax() for _, _, _, o, n in offdiag]) == 0).tolist()
+            for (bi, name, _, _, _), z in zip(offdiag, zero):
                 if z:
                     self.blocks[bi][name] = -1
+
+    def _pack(self, copies):
+        """Every block into the arena in one launch, when all are 2-D complex128 tensors of this GPU;
+        returns the per-piece nonzero flags, or None when the blocks go one by one."""
+        hs = self.hs
+        if not copies or any(t.device != hs.device or t.dtype != C128 or t.ndim != 2 or t.numel() == 0 or t.is_neg()
+                             for _, t in copies):
+            return None
+        tab = np.zeros(len(copies), dtype=_lib.PACK_DTYPE)
+        tab["src"] = [t.data_ptr() for _, t in copies]
+        tab["dst"] = [off for off, _ in copies]
+        tab["row_stride"] = [t.stride(0) for _, t in copies]
+        tab["col_stride"] = [t.stride(1) for _, t in copies]
+        tab["rows"] = [t.shape[0] for _, t in copies]
+        tab["cols"] = [t.shape[1] for _, t in copies]
+        tab["conj"] = [t.is_conj() for _, t in copies]
+        lib = _lib.load()
+        with torch.cuda.device(hs.device):
+            tab_t = torch.from_numpy(tab.view(np.uint8)).to(hs.device)
+            nonzero = torch.empty(len(copies), dtype=torch.int32, device=hs.device)
+            _lib.check(lib.negf_pack_run(tab_t.data_ptr(), len(copies), int((tab["rows"].astype(np.int64) * tab["cols"]).max()),
+                                         hs.data_ptr(), nonzero.data_ptr(), _lib.stream_handle()), "negf_pack_run")
+        return nonzero
 
     @property
     def n_orb(self):

@@ -180,6 +180,18 @@ typedef struct NegfRgfProblem {
   int32_t ckpt_blocks;      /* with ckpt > 0: the device's block count K (sizes the checkpoint area) */
 } NegfRgfProblem;
 
+/* ---- packing of H/S blocks ------------------------------------------- */
+
+/* One block to copy: dst[i * cols + j] = src[i * row_stride + j * col_stride], conjugated if conj. */
+typedef struct NegfPackPiece {
+  const double* src;          /* complex128, device memory */
+  int64_t dst;                /* element offset in the arena */
+  int64_t row_stride, col_stride; /* in complex elements */
+  int32_t rows, cols;
+  int32_t conj;
+  int32_t pad;
+} NegfPackPiece;
+
 /* ---- Lopez-Sancho lead decimation ------------------------------------ */
 
 /* One lead principal layer (energy independent).  Offsets into `arena`. */
@@ -338,6 +350,11 @@ int negf_rgf_static_slots(const NegfRgfProblem* p);
 /* Size in bytes of the static scratch array used by negf_rgf_run_static. */
 size_t negf_rgf_static_scratch_bytes(void);
 
+/* Copy n_pieces blocks (table in device memory; max_count = largest rows x cols) into the arena in one
+   launch; nonzero[i] (device memory) is set to 1 if piece i has an entry other than zero, else 0. */
+int negf_pack_run(const NegfPackPiece* pieces, int32_t n_pieces, int64_t max_count, double* arena, int32_t* nonzero,
+                  void* cuda_stream);
+
 /* Number of SMs of the current CUDA device (grid sizing helper). */
 int negf_sm_count(void);
 
@@ -346,7 +363,7 @@ const char* negf_version(void);
 
 /* sizeof of the ABI structs (0 NegfBlock, 1 NegfDevice, 2 NegfItem,
  * 3 NegfRgfProblem, 4 NegfLead, 5 NegfLsItem, 6 NegfLsProblem, 7 NegfGammaSum,
- * 8 NegfLeadAdjItem, 9 NegfLeadAdjProblem) so bindings
+ * 8 NegfLeadAdjItem, 9 NegfLeadAdjProblem, 10 NegfPackPiece) so bindings
  * can verify their mirrors; 0 if unknown. */
 size_t negf_abi_struct_size(int which);
 

@@ -90,3 +90,26 @@ def test_every_output_selection_agrees(dims, overlap):
         got, want = run(outputs=(tag,)).blocks[0][tag], full.blocks[0][tag]
         for x, y in [(got, want)] if tag == "g_trans" else zip(got, want):
             assert same(x, y), tag
+
+
+def test_packed_arena_equals_the_blocks():
+    """One launch packs blocks of any stride, conjugated views and transposes exactly; zero couplings
+    (and only those) are marked; other types and host blocks take the copy path with the same arena."""
+    from dpnegf_b200 import rgf_plan
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.complex(*(torch.randn(*s, generator=gen, dtype=torch.float64, device="cuda") for _ in range(2)))
+    dims = [3, 40, 33]
+    wide = r(80, 80)
+    hd = [r(3, 3).mT, wide[::2, 1::2], r(33, 33).mH]
+    hu = [r(40, 3).mH, r(1, 33).expand(40, 33)]
+    hl = [u.mH for u in hu]
+    sd = [torch.eye(n, dtype=torch.complex128, device="cuda") for n in dims]
+    su = [torch.zeros(3, 40, dtype=torch.complex128, device="cuda"), r(40, 33)]
+    sl = [-torch.zeros(40, 3, dtype=torch.complex128, device="cuda"), su[1].mH]
+    su[1] = su[1].clone()
+    g = rgf_plan.Geometry([rgf_plan.DeviceBlocks(hd, hu, hl, sd, su, sl)])
+    host = rgf_plan.Geometry([rgf_plan.DeviceBlocks(*[[t.cpu().resolve_conj() for t in x] for x in (hd, hu, hl, sd, su, sl)])])
+    assert torch.equal(g.hs, host.hs) and (g.blocks == host.blocks).all()
+    b = g.blocks
+    assert b[0]["su"] == b[0]["sl"] == b[0]["suT"] == b[0]["slT"] == -1
+    assert all(b[1][k] >= 0 for k in ("hu", "hl", "su", "sl", "suT", "slT")) and b[0]["hu"] >= 0
