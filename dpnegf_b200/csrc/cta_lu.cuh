@@ -90,7 +90,7 @@ NEGF_DEV void lu_gemm_sub(const LuCtx& c, int M, int N, int K, const cplx* A, in
 // Row swaps ipiv[ka..kb) applied in order to the ncols columns starting at col (row stride ld).
 // Each thread owns whole columns; ends with __syncthreads().
 NEGF_DEV void lu_laswp(const LuCtx& c, cplx* col0, int64_t ld, int ncols, int ka, int kb) {
-  for (int j = threadIdx.x; j < ncols; j += CTA_THREADS) {
+  for (int j = team_tid(); j < ncols; j += team_threads()) {
     cplx* col = col0 + j;
     for (int k = ka; k < kb; ++k) {
       const int p = c.ipiv[k];
@@ -101,7 +101,7 @@ NEGF_DEV void lu_laswp(const LuCtx& c, cplx* col0, int64_t ld, int ncols, int ka
       }
     }
   }
-  __syncthreads();
+  team_sync();
   c.mark(PH_INV_STAGE);
 }
 
@@ -197,7 +197,7 @@ NEGF_DEV void lu_panel(const LuCtx& c, int r0, int w) {
   }
   cp_async_commit();
   cp_async_wait<0>();
-  __syncthreads();
+  team_sync();  // every CTA of a team factorises its own copy of the panel; one stores it below
   cplx x[RT][NB];
 #pragma unroll
   for (int a = 0; a < RT; ++a) {
@@ -209,11 +209,11 @@ NEGF_DEV void lu_panel(const LuCtx& c, int r0, int w) {
   lu_panel_steps<NB, RT, NB>(c, x, P, rows, r0, m, 0, min(w, NB / 2));
   lu_panel_steps<NB, RT, NB / 2>(c, x, P, rows, r0, m, NB / 2, w);
   __syncthreads();
-  for (int e = tid; e < m * NB; e += CTA_THREADS) {
+  for (int e = team_rank() == 0 ? tid : m * NB; e < m * NB; e += CTA_THREADS) {
     const int r = e / NB, k = e % NB;
     if (k < w) Wp[(int64_t)r * c.ldw + k] = P[r * PP + k];
   }
-  __syncthreads();
+  team_sync();
   c.mark(PH_INV_PANEL);
 }
 
@@ -230,7 +230,7 @@ NEGF_DEV void lu_trsm_lower_leaf(const LuCtx& c, int r0, int hr, cplx* C, int64_
     Ls[i * TP + j] = c.W[(int64_t)(r0 + i) * c.ldw + r0 + j];
   }
   __syncthreads();
-  for (int col = threadIdx.x; col < N; col += CTA_THREADS) {
+  for (int col = team_tid(); col < N; col += team_threads()) {
     cplx* p = C + col;
     cplx x[LU_TB];
 #pragma unroll
@@ -246,7 +246,7 @@ NEGF_DEV void lu_trsm_lower_leaf(const LuCtx& c, int r0, int hr, cplx* C, int64_
     for (int j = 1; j < LU_TB; ++j)
       if (j < h) p[(int64_t)j * ldc] = x[j];
   }
-  __syncthreads();
+  team_sync();
   c.mark(PH_INV_GATHER);
 }
 
@@ -263,7 +263,7 @@ NEGF_DEV void lu_trsm_upper_leaf(const LuCtx& c, int r0, int hr, cplx* C, int64_
   __syncthreads();
   if (threadIdx.x < h) c.rdiag[threadIdx.x] = crcp_fast(Us[threadIdx.x * TP + threadIdx.x]);
   __syncthreads();
-  for (int col = threadIdx.x; col < N; col += CTA_THREADS) {
+  for (int col = team_tid(); col < N; col += team_threads()) {
     cplx* p = C + col;
     cplx x[LU_TB];
 #pragma unroll
@@ -281,7 +281,7 @@ NEGF_DEV void lu_trsm_upper_leaf(const LuCtx& c, int r0, int hr, cplx* C, int64_
     for (int j = 0; j < LU_TB; ++j)
       if (j < h) p[(int64_t)j * ldc] = x[j];
   }
-  __syncthreads();
+  team_sync();
   c.mark(PH_INV_GATHER);
 }
 

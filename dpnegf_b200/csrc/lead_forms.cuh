@@ -10,37 +10,23 @@ namespace NEGF_NS {
 // out[i][j] = conj(X[j][i]) - z conj(Y[j][i])   (n x n), i.e. X^H - z Y^H
 NEGF_DEV void form_herm_shift(cplx* out, const cplx* X, const cplx* Y, cplx z, int n) {
 #pragma unroll 4
-  for (int e = threadIdx.x; e < n * n; e += CTA_THREADS) {
+  for (int e = team_tid(); e < n * n; e += team_threads()) {
     int i = e / n, j = e % n;
     cplx x = cconj(X[(int64_t)j * n + i]), y = cconj(Y[(int64_t)j * n + i]);
     out[e] = csub(x, cmul(z, y));
   }
-  __syncthreads();
+  team_sync();
 }
 
 // out[i][j] = z conj(S[j][i]) - conj(H[j][i])   for an (rows x cols) H/S pair
 // stored (cols x rows): E S^H - H^H.
 NEGF_DEV void form_eS_minus_h_herm(cplx* out, const cplx* H, const cplx* S, cplx z, int rows, int cols) {
-  for (int e = threadIdx.x; e < rows * cols; e += CTA_THREADS) {
+  for (int e = team_tid(); e < rows * cols; e += team_threads()) {
     int i = e / cols, j = e % cols;
     cplx h = cconj(H[(int64_t)j * rows + i]), s = cconj(S[(int64_t)j * rows + i]);
     out[e] = csub(cmul(z, s), h);
   }
-  __syncthreads();
-}
-
-// Max of v over the CTA (NaN-free inputs); begins and ends with a barrier.
-NEGF_DEV double cta_max(double v, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double m = red[0];
-  for (int w = 1; w < CTA_THREADS / 32; ++w) m = fmax(m, red[w]);
-  __syncthreads();
-  return m;
+  team_sync();
 }
 
 // C = alpha op(A) op(B) (+ beta D when D is given).  By default conventional 4M complex products
@@ -63,8 +49,8 @@ NEGF_DEV int cta_lu_inverse(cplx* W, cplx* out, int n, char* smem_raw) {
   const int64_t n2 = (int64_t)n * n;
   const int f = cta_lu_factor(W, n, n, smem_raw);
   const int* perm = cta_lu_perm(smem_raw, n);
-  for (int64_t e = threadIdx.x; e < n2; e += CTA_THREADS) out[e] = cmk(perm[e / n] == e % n ? 1.0 : 0.0, 0.0);
-  __syncthreads();
+  for (int64_t e = team_tid(); e < n2; e += team_threads()) out[e] = cmk(perm[e / n] == e % n ? 1.0 : 0.0, 0.0);
+  team_sync();
   cta_lu_trsolve(W, n, n, out, n, n, smem_raw);
   return f;
 }

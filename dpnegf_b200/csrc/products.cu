@@ -13,7 +13,13 @@
 // decimation.  Sums over energies run in a fixed order, so
 // results are bitwise reproducible.
 #include "../../include/negf_b200.h"
-#include "lead_forms.cuh"
+#include "lead_adjoint.cuh"
+#include "team_launch.cuh"
+
+namespace negf_team {
+int lead_adjoint_launch(const NegfLeadAdjProblem& p, size_t smem, int slots, int cl, cudaStream_t s);
+int lead_adjoint_fit(size_t smem, int cl);
+}
 
 namespace NEGF_NS {
 
@@ -93,160 +99,6 @@ __global__ void gamma_sum_parts_kernel(double* out, const double* part, int64_t 
     for (int z = 1; z < split; ++z) s += part[(size_t)z * n2 + e];
     out[e] = s;
   }
-}
-
-// ---------------------------------------------------------------------------------------------
-// Lead adjoint.  Per energy (z = E + i eta, tau = z S01 - H01, tau' = z S01^H - H01^H, g = g_s):
-//   V = dL/dg from Sigma(g):  form 0  Sigma = L g[:b,:b] R,  L = E S_DL - H_DL, R = E S_DL^H - H_DL^H
-//                                      V[:b,:b] = L^H Gs R^H,  dL/dL = Gs R^H g_b^H,  dL/dR = g_b^H L^H Gs
-//                             form 1  Sigma = g^-1:           V = -g^-H Gs g^-H
-//                             form 2  Sigma = E S - H - g^-1: V = +g^-H Gs g^-H, dS += conj(E) Gs, dH -= Gs
-//   Lambda = V + P^H Lambda Q^H with P = g tau, Q = tau' g, by doubling
-//            (Lambda += P^H Lambda Q^H, P <- P^2, Q <- Q^2 until max|P| max|Q| < tol)
-//   F = (zS - H - tau g tau')^-1, dW = -F^H Lambda F^H
-//   dS += conj(z) dW, dH -= dW, dtau = -dW (g tau')^H, dtau' = -(tau g)^H dW,
-//   dS01 += conj(z) dtau + z dtau'^H, dH01 -= dtau + dtau'^H
-// (PyTorch's convention: the gradient of a real loss w.r.t. a complex tensor is dL/d conj(x)).
-// Energies go to the CTAs round-robin; each CTA sums its energies' contributions in its own slot,
-// and a second kernel sums the slots in slot order.
-
-constexpr int LA_NACC = 6, LA_NWORK = 12;
-
-__host__ __device__ inline int la_max_n(const NegfLead& ld) { return ld.nc > ld.n ? ld.nc : ld.n; }
-
-__host__ __device__ inline size_t la_slot_elems(const NegfLeadAdjProblem& p) {
-  const size_t mn = (size_t)la_max_n(p.lead);
-  return ((LA_NACC + LA_NWORK) * mn * mn + 15) & ~(size_t)15;
-}
-
-__host__ __device__ inline int64_t la_grad_elems(const NegfLeadAdjProblem& p) {
-  const int64_t n = p.lead.n, ncb = p.form == 0 ? (int64_t)p.lead.nc * p.lead.b : 0;
-  return 4 * n * n + 2 * ncb;
-}
-
-NEGF_DEV void la_item(const NegfLeadAdjProblem& P, int idx, cplx* slot, char* smem_raw, double* red) {
-  cplx* smem = reinterpret_cast<cplx*>(smem_raw);
-  const NegfLead ld = P.lead;
-  const int n = ld.n;
-  const int64_t n2 = (int64_t)n * n;
-  const size_t mn = (size_t)la_max_n(ld), mn2 = mn * mn;
-  const NegfLeadAdjItem it = P.items[idx];
-  const cplx* ar = reinterpret_cast<const cplx*>(P.arena);
-  const cplx *H = ar + ld.h, *S = ar + ld.s, *H01 = ar + ld.h01, *S01 = ar + ld.s01;
-  const cplx* g = reinterpret_cast<const cplx*>(it.gs);
-  const cplx* Gs = reinterpret_cast<const cplx*>(it.gsig);
-  const cplx E = cmk(it.e_re, it.e_im);
-  const cplx z = cmk(it.e_re, it.e_im + P.eta);
-  const cplx ONE = cmk(1.0, 0.0), MONE = cmk(-1.0, 0.0);
-  cplx* acc[LA_NACC];
-  for (int r = 0; r < LA_NACC; ++r) acc[r] = slot + r * mn2;
-  cplx* w_[LA_NWORK];
-  for (int r = 0; r < LA_NWORK; ++r) w_[r] = slot + (LA_NACC + r) * mn2;
-  cplx *lam = w_[0], *Pm = w_[1], *Qm = w_[2], *P2 = w_[3], *Q2 = w_[4], *T1 = w_[5];
-  cplx *tau = w_[6], *taup = w_[7], *Y1 = w_[8], *W = w_[9], *F = w_[10], *gW = w_[11];
-  int bad = 0;
-
-  // ---- V = dL/dg into lam
-  for (int64_t e = threadIdx.x; e < n2; e += CTA_THREADS) lam[e] = cmk(0.0, 0.0);
-  __syncthreads();
-  if (P.form == 0) {
-    const int nc = ld.nc, b = ld.b;
-    const cplx *hdl = ar + ld.hdl, *sdl = ar + ld.sdl;
-    cplx *Lm = Pm, *Rm = Qm, *T2 = P2, *gL = Q2, *gR = Y1;
-    for (int e = threadIdx.x; e < nc * b; e += CTA_THREADS) Lm[e] = csub(cmul(E, sdl[e]), hdl[e]);
-    __syncthreads();
-    form_eS_minus_h_herm(Rm, hdl, sdl, E, b, nc);                       // b x nc
-    gemm_ls<OP_C, OP_N, true>(smem, b, nc, nc, Lm, b, Gs, nc, T1, nc);        // L^H Gs       (b x nc)
-    gemm_ls<OP_N, OP_C, true>(smem, b, b, nc, T1, nc, Rm, nc, lam, n);        // V[:b,:b]
-    gemm_ls<OP_N, OP_C, true>(smem, nc, b, nc, Gs, nc, Rm, nc, T2, b);        // Gs R^H       (nc x b)
-    gemm_ls<OP_N, OP_C, true>(smem, nc, b, b, T2, b, g, n, gL, b);            // dL/dL        (nc x b)
-    gemm_ls<OP_C, OP_N, true>(smem, b, nc, b, g, n, T1, nc, gR, nc);          // dL/dR        (b x nc)
-    const cplx Ec = cconj(E);
-    for (int e = threadIdx.x; e < nc * b; e += CTA_THREADS) {
-      const int i = e / b, j = e % b;
-      const cplx l = gL[e], rH = cconj(gR[(int64_t)j * nc + i]);
-      acc[4][e] = csub(acc[4][e], cadd(l, rH));                          // H_DL
-      acc[5][e] = cadd(acc[5][e], cadd(cmul(Ec, l), cmul(E, rH)));      // S_DL
-    }
-    __syncthreads();
-  } else {
-    for (int64_t e = threadIdx.x; e < n2; e += CTA_THREADS) F[e] = g[e];
-    __syncthreads();
-    bad |= cta_lu_inverse(F, W, n, smem_raw);                           // W = g^-1
-    gemm_ls<OP_C, OP_N, true>(smem, n, n, n, W, n, Gs, n, T1, n);             // g^-H Gs
-    gemm_ls<OP_N, OP_C, true>(smem, n, n, n, T1, n, W, n, lam, n, nullptr, 0, P.form == 1 ? MONE : ONE);
-    if (P.form == 2) {
-      const cplx Ec = cconj(E);
-      for (int64_t e = threadIdx.x; e < n2; e += CTA_THREADS) {
-        acc[0][e] = csub(acc[0][e], Gs[e]);
-        acc[2][e] = cadd(acc[2][e], cmul(Ec, Gs[e]));
-      }
-      __syncthreads();
-    }
-  }
-
-  // ---- Lambda by doubling
-  cta_shift_form<true>(tau, H01, S01, z, MONE, (int)n2, smem);                // z S01 - H01
-  form_eS_minus_h_herm(taup, H01, S01, z, n, n);                        // z S01^H - H01^H
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, g, n, tau, n, Pm, n);              // P = g tau
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, taup, n, g, n, Qm, n);             // Q = tau' g
-  int steps = 0;
-  bool finite = true;
-  for (int s = 0; s < P.max_iter; ++s) {
-    steps = s + 1;
-    gemm_ls<OP_C, OP_N, true>(smem, n, n, n, Pm, n, lam, n, T1, n);           // P^H Lambda
-    gemm_ls<OP_N, OP_C, true>(smem, n, n, n, T1, n, Qm, n, lam, n, lam, n);   // Lambda += ... Q^H
-    gemm_ls<OP_N, OP_N, true>(smem, n, n, n, Pm, n, Pm, n, P2, n);
-    gemm_ls<OP_N, OP_N, true>(smem, n, n, n, Qm, n, Qm, n, Q2, n);
-    cplx* t = Pm; Pm = P2; P2 = t;
-    t = Qm; Qm = Q2; Q2 = t;
-    double mp = 0.0, mq = 0.0;
-    for (int64_t e = threadIdx.x; e < n2; e += CTA_THREADS) {
-      const double a = hypot(Pm[e].x, Pm[e].y), c = hypot(Qm[e].x, Qm[e].y);
-      mp = (a == a) ? fmax(mp, a) : INFINITY;
-      mq = (c == c) ? fmax(mq, c) : INFINITY;
-    }
-    mp = cta_max(mp, red);
-    mq = cta_max(mq, red);
-    if (!isfinite(mp) || !isfinite(mq)) { finite = false; break; }
-    if (mp * mq < P.tol) break;
-  }
-
-  // ---- F = (zS - H - tau g tau')^-1 and the parameter gradients
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, g, n, taup, n, Y1, n);             // g tau'
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, tau, n, Y1, n, W, n);              // tau g tau'
-  for (int64_t e = threadIdx.x; e < n2; e += CTA_THREADS) W[e] = csub(csub(cmul(z, S[e]), H[e]), W[e]);
-  __syncthreads();
-  bad |= cta_lu_inverse(W, F, n, smem_raw);
-  gemm_ls<OP_C, OP_N, true>(smem, n, n, n, F, n, lam, n, T1, n);              // F^H Lambda
-  gemm_ls<OP_N, OP_C, true>(smem, n, n, n, T1, n, F, n, gW, n, nullptr, 0, MONE);  // dW
-  gemm_ls<OP_N, OP_C, true>(smem, n, n, n, gW, n, Y1, n, T1, n, nullptr, 0, MONE);  // dtau = -dW (g tau')^H
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, tau, n, g, n, Pm, n);              // tau g
-  gemm_ls<OP_C, OP_N, true>(smem, n, n, n, Pm, n, gW, n, Qm, n, nullptr, 0, MONE);  // dtau' = -(tau g)^H dW
-  const cplx zc = cconj(z);
-  for (int64_t e = threadIdx.x; e < n2; e += CTA_THREADS) {
-    const int64_t i = e / n, j = e % n;
-    const cplx dw = gW[e], dt = T1[e], dtpH = cconj(Qm[j * n + i]);
-    acc[0][e] = csub(acc[0][e], dw);                                      // H
-    acc[2][e] = cadd(acc[2][e], cmul(zc, dw));                            // S
-    acc[1][e] = csub(acc[1][e], cadd(dt, dtpH));                          // H01
-    acc[3][e] = cadd(acc[3][e], cadd(cmul(zc, dt), cmul(z, dtpH)));       // S01
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    P.status[idx] = bad ? NEGF_ERR_SINGULAR : (finite ? NEGF_OK : NEGF_ERR_NONFINITE);
-    if (P.iters) P.iters[idx] = steps;
-  }
-}
-
-__global__ void __launch_bounds__(CTA_THREADS, 1) lead_adjoint_kernel(const NegfLeadAdjProblem P) {
-  char* const smem = negf_smem;
-  __shared__ double red[CTA_THREADS / 32];
-  cplx* slot = reinterpret_cast<cplx*>(P.scratch) + (size_t)blockIdx.x * la_slot_elems(P);
-  const size_t mn = (size_t)la_max_n(P.lead);
-  for (size_t e = threadIdx.x; e < LA_NACC * mn * mn; e += CTA_THREADS) slot[e] = cmk(0.0, 0.0);
-  __syncthreads();
-  for (int i = blockIdx.x; i < P.n_items; i += gridDim.x) la_item(P, i, slot, smem, red);
 }
 
 // grad[e] = sum over slots, in slot order, of the slots' accumulators.
@@ -341,7 +193,13 @@ int negf_lead_adjoint_run(const NegfLeadAdjProblem* p, void* stream) {
       cudaSuccess)
     return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
-  negf::lead_adjoint_kernel<<<grid, negf::CTA_THREADS, smem, s>>>(*p);
+  const int cl = negf::team_ctas(ld.n, grid, [&](int c) { return negf_team::lead_adjoint_fit(smem, c); });
+  if (cl > 1) {
+    const int st = negf_team::lead_adjoint_launch(*p, smem, grid, cl, s);
+    if (st != NEGF_OK) return st;
+  } else {
+    negf::lead_adjoint_kernel<<<grid, negf::CTA_THREADS, smem, s>>>(*p);
+  }
   const int64_t total = negf::la_grad_elems(*p);
   const int rgrid = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
   negf::lead_adjoint_sum_kernel<<<rgrid, 256, 0, s>>>(*p, grid);

@@ -1,6 +1,7 @@
 // The C ABI of the RGF sweep (include/negf_b200.h) and its FP64 kernels; the sweep itself is
 // in rgf_sweep.cuh, the mixed-precision kernel in rgf_mx.cu.
 #include "rgf_sweep.cuh"
+#include "team_launch.cuh"
 
 namespace negf_team {
 int rgf_launch_team(int feat, const NegfRgfProblem& p, size_t smem, int slots, int cl, cudaStream_t s);
@@ -8,20 +9,6 @@ int rgf_team_fit(int feat, size_t smem, int cl);
 }
 
 namespace negf {
-
-// CTAs per work slot.  A launch with fewer slots than half the SMs leaves the others idle, so each
-// item gets a cluster of 2, 4 or 8 CTAs while all slots still run at once and the block products
-// have a 32 x 64 output piece for every CTA.
-static int team_ctas(int feat, const NegfRgfProblem& p, size_t smem, int slots) {
-  int dev = 0, sms = 0;
-  if (p.max_n <= 32 || cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return 1;
-  const int pieces = ((p.max_n + 31) / 32) * ((p.max_n + 63) / 64);
-  for (int cl = 8; cl > 1; cl /= 2)
-    if (cl <= pieces && slots * cl <= sms && negf_team::rgf_team_fit(feat, smem, cl) >= slots) return cl;
-  return 1;
-}
 
 int rgf_launch_fp64(int feat, const NegfRgfProblem& p, size_t smem, int grid, cudaStream_t s) {
   if (feat == FEAT_ADJOINT) return rgf_launch_impl<false, FEAT_ADJOINT>(p, smem, grid, s);
@@ -79,7 +66,7 @@ int negf_rgf_run(const NegfRgfProblem* p, void* stream) {
   if (cudaMemsetAsync(p->scratch, 0, negf::RGF_SCRATCH_HEADER, s) != cudaSuccess) return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
   if (!mixed) {
-    const int cl = negf::team_ctas(feat, *p, smem, grid);
+    const int cl = negf::team_ctas(p->max_n, grid, [&](int c) { return negf_team::rgf_team_fit(feat, smem, c); });
     if (cl > 1) return negf_team::rgf_launch_team(feat, *p, smem, grid, cl, s);
     return negf::rgf_launch_fp64(feat, *p, smem, grid, s);
   }

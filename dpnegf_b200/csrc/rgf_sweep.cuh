@@ -181,64 +181,6 @@ NEGF_DEV void form_gamma(cplx* out, const cplx* se, int ns, int r0, int c) {
   }
 }
 
-NEGF_DEV double cta_max(double v, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double s = red[0];
-  for (int w = 1; w < CTA_THREADS / 32; ++w) s = fmax(s, red[w]);
-  __syncthreads();
-  return s;
-}
-
-NEGF_DEV double cta_sum(double v, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double s = 0.0;
-  for (int w = 0; w < CTA_THREADS / 32; ++w) s += red[w];
-  __syncthreads();
-  return s;
-}
-
-#ifdef NEGF_TEAM
-static __shared__ unsigned long long team_slot;  // what the team's other CTAs may read of this one
-
-// v of every CTA's thread 0, folded in rank order by every thread: each sees the same bits.
-template <class F>
-NEGF_DEV double team_fold(double v, F f) {
-  if (threadIdx.x == 0) team_slot = (unsigned long long)__double_as_longlong(v);
-  team_sync();
-  double s = __longlong_as_double((long long)team_peek(&team_slot, 0));
-  for (int r = 1; r < team_size(); ++r) s = f(s, __longlong_as_double((long long)team_peek(&team_slot, r)));
-  team_sync();
-  return s;
-}
-NEGF_DEV double team_max(double v, double* red) {
-  return team_fold(cta_max(v, red), [](double x, double y) { return fmax(x, y); });
-}
-NEGF_DEV double team_sum(double v, double* red) {
-  return team_fold(cta_sum(v, red), [](double x, double y) { return x + y; });
-}
-// rank 0's value of v (uniform in that CTA)
-NEGF_DEV int team_from_first(int v) {
-  if (threadIdx.x == 0) team_slot = (unsigned long long)(unsigned)v;
-  team_sync();
-  const int f = (int)(unsigned)team_peek(&team_slot, 0);
-  team_sync();
-  return f;
-}
-#else
-NEGF_DEV double team_max(double v, double* red) { return cta_max(v, red); }
-NEGF_DEV double team_sum(double v, double* red) { return cta_sum(v, red); }
-#endif
-
 // C = alpha op(A) op(B) (+ beta D) on the FP64 DMMA GEMM, or on the tcgen05
 // 3xTF32 GEMM when MX.
 template <int OPA, int OPB, bool MX>

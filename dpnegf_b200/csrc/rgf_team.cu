@@ -3,6 +3,7 @@
 // pass, repeat the in-register leaves of the inverse, and meet at cluster barriers.
 #define NEGF_TEAM
 #include "rgf_sweep.cuh"
+#include "team_launch.cuh"
 
 namespace negf_team {
 
@@ -14,39 +15,10 @@ static SweepKernel team_kernel(int feat) {
   return rgf_kernel<false, FEAT_RETARDED>;
 }
 
-static void team_config(cudaLaunchConfig_t& c, cudaLaunchAttribute& a, size_t smem, int slots, int cl, cudaStream_t s) {
-  a.id = cudaLaunchAttributeClusterDimension;
-  a.val.clusterDim.x = (unsigned)cl;
-  a.val.clusterDim.y = a.val.clusterDim.z = 1;
-  c = cudaLaunchConfig_t{};
-  c.gridDim = dim3((unsigned)(slots * cl));
-  c.blockDim = dim3(CTA_THREADS);
-  c.dynamicSmemBytes = smem;
-  c.stream = s;
-  c.attrs = &a;
-  c.numAttrs = 1;
-}
-
-int rgf_team_fit(int feat, size_t smem, int cl) {
-  cudaLaunchConfig_t c;
-  cudaLaunchAttribute a;
-  team_config(c, a, smem, 1, cl, nullptr);
-  int n = 0;
-  if (cudaFuncSetAttribute(team_kernel(feat), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, team_kernel(feat), &c) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return n;
-}
+int rgf_team_fit(int feat, size_t smem, int cl) { return negf::team_fit(team_kernel(feat), smem, cl); }
 
 int rgf_launch_team(int feat, const NegfRgfProblem& p, size_t smem, int slots, int cl, cudaStream_t s) {
-  cudaLaunchConfig_t c;
-  cudaLaunchAttribute a;
-  team_config(c, a, smem, slots, cl, s);
-  if (cudaFuncSetAttribute(team_kernel(feat), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return NEGF_ERR_CUDA;
-  return cudaLaunchKernelEx(&c, team_kernel(feat), p) == cudaSuccess ? NEGF_OK : NEGF_ERR_CUDA;
+  return negf::team_launch(team_kernel(feat), p, smem, slots, cl, s);
 }
 
 }  // namespace negf_team

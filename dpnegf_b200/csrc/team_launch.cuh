@@ -1,0 +1,61 @@
+// Host side of the cluster launches.
+#pragma once
+#include <cuda_runtime.h>
+#include "../../include/negf_b200.h"
+
+namespace negf {
+
+// CTAs per work slot.  A launch with fewer slots than half the SMs leaves the others idle, so each
+// slot gets a cluster of 2, 4 or 8 CTAs while all slots still run at once (fit(c): clusters of c
+// that fit the GPU together) and an n x n product has a 32 x 64 output piece for every CTA.
+template <class Fit>
+inline int team_ctas(int n, int slots, Fit fit) {
+  int dev = 0, sms = 0;
+  if (n <= 32 || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  const int pieces = ((n + 31) / 32) * ((n + 63) / 64);
+  for (int cl = 8; cl > 1; cl /= 2)
+    if (cl <= pieces && slots * cl <= sms && fit(cl) >= slots) return cl;
+  return 1;
+}
+
+inline void team_config(cudaLaunchConfig_t& c, cudaLaunchAttribute& a, size_t smem, int slots, int cl, cudaStream_t s) {
+  a.id = cudaLaunchAttributeClusterDimension;
+  a.val.clusterDim.x = (unsigned)cl;
+  a.val.clusterDim.y = a.val.clusterDim.z = 1;
+  c = cudaLaunchConfig_t{};
+  c.gridDim = dim3((unsigned)(slots * cl));
+  c.blockDim = dim3(256);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &a;
+  c.numAttrs = 1;
+}
+
+// Clusters of `cl` CTAs that run at once; 0 when the GPU cannot run them.
+template <class Problem>
+inline int team_fit(void (*kernel)(const Problem), size_t smem, int cl) {
+  cudaLaunchConfig_t c;
+  cudaLaunchAttribute a;
+  team_config(c, a, smem, 1, cl, nullptr);
+  int n = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &c) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+template <class Problem>
+inline int team_launch(void (*kernel)(const Problem), const Problem& p, size_t smem, int slots, int cl, cudaStream_t s) {
+  cudaLaunchConfig_t c;
+  cudaLaunchAttribute a;
+  team_config(c, a, smem, slots, cl, s);
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return NEGF_ERR_CUDA;
+  return cudaLaunchKernelEx(&c, kernel, p) == cudaSuccess ? NEGF_OK : NEGF_ERR_CUDA;
+}
+
+}  // namespace negf
