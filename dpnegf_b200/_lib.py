@@ -191,6 +191,8 @@ def load():
     lib.negf_pack_run.restype = ctypes.c_int
     lib.negf_pack_run.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p,
                                   ctypes.c_void_p]
+    lib.negf_rgf_slots_per_sm.restype = ctypes.c_int
+    lib.negf_rgf_slots_per_sm.argtypes = [ctypes.c_int]
     lib.negf_sm_count.restype = ctypes.c_int
     lib.negf_sm_count.argtypes = []
     lib.negf_version.restype = ctypes.c_char_p

@@ -18,11 +18,16 @@ namespace NEGF_NS {
 #ifndef NEGF_GT_K
 #define NEGF_GT_K 16
 #endif
+constexpr int CTA_THREADS = TEAM_THREADS_PER_CTA;
+#ifdef NEGF_SMALL
+constexpr int GT_M = 32, GT_N = 32, GT_K = NEGF_GT_K;
+#else
 constexpr int GT_M = 64, GT_N = 64, GT_K = NEGF_GT_K;
+#endif
 static_assert(GT_K == 16 || GT_K == 32, "k slab of 16 or 32");
 constexpr int PITCH_MK = GT_K + 4;  // [64 rows][GT_K k] tiles (pitch = 4 mod 8)
 constexpr int PITCH_KN = GT_N + 2;  // [GT_K k][64 cols] tiles (pitch = 2 mod 8)
-constexpr int GT_LOADS = GT_M * GT_K / 256;  // 16-byte copies per thread per operand tile
+constexpr int GT_LOADS = GT_M * GT_K / CTA_THREADS;  // 16-byte copies per thread per operand tile
 constexpr int GT_TILE = (GT_M * PITCH_MK > GT_K * PITCH_KN) ? GT_M * PITCH_MK : GT_K * PITCH_KN;
 #ifndef NEGF_GT_STAGES
 #define NEGF_GT_STAGES 3
@@ -33,7 +38,6 @@ constexpr int GT_TILE = (GT_M * PITCH_MK > GT_K * PITCH_KN) ? GT_M * PITCH_MK : 
 constexpr int GT_STAGES = NEGF_GT_STAGES;
 static_assert(GT_STAGES == 3 || GT_STAGES == 4, "3- or 4-stage ring");
 constexpr int GEMM_SMEM_BYTES = 2 * GT_STAGES * GT_TILE * (int)sizeof(cplx);  // stages x (A,B)
-constexpr int CTA_THREADS = 256;
 
 struct GemmArgs {
   int M, N, K;
@@ -101,7 +105,7 @@ NEGF_DEV void load_b_tile(cplx* sB, const GemmArgs& g, int k0, int n0, int tid) 
       const cplx* src = v ? g.B + (int64_t)n * g.ldb + k : g.B;
       cp_async16(sB + r * PITCH_MK + c, src, v);
     } else {  // stored B is K x N: tile rows k, cols n
-      int r = e >> 6, c = e & 63;
+      int r = e / GT_N, c = e % GT_N;
       int k = k0 + r, n = n0 + c;
       bool v = (k < g.K) && (n < g.N);
       const cplx* src = v ? g.B + (int64_t)k * g.ldb + n : g.B;

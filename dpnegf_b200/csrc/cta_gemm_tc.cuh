@@ -49,7 +49,9 @@ constexpr int TC_SMEM_BYTES = 4 * TC_STAGE_BYTES;
 constexpr int TC_TMEM_COLS = 512;
 constexpr int TC_EPI_PITCH = 17;                               // complex entries per transposed row
 constexpr long long TC_WAIT_CYCLES = 4000000000LL;             // about two seconds
+#ifndef NEGF_SMALL
 static_assert(CTA_THREADS == 256, "the tensor-core GEMM assumes 256-thread CTAs");
+#endif
 static_assert(8 * 32 * TC_EPI_PITCH * 16 <= 2 * TC_STAGE_BYTES, "epilogue transpose buffers fit in the planes area");
 static_assert(TC_M * TC_KC * 16 + TC_N * TC_KC * 16 == TC_STAGE_BYTES, "a raw slab pair fills one stage");
 

@@ -407,6 +407,13 @@ NEGF_DEV cplx crcp_scaled(cplx a) {
   return cmk(x * r, -y * r);
 }
 
+// f(integral_constant<int, 0>) ... f(integral_constant<int, N - 1>)
+template <int N, class F>
+NEGF_DEV void static_groups(F f) {
+  if constexpr (N > 1) static_groups<N - 1>(f);
+  f(std::integral_constant<int, N - 1>());
+}
+
 // Inverse of a block of n <= 64 held in registers, W -> G: blocked Gauss-Jordan with implicit
 // partial pivoting (the in-place transform of the form above, PW columns to a panel).
 //
@@ -423,13 +430,12 @@ NEGF_DEV cplx crcp_scaled(cplx a) {
 // at n = 128 324 -> 219 us, at 256 1278 -> 1072.
 template <int RA, int CW, int PW>
 __device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, cplx* G, int64_t ldg) {
-  constexpr int NM = 32 * RA, NSUB = CW / PW, NPAN = 8 * NSUB;
-  static_assert(NSUB == 1 || NSUB == 2, "one or two panels per warp");
+  constexpr int NM = 32 * RA, NSUB = CW / PW, NW = CTA_THREADS / 32, NPAN = NW * NSUB;
   cplx* pan = smem_cplx();                      // [NPAN][PW][NM] factorised panels
-  cplx* rows = pan + NPAN * PW * NM;                                  // [8 warps][PW][PW] pivot-row entries
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(rows + 8 * PW * PW);  // [NPAN] panel published
-  int* piv = reinterpret_cast<int*>(bar + NPAN);                      // [8 CW] logical column -> physical row
-  int* pinv = piv + 8 * CW;                                           // [NM] physical row -> logical column
+  cplx* rows = pan + NPAN * PW * NM;                                  // [NW warps][PW][PW] pivot-row entries
+  unsigned long long* bar = reinterpret_cast<unsigned long long*>(rows + NW * PW * PW);  // [NPAN] panel published
+  int* piv = reinterpret_cast<int*>(bar + NPAN);                      // [NW CW] logical column -> physical row
+  int* pinv = piv + NW * CW;                                          // [NM] physical row -> logical column
   int* flag = pinv + NM;                                              // [0] singular pivot, [1] a panel never came
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   cplx x[RA][CW];
@@ -560,35 +566,32 @@ __device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, c
   };
 
   constexpr std::integral_constant<int, 0> G0{};
-  constexpr std::integral_constant<int, NSUB - 1> GL{};
   bool lost = false;
-  if (warp == 0) factor(G0);
-  for (int w0 = 0; w0 < 8 && CW * w0 < n; ++w0) {
-    const int c0 = CW * w0, c1 = c0 + PW;
-    if (warp != w0) {
-      lost |= !mbar_wait_once(bar + c0 / PW);
+  // Panel g of warp w0: the owner factorises it (its first panel it has factorised already) and
+  // applies it to its other column groups; the next panel's owner goes ahead after its first group.
+  auto panel = [&](auto g_c, int w0) {
+    constexpr int g = decltype(g_c)::value;
+    const int c0 = CW * w0 + PW * g;
+    if (c0 >= n || lost) return;
+    if (warp == w0) {
+      if constexpr (g > 0) factor(g_c);
+      static_groups<NSUB>([&](auto h_c) {
+        if constexpr (decltype(h_c)::value != g) apply(h_c, c0);
+      });
+    } else {
+      const bool ok = mbar_wait_once(bar + c0 / PW);
       __syncwarp();
-      if (__any_sync(0xffffffffu, lost)) break;
+      lost = !__all_sync(0xffffffffu, ok);
+      if (lost) return;
       apply(G0, c0);
-      if (NSUB == 1 && warp == w0 + 1) factor(G0);
+      if (g == NSUB - 1 && warp == w0 + 1) factor(G0);
+      static_groups<NSUB>([&](auto h_c) {
+        if constexpr (decltype(h_c)::value != 0) apply(h_c, c0);
+      });
     }
-    if constexpr (NSUB == 2) {
-      apply(GL, c0);
-      if (c1 < n) {
-        if (warp == w0) {
-          factor(GL);
-          apply(G0, c1);
-        } else {
-          lost |= !mbar_wait_once(bar + c1 / PW);
-          __syncwarp();
-          if (__any_sync(0xffffffffu, lost)) break;
-          apply(G0, c1);
-          if (warp == w0 + 1) factor(G0);
-          apply(GL, c1);
-        }
-      }
-    }
-  }
+  };
+  if (warp == 0) factor(G0);
+  for (int w0 = 0; w0 < NW; ++w0) static_groups<NSUB>([&](auto g_c) { panel(g_c, w0); });
   if (lost) flag[1] = 1;
   __syncthreads();
   // G[i][j] = W[p(i)][p^-1(j)] (every CTA of a team holds the same result; one stores it)
@@ -632,14 +635,20 @@ NEGF_DEV int cta_inverse(cplx* W, int64_t ldw, int n, cplx* G, int64_t ldg, char
   // FP32-accurate products amplify every rounding of the leaves, so its results would move.
   if constexpr (!TC) {
     if (n <= 64) {
+#ifdef NEGF_SMALL
+      const int f = n <= 8    ? cta_inverse_reg<1, 4, 4>(W, ldw, n, G, ldg)
+                    : n <= 16 ? cta_inverse_reg<1, 8, 4>(W, ldw, n, G, ldg)
+                              : cta_inverse_reg<1, 16, 4>(W, ldw, n, G, ldg);  // n <= 32
+#else
       const int f = n <= 16   ? cta_inverse_reg<1, 2, 2>(W, ldw, n, G, ldg)
                     : n <= 32 ? cta_inverse_reg<1, 4, 4>(W, ldw, n, G, ldg)
                               : cta_inverse_reg<2, 8, 4>(W, ldw, n, G, ldg);
+#endif
       pc->mark(PH_INV_PANEL);
       return f;
     }
   }
-#ifdef NEGF_TEAM
+#if defined(NEGF_TEAM) || defined(NEGF_SMALL)
   return 1;  // not reached: a team's larger blocks go through the block inverse or one CTA's pivoted form
 #else
   return cta_inverse_pivoted<G3, TC>(W, ldw, n, G, ldg, smem_raw, pc, snap, ob);

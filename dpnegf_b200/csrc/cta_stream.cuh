@@ -11,7 +11,7 @@
 
 namespace NEGF_NS {
 
-constexpr int STREAM_CHUNK = 2048;
+constexpr int STREAM_CHUNK = 8 * TEAM_THREADS_PER_CTA;
 constexpr int STREAM_SMEM_BYTES = 4 * STREAM_CHUNK * (int)sizeof(cplx);
 
 // out[e] = alpha * (X[e] - z * Y[e]) for e < count; a null X or Y is zero.
@@ -31,8 +31,8 @@ NEGF_DEV void cta_shift_form(cplx* out, const cplx* X, const cplx* Y, cplx z, cp
   auto issue = [&](int c) {
     const int base = (team_rank() + c * team_size()) * STREAM_CHUNK;
 #pragma unroll
-    for (int s = 0; s < STREAM_CHUNK / 256; ++s) {
-      const int k = tid + s * 256, e = base + k;
+    for (int s = 0; s < STREAM_CHUNK / TEAM_THREADS_PER_CTA; ++s) {
+      const int k = tid + s * TEAM_THREADS_PER_CTA, e = base + k;
       const bool v = e < count;
       if (X) cp_async16(sx[c & 1] + k, v ? X + e : X, v);
       if (Y) cp_async16(sy[c & 1] + k, v ? Y + e : Y, v);
@@ -46,8 +46,8 @@ NEGF_DEV void cta_shift_form(cplx* out, const cplx* X, const cplx* Y, cplx z, cp
     cp_async_wait<1>();
     const int base = (team_rank() + c * team_size()) * STREAM_CHUNK;
 #pragma unroll
-    for (int s = 0; s < STREAM_CHUNK / 256; ++s) {
-      const int k = tid + s * 256, e = base + k;
+    for (int s = 0; s < STREAM_CHUNK / TEAM_THREADS_PER_CTA; ++s) {
+      const int k = tid + s * TEAM_THREADS_PER_CTA, e = base + k;
       if (e < count) {
         cplx x = X ? lds_after_wait(sx[c & 1] + k) : cmk(0.0, 0.0);
         cplx y = Y ? lds_after_wait(sy[c & 1] + k) : cmk(0.0, 0.0);

@@ -11,16 +11,23 @@
 
 // The CTA building blocks and the sweep compile twice: one CTA per work item (namespace negf), and,
 // with NEGF_TEAM, a thread-block cluster per item (namespace negf_team), whose CTAs split the output
-// tiles and the elementwise passes and repeat the small serial parts.
-#ifdef NEGF_TEAM
+// tiles and the elementwise passes and repeat the small serial parts.  NEGF_SMALL compiles the sweep
+// a third time, for blocks of up to 32: CTAs of two warps with 32 x 32 tiles, three to an SM.
+#if defined(NEGF_TEAM)
 #define NEGF_NS negf_team
+#elif defined(NEGF_SMALL)
+#define NEGF_NS negf_small
 #else
 #define NEGF_NS negf
 #endif
 
 namespace NEGF_NS {
 
-constexpr int TEAM_THREADS_PER_CTA = 256;
+#ifdef NEGF_SMALL
+constexpr int TEAM_THREADS_PER_CTA = 64, MIN_CTAS = 3;
+#else
+constexpr int TEAM_THREADS_PER_CTA = 256, MIN_CTAS = 1;
+#endif
 #ifdef NEGF_TEAM
 NEGF_DEV int team_rank() {
   uint32_t r;

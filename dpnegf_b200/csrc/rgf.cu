@@ -8,6 +8,10 @@ int rgf_launch_team(int feat, const NegfRgfProblem& p, size_t smem, int slots, i
 int rgf_team_fit(int feat, size_t smem, int cl);
 }
 
+namespace negf_small {
+int rgf_launch_small(int feat, const NegfRgfProblem& p, int grid, cudaStream_t s);
+}
+
 namespace negf {
 
 int rgf_launch_fp64(int feat, const NegfRgfProblem& p, size_t smem, int grid, cudaStream_t s) {
@@ -68,10 +72,14 @@ int negf_rgf_run(const NegfRgfProblem* p, void* stream) {
   if (!mixed) {
     const int cl = negf::team_ctas(p->max_n, grid, [&](int c) { return negf_team::rgf_team_fit(feat, smem, c); });
     if (cl > 1) return negf_team::rgf_launch_team(feat, *p, smem, grid, cl, s);
+    // more slots than SMs are asked for only where three small CTAs share one (negf_rgf_slots_per_sm)
+    if (p->max_n <= 32 && grid > negf_sm_count()) return negf_small::rgf_launch_small(feat, *p, grid, s);
     return negf::rgf_launch_fp64(feat, *p, smem, grid, s);
   }
   return negf::rgf_launch_mx(*p, smem, grid, s);  // one mixed instantiation with every feature
 }
+
+int negf_rgf_slots_per_sm(int max_n) { return max_n <= 32 ? 3 : 1; }
 
 int negf_sm_count(void) {
   int dev = 0, n = 0;

@@ -1034,7 +1034,7 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
 }
 
 template <bool MX, int FEAT>
-__global__ void __launch_bounds__(CTA_THREADS, 1) rgf_kernel(const NegfRgfProblem P) {
+__global__ void __launch_bounds__(CTA_THREADS, MIN_CTAS) rgf_kernel(const NegfRgfProblem P) {
   char* const smem = negf_smem;
   __shared__ unsigned long long s_item;
   __shared__ double red[CTA_THREADS / 32];
@@ -1069,7 +1069,6 @@ inline size_t rgf_smem_bytes(int max_n, bool mixed) {
   size_t m = a > b ? a : b;
   return m > c ? m : c;
 }
-static_assert(CTA_THREADS == 256, "cta_stream.cuh assumes 256-thread CTAs");
 
 
 #ifdef NEGF_TEAM

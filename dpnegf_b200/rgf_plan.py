@@ -478,7 +478,8 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     orbar_t = torch.zeros(max(orb_cursor, 1), dtype=torch.float64, device=dev) if orb_ar else None
     status_t = torch.empty(max(item_cursor, 1), dtype=torch.int32, device=dev)
     if n_slots is None:
-        n_slots = max(1, min(n_items, lib.negf_sm_count()))
+        per_sm = lib.negf_rgf_slots_per_sm(geom.max_n) if precision == "fp64" else 1
+        n_slots = max(1, min(n_items, per_sm * lib.negf_sm_count()))
     prob = _lib.NegfRgfProblem()
     prob.blocks = blocks_t.data_ptr()
     prob.devices = devs_t.data_ptr()

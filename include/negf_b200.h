@@ -355,6 +355,10 @@ size_t negf_rgf_static_scratch_bytes(void);
 int negf_pack_run(const NegfPackPiece* pieces, int32_t n_pieces, int64_t max_count, double* arena, int32_t* nonzero,
                   void* cuda_stream);
 
+/* Work slots worth having per SM for blocks of up to max_n in an FP64 sweep: small blocks run on two-warp
+   CTAs, three to an SM, when a launch has more slots in use than SMs. */
+int negf_rgf_slots_per_sm(int max_n);
+
 /* Number of SMs of the current CUDA device (grid sizing helper). */
 int negf_sm_count(void);
 
