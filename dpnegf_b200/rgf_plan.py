@@ -478,8 +478,13 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     orbar_t = torch.zeros(max(orb_cursor, 1), dtype=torch.float64, device=dev) if orb_ar else None
     status_t = torch.empty(max(item_cursor, 1), dtype=torch.int32, device=dev)
     if n_slots is None:
-        per_sm = lib.negf_rgf_slots_per_sm(geom.max_n) if precision == "fp64" else 1
-        n_slots = max(1, min(n_items, per_sm * lib.negf_sm_count()))
+        sms = lib.negf_sm_count()
+        n_slots = max(1, min(n_items, sms))
+        # small blocks: several slots per SM, while their scratch stays a sixteenth of the GPU's memory
+        per_sm = lib.negf_rgf_slots_per_sm(geom.max_n) if precision == "fp64" and not adjoint else 1
+        slot_bytes = 16 * (20 * geom.max_n ** 2 + 4 * geom.max_g_slab)
+        if per_sm > 1 and per_sm * sms * slot_bytes <= torch.cuda.get_device_properties(dev).total_memory // 16:
+            n_slots = max(1, min(n_items, per_sm * sms))
     prob = _lib.NegfRgfProblem()
     prob.blocks = blocks_t.data_ptr()
     prob.devices = devs_t.data_ptr()
@@ -527,10 +532,11 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     need = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
     try:
         scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
-    except torch.cuda.OutOfMemoryError:
-        if prob.flags == flags:
+    except torch.cuda.OutOfMemoryError:  # do without the kept L g and the extra slots
+        fewer = min(n_slots, lib.negf_sm_count())
+        if prob.flags == flags and fewer == n_slots:
             raise
-        prob.flags = flags
+        prob.flags, prob.n_slots, n_slots = flags, fewer, fewer
         need = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
         scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
     prob.scratch = scratch.data_ptr()

@@ -113,3 +113,36 @@ def test_packed_arena_equals_the_blocks():
     b = g.blocks
     assert b[0]["su"] == b[0]["sl"] == b[0]["suT"] == b[0]["slT"] == -1
     assert all(b[1][k] >= 0 for k in ("hu", "hl", "su", "sl", "suT", "slT")) and b[0]["hu"] >= 0
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 16, 17, 24, 31, 32])
+def test_small_ctas_agree_with_large(n):
+    """More items than SMs with blocks of up to 32 run on two-warp CTAs; the same sweep with fewer
+    slots runs on eight-warp ones.  Only the order of reductions and of the inverse's panels differs
+    (TOL); n at the edges of the inverse's 8, 16 and 32-wide layouts."""
+    from dpnegf_b200 import rgf_plan
+    dims = [n, max(1, n - 1), n, n]
+    hd, hu, hl, sd, su, sl, (seL, seR) = _device(dims, 300 + n)
+    t = lambda x: torch.as_tensor(np.ascontiguousarray(x), dtype=torch.complex128, device="cuda")
+    ts = lambda xs: [t(x) for x in xs]
+    geom = rgf_plan.Geometry([rgf_plan.DeviceBlocks(ts(hd), ts(hu), ts(hl), ts(sd), ts(su), ts(sl))])
+    B = 460
+    E = [torch.linspace(-0.7, 0.9, B, dtype=torch.float64).cuda()]
+    L, R = [t(seL).expand(B, -1, -1)], [t(seR).expand(B, -1, -1)]
+    s_in = [[torch.ones(B, 1, 1, dtype=torch.complex128, device="cuda") * t(np.eye(m)) for m in dims]]
+    for kw in (dict(outputs=(), trans=True, dos=True, orb_g=True, orb_ar=True),
+               dict(outputs=("grd", "gru"), trans=True, s_in=s_in)):
+        a = rgf_plan.run(geom, E, L, R, eta=ETA, **kw)
+        b = rgf_plan.run(geom, E, L, R, eta=ETA, n_slots=100, **kw)
+        same = lambda x, y: float((x - y).abs().max()) <= TOL * float(y.abs().max())
+        for key in ("trans", "dos", "orb_g", "orb_ar"):
+            if getattr(a, key) is not None:
+                assert same(getattr(a, key), getattr(b, key)), key
+        for tag in a.blocks[0]:
+            for x, y in zip(a.blocks[0][tag], b.blocks[0][tag]):
+                assert same(x, y), tag
+    w = torch.linspace(0.2, 1.0, B, dtype=torch.float64)
+    g = [rgf_plan.run(geom, E, L, R, eta=ETA, outputs=(), adjoint_w=w, adjoint_w_dos=w, n_slots=m).grads for m in (B, 100)]
+    for key in ("hd", "hu", "sd", "sl"):
+        for x, y in zip(g[0][key], g[1][key]):
+            assert same(x, y), key
