@@ -110,7 +110,7 @@ NEGF_DEV void lu_laswp(const LuCtx& c, cplx* col0, int64_t ld, int ncols, int ka
 // rank-1 update writes one place to the left, so that no register index depends on the column.  The
 // multipliers go to shared memory, where the row swaps reach them.  Two barriers per column, for
 // the pivot candidates of the warps and for the two rows that trade places (with the panel in shared
-// memory and every operand read from it, a column took 3000-3400 cycles; now about 1200).
+// memory and every operand read from it, a column took 3000-3400 cycles; now 2300-2700).
 template <int NB, int RT, int WID>
 NEGF_DEV void lu_panel_steps(const LuCtx& c, cplx (&x)[RT][NB], cplx* P, cplx* rows, int r0, int m, int j0, int j1) {
   constexpr int PP = LuLayout<NB>::PP;
