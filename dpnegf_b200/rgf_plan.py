@@ -33,6 +33,14 @@ class DeviceBlocks:
         return [int(h.shape[-1]) for h in self.hd]
 
 
+def _packable(copies, device):
+    """Whether the one-launch pack takes these (offset, tensor) pieces: it loads whole 16-byte entries, while
+    complex128 memory that torch did not allocate (DLPack, ``__cuda_array_interface__``) may start at any
+    multiple of 8."""
+    return bool(copies) and all(t.device == device and t.dtype == C128 and t.ndim == 2 and t.numel() > 0
+                                and not t.is_neg() and t.data_ptr() % 16 == 0 for _, t in copies)
+
+
 class Geometry:
     """Packed H/S arena + block table for a list of devices (energy independent).
 
@@ -141,11 +149,11 @@ class Geometry:
                     self.blocks[bi][name] = -1
 
     def _pack(self, copies):
-        """Every block into the arena in one launch, when all are 2-D complex128 tensors of this GPU;
-        returns the per-piece nonzero flags, or None when the blocks go one by one."""
+        """Every block into the arena in one launch, when all are 2-D complex128 tensors of this GPU at
+        16-byte aligned addresses; returns the per-piece nonzero flags, or None when the blocks go one
+        by one."""
         hs = self.hs
-        if not copies or any(t.device != hs.device or t.dtype != C128 or t.ndim != 2 or t.numel() == 0 or t.is_neg()
-                             for _, t in copies):
+        if not _packable(copies, hs.device):
             return None
         tab = np.zeros(len(copies), dtype=_lib.PACK_DTYPE)
         tab["src"] = [t.data_ptr() for _, t in copies]

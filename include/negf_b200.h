@@ -184,7 +184,7 @@ typedef struct NegfRgfProblem {
 
 /* One block to copy: dst[i * cols + j] = src[i * row_stride + j * col_stride], conjugated if conj. */
 typedef struct NegfPackPiece {
-  const double* src;          /* complex128, device memory */
+  const double* src;          /* complex128, device memory, 16-byte aligned */
   int64_t dst;                /* element offset in the arena */
   int64_t row_stride, col_stride; /* in complex elements */
   int32_t rows, cols;
