@@ -36,9 +36,12 @@ class DeviceBlocks:
 def _packable(copies, device):
     """Whether the one-launch pack takes these (offset, tensor) pieces: it loads whole 16-byte entries, while
     complex128 memory that torch did not allocate (DLPack, ``__cuda_array_interface__``) may start at any
-    multiple of 8."""
-    return bool(copies) and all(t.device == device and t.dtype == C128 and t.ndim == 2 and t.numel() > 0
-                                and not t.is_neg() and t.data_ptr() % 16 == 0 for _, t in copies)
+    multiple of 8.  Tensors without an address of their own (inside torch.func transforms) are copied."""
+    try:
+        return bool(copies) and all(t.device == device and t.dtype == C128 and t.ndim == 2 and t.numel() > 0
+                                    and not t.is_neg() and t.data_ptr() % 16 == 0 for _, t in copies)
+    except RuntimeError:
+        return False
 
 
 class Geometry:

@@ -32,3 +32,17 @@ def test_other_blocks_are_not_packed():
     assert not rgf_plan._packable([(0, t[:0])], CPU)
     assert not rgf_plan._packable([(0, torch._neg_view(t))], CPU)
     assert not rgf_plan._packable([(0, t)], torch.device("meta"))
+
+
+def test_tensors_of_a_function_transform_are_not_packed():
+    """Inside torch.func.grad and jvp a tensor has no address; the copy path takes it."""
+    seen = []
+
+    def f(x):
+        seen.append(rgf_plan._packable([(0, x)], CPU))
+        return x.abs().sum()
+
+    t = torch.ones(2, 2, dtype=torch.complex128)
+    torch.func.grad(f)(t)
+    torch.func.jvp(f, (t,), (t,))
+    assert seen == [False, False]
