@@ -154,9 +154,9 @@ class Geometry:
     def _pack(self, copies):
         """Every block into the arena in one launch, when all are 2-D complex128 tensors of this GPU at
         16-byte aligned addresses; returns the per-piece nonzero flags, or None when the blocks go one
-        by one."""
+        by one (also under stream capture, where the piece table cannot be uploaded)."""
         hs = self.hs
-        if not _packable(copies, hs.device):
+        if torch.cuda.is_current_stream_capturing() or not _packable(copies, hs.device):
             return None
         tab = np.zeros(len(copies), dtype=_lib.PACK_DTYPE)
         tab["src"] = [t.data_ptr() for _, t in copies]

@@ -1,0 +1,25 @@
+"""How calls reach the kernels: packing under stream capture."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def test_geometry_is_built_under_capture():
+    """With detect_zero_offdiag=False a Geometry of device tensors reads nothing back, so it can be captured; a
+    replay packs the blocks' new values."""
+    from dpnegf_b200 import rgf_plan
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    r = lambda *s: torch.complex(*(torch.randn(*s, generator=gen, dtype=torch.float64, device="cuda") for _ in range(2)))
+    parts = [[r(3, 3), r(5, 5)], [r(3, 5)], [r(5, 3)], [r(3, 3), r(5, 5)], [r(3, 5)], [r(5, 3)]]
+    build = lambda: rgf_plan.Geometry([rgf_plan.DeviceBlocks(*parts)], detect_zero_offdiag=False)
+    build()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        geom = build()
+    for t in (t for p in parts for t in p):
+        t.copy_(r(*t.shape))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(geom.hs, build().hs)
