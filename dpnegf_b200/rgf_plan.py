@@ -69,6 +69,7 @@ class Geometry:
 
         self.max_n = 0
         self.max_g_slab = 0
+        self.max_blocks = 0
         for d in devices:
             K = len(d.hd)
             if not (len(d.sd) == K and len(d.hu) == len(d.hl) == len(d.su) == len(d.sl) == K - 1):
@@ -125,7 +126,7 @@ class Geometry:
             dv["g_slab"] = g
             devs.append(dv)
             self.max_g_slab = max(self.max_g_slab, g)
-            self.max_blocks = max(getattr(self, "max_blocks", 0), K)
+            self.max_blocks = max(self.max_blocks, K)
             self.col_slab = max(getattr(self, "col_slab", 0), gc)
             self.u_slab = max(getattr(self, "u_slab", 0), gu)
         if self.max_n > _lib.NEGF_MAX_BLOCK:

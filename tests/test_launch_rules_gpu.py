@@ -1,4 +1,4 @@
-"""How calls reach the kernels: packing under stream capture."""
+"""How calls reach the kernels: packing under stream capture, empty problems."""
 import pytest
 import torch
 
@@ -23,3 +23,15 @@ def test_geometry_is_built_under_capture():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(geom.hs, build().hs)
+
+
+def test_no_devices():
+    """A plan over no devices launches nothing and has empty results; a direct call is refused."""
+    from dpnegf_b200 import _lib, rgf_plan
+    kw = dict(eta=1e-5, outputs=(), trans=True, dos=True)
+    plan = rgf_plan.run(rgf_plan.Geometry([]), [], [], [], defer=True, **kw)
+    plan.launch()
+    plan.check()
+    assert plan.result.trans.numel() == plan.result.dos.numel() == 0 and plan.result.blocks == []
+    with pytest.raises(_lib.NegfError, match="invalid argument"):
+        rgf_plan.run(rgf_plan.Geometry([]), [], [], [], **kw)
