@@ -541,11 +541,18 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
         prob.flags = flags | _lib.KEEP_LG
         if lib.negf_rgf_scratch_bytes(ctypes.byref(prob)) > torch.cuda.get_device_properties(dev).total_memory // 4:
             prob.flags = flags
+    # the gradient accumulators first: only what is left is there for the kept L g and the extra slots
+    grad_t = None
+    if adjoint:
+        grad_slab = 2 * int(geom.devs[0]["g_slab"]) + 4 * int(geom.u_slab)
+        grad_t = torch.zeros((n_slots, max(grad_slab, 1)), dtype=C128, device=dev)
+        prob.grad = grad_t.data_ptr()
+        prob.grad_slab = grad_slab
     need = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
     try:
         scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
-    except torch.cuda.OutOfMemoryError:  # do without the kept L g and the extra slots
-        fewer = min(n_slots, lib.negf_sm_count())
+    except torch.cuda.OutOfMemoryError:  # do without them
+        fewer = n_slots if adjoint else min(n_slots, lib.negf_sm_count())
         if prob.flags == flags and fewer == n_slots:
             raise
         prob.flags, prob.n_slots, n_slots = flags, fewer, fewer
@@ -553,18 +560,6 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
         scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
     prob.scratch = scratch.data_ptr()
     prob.scratch_bytes = scratch.numel()
-    grad_t = None
-    if adjoint:
-        g_slab = int(geom.devs[0]["g_slab"])
-        grad_slab = 2 * g_slab + 4 * int(geom.u_slab)
-        grad_t = torch.zeros((n_slots, max(grad_slab, 1)), dtype=C128, device=dev)
-        prob.grad = grad_t.data_ptr()
-        prob.grad_slab = grad_slab
-        need = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
-        if need > scratch.numel():
-            scratch = torch.empty(need, dtype=torch.uint8, device=dev)
-            prob.scratch = scratch.data_ptr()
-            prob.scratch_bytes = scratch.numel()
     phase_t = None
     if phase:
         phase_t = torch.zeros((n_slots, len(_lib.PHASES)), dtype=torch.int64, device=dev)

@@ -1,4 +1,5 @@
-"""How calls reach the kernels: packing under stream capture, empty problems."""
+"""How calls reach the kernels: packing under stream capture, empty problems, little
+memory."""
 import pytest
 import torch
 
@@ -35,3 +36,40 @@ def test_no_devices():
     assert plan.result.trans.numel() == plan.result.dos.numel() == 0 and plan.result.blocks == []
     with pytest.raises(_lib.NegfError, match="invalid argument"):
         rgf_plan.run(rgf_plan.Geometry([]), [], [], [], **kw)
+
+
+def _device(K, n, B, seed):
+    from dpnegf_b200 import rgf_plan, workload
+    d = workload.random_device(n, K, seed=seed)
+    geom = rgf_plan.Geometry([rgf_plan.DeviceBlocks(d.hd, d.hu, d.hl, d.sd, d.su, d.sl)])
+    E = workload.energy_grid(B).to(torch.complex128).cuda()
+    seL, seR = (workload.random_self_energy(B, n, seed=seed + k).cuda() for k in (1, 2))
+    return geom, [E], [seL], [seR]
+
+
+def test_gradient_fits_where_only_the_kept_products_do_not():
+    """Memory for everything but half of the kept L g: the gradient call does without it.  L g alone is one
+    product regrouped, so the results agree to rounding."""
+    from dpnegf_b200 import rgf_plan
+    K, n, B = 64, 64, 80
+    args = _device(K, n, B, 40)
+    w = torch.linspace(0.2, 1.0, B, dtype=torch.float64)
+    run = lambda: rgf_plan.run(*args, eta=1e-3, outputs=(), adjoint_w=w)
+    run()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    want = run()
+    peak = torch.cuda.max_memory_allocated()
+    want = want.trans.clone(), [x.clone() for x in want.grads["hd"]]
+    torch.cuda.empty_cache()
+    kept = B * K * n * n * 16
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((peak - kept // 2) / total)
+    try:
+        got = run()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert float((got.trans - want[0]).abs().max()) <= 1e-10 * float(want[0].abs().max())
+    for x, y in zip(got.grads["hd"], want[1]):
+        assert float((x - y).abs().max()) <= 1e-10 * float(y.abs().max())
