@@ -196,7 +196,9 @@ def check_status(status: torch.Tensor):
 
 @dataclass
 class RgfPlan:
-    """A prepared sweep (``run(..., defer=True)``): descriptors, scratch and outputs stay allocated."""
+    """A prepared sweep (``run(..., defer=True)``): descriptors, scratch and outputs stay allocated.  Of the
+    scratch, what only makes the sweep faster is at most a 1/PLAN_EXTRA of the GPU's memory twice (extra
+    slots, kept L g)."""
     prob: object
     keep: list
     n_items: int
@@ -226,6 +228,9 @@ class RgfResult:
     orb_ar: Optional[torch.Tensor] = None   # concatenated per-item [n_orb] diag(G_qN Gamma_R G_qN^H)
     grads: Optional[dict] = None            # adjoint: block gradients and per-energy dT/dSigma
 
+
+# Bound on each optional part of a deferred plan's scratch: memory / 256, 0.7 GB of a B200.
+PLAN_EXTRA = 256
 
 _FAMILY = {  # output tag -> (flag, block field, shape fn (n_q, n_next, n_last))
     "grd": (_lib.OUT_GRD, "o_grd", lambda n, nn, nl: (n, n), False),
@@ -489,13 +494,18 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     orbg_t = torch.empty(max(orb_cursor, 1), dtype=C128, device=dev) if orb_g else None
     orbar_t = torch.zeros(max(orb_cursor, 1), dtype=torch.float64, device=dev) if orb_ar else None
     status_t = torch.empty(max(item_cursor, 1), dtype=torch.int32, device=dev)
+    # Memory for speed alone, extra slots for small blocks and a kept L g: a call gives it back when it
+    # returns; a deferred plan holds it beside other plans and tensors, so it takes little.
+    memory = torch.cuda.get_device_properties(dev).total_memory
+    sms = lib.negf_sm_count()
     if n_slots is None:
-        sms = lib.negf_sm_count()
         n_slots = max(1, min(n_items, sms))
         # small blocks: several slots per SM, while their scratch stays a sixteenth of the GPU's memory
         per_sm = lib.negf_rgf_slots_per_sm(geom.max_n) if precision == "fp64" and not adjoint else 1
         slot_bytes = 16 * (20 * geom.max_n ** 2 + 4 * geom.max_g_slab)
-        if per_sm > 1 and per_sm * sms * slot_bytes <= torch.cuda.get_device_properties(dev).total_memory // 16:
+        fits = (per_sm - 1) * sms * slot_bytes <= memory // PLAN_EXTRA if defer else \
+            per_sm * sms * slot_bytes <= memory // 16
+        if per_sm > 1 and fits:
             n_slots = max(1, min(n_items, per_sm * sms))
     prob = _lib.NegfRgfProblem()
     prob.blocks = blocks_t.data_ptr()
@@ -533,13 +543,15 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     if inverse not in ("gj", "block"):
         raise ValueError(f"inverse must be 'gj' or 'block', not {inverse!r}")
     prob.inv_mode = 1 if inverse == "block" else 0
-    # L g kept for the backward sweep: one block product of eight less, while its slab leaves the
+    # L g kept for the backward sweep: one block product of nine less, while its slab leaves the
     # scratch within a quarter of the GPU's memory
     if precision == "fp64" and not (lesser or greater or ckpt or adjoint_w_dos is not None) and geom.max_blocks > 1 \
             and flags & (_lib.OUT_GRD | _lib.OUT_GRL | _lib.OUT_GRU | _lib.DOS | _lib.ORB_DOS | _lib.ORB_GDIAG
                          | _lib.ADJOINT):
+        need = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
         prob.flags = flags | _lib.KEEP_LG
-        if lib.negf_rgf_scratch_bytes(ctypes.byref(prob)) > torch.cuda.get_device_properties(dev).total_memory // 4:
+        kept = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
+        if kept - need > memory // PLAN_EXTRA if defer else kept > memory // 4:
             prob.flags = flags
     # the gradient accumulators first: only what is left is there for the kept L g and the extra slots
     grad_t = None

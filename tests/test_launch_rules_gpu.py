@@ -73,3 +73,22 @@ def test_gradient_fits_where_only_the_kept_products_do_not():
     assert float((got.trans - want[0]).abs().max()) <= 1e-10 * float(want[0].abs().max())
     for x, y in zip(got.grads["hd"], want[1]):
         assert float((x - y).abs().max()) <= 1e-10 * float(y.abs().max())
+
+
+@pytest.mark.parametrize("K,n,keeps", [(4, 64, True), (96, 64, False)])
+def test_deferred_plan_keeps_little(K, n, keeps):
+    """A deferred plan holds its scratch for its life: L g is kept where it is small, and only there."""
+    from dpnegf_b200 import _lib, rgf_plan
+    sms = _lib.load().negf_sm_count()
+    plan = rgf_plan.run(*_device(K, n, sms, 41), eta=1e-3, outputs=(), trans=True, dos=True, defer=True)
+    kept = sms * K * n * n * 16
+    assert (kept <= torch.cuda.get_device_properties(0).total_memory // rgf_plan.PLAN_EXTRA) == keeps
+    assert bool(plan.prob.flags & _lib.KEEP_LG) == keeps
+
+
+@pytest.mark.parametrize("K,n,many", [(4, 8, True), (64, 32, False)])
+def test_deferred_plan_takes_extra_slots_where_they_are_small(K, n, many):
+    from dpnegf_b200 import _lib, rgf_plan
+    sms = _lib.load().negf_sm_count()
+    plan = rgf_plan.run(*_device(K, n, 3 * sms, 42), eta=1e-3, outputs=(), trans=True, dos=True, defer=True)
+    assert plan.prob.n_slots == (3 * sms if many else sms)
