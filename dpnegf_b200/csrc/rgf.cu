@@ -70,7 +70,11 @@ int negf_rgf_run(const NegfRgfProblem* p, void* stream) {
   if (cudaMemsetAsync(p->scratch, 0, negf::RGF_SCRATCH_HEADER, s) != cudaSuccess) return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
   if (!mixed) {
-    const int cl = negf::team_ctas(p->max_n, grid, [&](int c) { return negf_team::rgf_team_fit(feat, smem, c); });
+    // The pivoted inverse of a block above 64 runs on one CTA, with outer updates of inv_ob columns that a
+    // cluster could not split: a problem that asks for it throughout takes one CTA per item.
+    const bool pivoted = p->inv_mode == 0 && p->max_n > 64;
+    const int cl =
+        pivoted ? 1 : negf::team_ctas(p->max_n, grid, [&](int c) { return negf_team::rgf_team_fit(feat, smem, c); });
     if (cl > 1) return negf_team::rgf_launch_team(feat, *p, smem, grid, cl, s);
     // more slots than SMs are asked for only where three small CTAs share one (negf_rgf_slots_per_sm)
     if (p->max_n <= 32 && grid > negf_sm_count()) return negf_small::rgf_launch_small(feat, *p, grid, s);

@@ -287,9 +287,10 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     ``inverse="gj"`` uses the pivoted Gauss-Jordan inverse throughout; by
     default the autotuned scheme for this GPU, block size and precision, else
     "block".
-    ``inv_ob`` is the inverse's outer block width (32..512); by default the
+    ``inv_ob`` is the pivoted inverse's outer block width (32..512); by default the
     autotuned value for this GPU, block size and precision (``autotune.lookup``),
-    else 128.
+    else 128.  The block inverse uses it in its fallback, except where few items
+    run on clusters of CTAs (whose fallback takes the whole block at once).
     ``checkpoint`` (adjoint only): 0 keeps every left-connected g_q of an item in its scratch slot;
     s > 0 keeps g_0, g_s, g_2s, ... and one segment of s blocks, recomputing each segment from its
     checkpoint when the backward sweep and the adjoint pass reach it (``"sqrt"``: s = ceil(sqrt(K))),

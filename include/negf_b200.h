@@ -147,8 +147,9 @@ typedef struct NegfRgfProblem {
   double* orb_ar;           /* per-orbital diag(G_qN Gamma_R G_qN^H), offset NegfItem.orb (NEGF_ORB_AR) */
   int32_t* status;          /* [n_items] per-item status (always written) */
   uint32_t flags;
-  int32_t n_slots;          /* concurrent work slots; each runs on one CTA, or (FP64) on a cluster of 2, 4 or
-                               8 CTAs when the slots in use leave that many SMs free */
+  int32_t n_slots;          /* concurrent work slots; each runs on one CTA, or (FP64, max_n > 32, and not with
+                               inv_mode 0 and max_n > 64) on a cluster of 2, 4 or 8 CTAs when the slots in use
+                               leave that many SMs free */
   void* scratch;            /* >= negf_rgf_scratch_bytes(problem) bytes, 256-aligned */
   size_t scratch_bytes;
   unsigned long long* phase_cycles; /* optional [n_slots x NEGF_PHASES] SM-cycle counters; NULL = off */
@@ -162,7 +163,9 @@ typedef struct NegfRgfProblem {
   int32_t refine_steps;     /* NEGF_REFINE: at most this many refinement steps (<= 0 means 1); an item
                                stops early once the correction to G_1N is below 1e-10 relative */
   int32_t inv_ob;           /* Gauss-Jordan outer block width: 32, 64, 128, 256 or 512 columns (0 = 128);
-                               results agree to rounding, the speed depends on block size and precision */
+                               results agree to rounding, the speed depends on block size and precision.
+                               inv_mode 1 uses it when a block falls back to Gauss-Jordan, except in a
+                               cluster, where the fallback takes the whole block at once */
   const double* s_out;      /* complex128 arena of Sigma^out blocks (NEGF_GREATER) */
   int32_t inv_mode;         /* 0: Gauss-Jordan with partial pivoting over the whole block (inv_ob);
                                1: recursive 2x2 block inverse, pivoting only inside 64-wide leaves and

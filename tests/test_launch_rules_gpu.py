@@ -92,3 +92,15 @@ def test_deferred_plan_takes_extra_slots_where_they_are_small(K, n, many):
     sms = _lib.load().negf_sm_count()
     plan = rgf_plan.run(*_device(K, n, 3 * sms, 42), eta=1e-3, outputs=(), trans=True, dos=True, defer=True)
     assert plan.prob.n_slots == (3 * sms if many else sms)
+
+
+def test_outer_block_width_is_honoured_with_few_items():
+    """inverse="gj" runs with the outer block width it is given, however few the items: two widths sum in two
+    orders, so they agree to rounding (TOL of test_rgf_gpu's blocks) and not bitwise."""
+    from dpnegf_b200 import rgf_plan
+    args = _device(3, 160, 2, 43)
+    grd = [rgf_plan.run(*args, eta=1e-3, outputs=("grd",), inverse="gj", inv_ob=ob).blocks[0]["grd"][0]
+           for ob in (32, 64, 128)]
+    for x in grd[1:]:
+        assert not torch.equal(x, grd[0])
+        assert float((x - grd[0]).abs().max()) <= 1e-10 * float(grd[0].abs().max())
