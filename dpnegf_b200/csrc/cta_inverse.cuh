@@ -29,6 +29,7 @@
 // produced.  Two barriers per column.
 #pragma once
 #include "cta_gemm_tc.cuh"
+#include "item_status.cuh"
 
 namespace NEGF_NS {
 
@@ -423,7 +424,8 @@ NEGF_DEV void static_groups(F f) {
 //     x[i][j] = (i a pivot of the panel ? 0 : x[i][j]) + sum_s P[i][s] v_s,   v_s = x[p_s][j],
 // where the pivot rows' entries are exchanged inside the warp.  Every panel has its own slot in
 // shared memory, so the warps need not be in step.  The pivot is the row whose |re| + |im| has the
-// largest leading 32 bits (within 2^-20 of the largest), the lowest lane among equals.
+// largest leading 32 bits (within 2^-20 of the largest), the lowest lane among equals.  Returns the
+// flags of item_status.cuh.
 // Bound by the latency of the panel chain (per column a reduction, a reciprocal and a rank-1 step
 // of PW columns).  Against the blocked form with 8-wide panels in shared memory, every SM inverting
 // its own matrices: n = 16 22.7 -> 7.4 us, 32 47 -> 17, 64 108 -> 57; the block inverse built on it
@@ -604,7 +606,7 @@ __device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, c
         if (i < n && c < n) G[(int64_t)pinv[i] * ldg + piv[c]] = x[a][j];
       }
   }
-  const int f = flag[0] | flag[1];
+  const int f = (flag[0] ? INV_SINGULAR : 0) | (flag[1] ? INV_LOST : 0);
   if (tid < NPAN) mbar_inval(bar + tid);
   team_sync();
   return f;

@@ -353,7 +353,7 @@ struct EpiGrad {
 // (null for q = 0), and with dgq its z-tangent dg_q from dgprev.  Uses the slot's W, T1, Lz, Uz
 // and tA..tE; leaves L_{q-1}, U_{q-1} in Lz, Uz for the lesser and greater steps, and
 // L_{q-1} g_{q-1} in lg (T1 when null; the tangent reads it from T1).  Inlined into the sweep; the checkpointed adjoint recomputes its segments
-// through the non-inlined copy below.  Returns the singular-pivot flag.
+// through the non-inlined copy below.  Returns the flags of the inverse (item_status.cuh).
 template <bool MX>
 NEGF_DEV int forward_block_body(const NegfRgfProblem& P, const NegfItem& it, const SlotBufs& sb,
                                 char* smem_raw, double* red, PhaseClock& pc, int q,
@@ -1023,11 +1023,9 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
   if (team_tid() == 0) {
     if (fl & NEGF_TRANS) P.trans[it.out] = tval;
     if (fl & NEGF_DOS) P.dos[it.out] = dos_total;
-    int st = NEGF_OK;
-    if (bad) st = NEGF_ERR_SINGULAR;
-    else if (MX && tc_err) st = NEGF_ERR_TIMEOUT;
-    else if (!isfinite(tval) || !isfinite(dos_total)) st = NEGF_ERR_NONFINITE;
-    P.status[it.out] = st;
+    bool tc_lost = false;
+    if constexpr (MX) tc_lost = tc_err != 0;
+    P.status[it.out] = item_status(bad, tc_lost, isfinite(tval) && isfinite(dos_total));
   }
   team_sync();
   pc.mark(PH_TRANS);

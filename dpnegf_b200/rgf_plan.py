@@ -190,7 +190,7 @@ def check_status(status: torch.Tensor):
             raise torch.linalg.LinAlgError(
                 f"RGF: a left-connected block is singular (item {bad}); the matrix is not invertible")
         if code == _lib.NEGF_ERR_TIMEOUT:
-            raise _lib.NegfError(f"RGF: a tensor-core completion wait expired (item {bad})")
+            raise _lib.NegfError(f"RGF: a bounded wait inside the kernel expired (item {bad})")
         raise _lib.NegfError(f"RGF failed for item {bad} with status {code}")
 
 

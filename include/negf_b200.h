@@ -36,7 +36,8 @@ extern "C" {
 #define NEGF_ERR_LS_RESIDUAL 3      /* residual >= 3e-5: surface_green.py:154 (ArithmeticError) */
 #define NEGF_ERR_SINGULAR 4         /* zero / non-finite pivot (torch.linalg.solve raises) */
 #define NEGF_ERR_NONFINITE 5        /* non-finite result */
-#define NEGF_ERR_TIMEOUT 6          /* a bounded tensor-core completion wait expired (NEGF_MIXED) */
+#define NEGF_ERR_TIMEOUT 6          /* a bounded wait inside the kernel expired (tensor-core completion in
+                                       NEGF_MIXED, a panel of the in-register inverse in FP64) */
 #define NEGF_ERR_ARGUMENT -1        /* malformed descriptor (call-level) */
 #define NEGF_ERR_UNSUPPORTED -2     /* block size above the compiled maximum (call-level) */
 #define NEGF_ERR_CUDA -3            /* CUDA launch / attribute error (call-level) */
