@@ -188,6 +188,8 @@ def load():
     lib.negf_rgf_scratch_bytes.argtypes = [ctypes.POINTER(NegfRgfProblem)]
     lib.negf_rgf_run.restype = ctypes.c_int
     lib.negf_rgf_run.argtypes = [ctypes.POINTER(NegfRgfProblem), ctypes.c_void_p]
+    lib.negf_rgf_run_ctas.restype = ctypes.c_int
+    lib.negf_rgf_run_ctas.argtypes = [ctypes.POINTER(NegfRgfProblem), ctypes.c_int32, ctypes.c_void_p]
     lib.negf_pack_run.restype = ctypes.c_int
     lib.negf_pack_run.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p,
                                   ctypes.c_void_p]
@@ -202,6 +204,8 @@ def load():
     lib.negf_lopez_sancho_scratch_bytes.argtypes = [ctypes.POINTER(NegfLsProblem)]
     lib.negf_lopez_sancho_run.restype = ctypes.c_int
     lib.negf_lopez_sancho_run.argtypes = [ctypes.POINTER(NegfLsProblem), ctypes.c_void_p]
+    lib.negf_lopez_sancho_run_ctas.restype = ctypes.c_int
+    lib.negf_lopez_sancho_run_ctas.argtypes = [ctypes.POINTER(NegfLsProblem), ctypes.c_int32, ctypes.c_void_p]
     lib.negf_gamma_sum_scratch_bytes.restype = ctypes.c_size_t
     lib.negf_gamma_sum_scratch_bytes.argtypes = [ctypes.POINTER(NegfGammaSum)]
     lib.negf_gamma_sum_run.restype = ctypes.c_int
@@ -210,6 +214,8 @@ def load():
     lib.negf_lead_adjoint_scratch_bytes.argtypes = [ctypes.POINTER(NegfLeadAdjProblem)]
     lib.negf_lead_adjoint_run.restype = ctypes.c_int
     lib.negf_lead_adjoint_run.argtypes = [ctypes.POINTER(NegfLeadAdjProblem), ctypes.c_void_p]
+    lib.negf_lead_adjoint_run_ctas.restype = ctypes.c_int
+    lib.negf_lead_adjoint_run_ctas.argtypes = [ctypes.POINTER(NegfLeadAdjProblem), ctypes.c_int32, ctypes.c_void_p]
     _lib = lib
     return lib
 

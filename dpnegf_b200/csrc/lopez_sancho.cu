@@ -20,7 +20,9 @@ size_t negf_lopez_sancho_scratch_bytes(const NegfLsProblem* p) {
   return negf::LS_SCRATCH_HEADER + (size_t)p->n_slots * negf::ls_slot_elems(*p) * sizeof(double2);
 }
 
-int negf_lopez_sancho_run(const NegfLsProblem* p, void* stream) {
+int negf_lopez_sancho_run(const NegfLsProblem* p, void* stream) { return negf_lopez_sancho_run_ctas(p, 0, stream); }
+
+int negf_lopez_sancho_run_ctas(const NegfLsProblem* p, int32_t ctas, void* stream) {
   if (!p || !p->leads || !p->items || !p->arena || !p->status || !p->scratch) return NEGF_ERR_ARGUMENT;
   if (p->n_items <= 0) return NEGF_OK;
   if (p->max_n <= 0 || p->n_slots <= 0 || p->max_iter < 0) return NEGF_ERR_ARGUMENT;
@@ -31,10 +33,11 @@ int negf_lopez_sancho_run(const NegfLsProblem* p, void* stream) {
   const size_t smem = negf::ls_smem_bytes(p->max_n);
   if (cudaFuncSetAttribute(negf::ls_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return NEGF_ERR_CUDA;
-  if (cudaMemsetAsync(p->scratch, 0, negf::LS_SCRATCH_HEADER, s) != cudaSuccess) return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
   // a 2n x 2n product per step: one 32 x 64 piece for every CTA
-  const int cl = negf::team_ctas(2 * p->max_n, grid, [&](int c) { return negf_team::ls_fit(smem, c); });
+  const int cl = negf::team_choice(ctas, 2 * p->max_n, grid, [&](int c) { return negf_team::ls_fit(smem, c); });
+  if (cl < 0) return NEGF_ERR_ARGUMENT;
+  if (cudaMemsetAsync(p->scratch, 0, negf::LS_SCRATCH_HEADER, s) != cudaSuccess) return NEGF_ERR_CUDA;
   if (cl > 1) return negf_team::ls_launch(*p, smem, grid, cl, s);
   negf::ls_kernel<<<grid, negf::CTA_THREADS, smem, s>>>(*p);
   return cudaGetLastError() == cudaSuccess ? NEGF_OK : NEGF_ERR_CUDA;

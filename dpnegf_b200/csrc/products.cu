@@ -176,7 +176,9 @@ size_t negf_lead_adjoint_scratch_bytes(const NegfLeadAdjProblem* p) {
   return (size_t)p->n_slots * negf::la_slot_elems(*p) * sizeof(double2);
 }
 
-int negf_lead_adjoint_run(const NegfLeadAdjProblem* p, void* stream) {
+int negf_lead_adjoint_run(const NegfLeadAdjProblem* p, void* stream) { return negf_lead_adjoint_run_ctas(p, 0, stream); }
+
+int negf_lead_adjoint_run_ctas(const NegfLeadAdjProblem* p, int32_t ctas, void* stream) {
   if (!p || !p->arena || !p->items || !p->grad || !p->status || !p->scratch) return NEGF_ERR_ARGUMENT;
   const NegfLead& ld = p->lead;
   if (ld.n <= 0 || p->n_slots <= 0 || p->max_iter < 0 || p->form < 0 || p->form > 2) return NEGF_ERR_ARGUMENT;
@@ -193,7 +195,8 @@ int negf_lead_adjoint_run(const NegfLeadAdjProblem* p, void* stream) {
       cudaSuccess)
     return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
-  const int cl = negf::team_ctas(ld.n, grid, [&](int c) { return negf_team::lead_adjoint_fit(smem, c); });
+  const int cl = negf::team_choice(ctas, ld.n, grid, [&](int c) { return negf_team::lead_adjoint_fit(smem, c); });
+  if (cl < 0) return NEGF_ERR_ARGUMENT;
   if (cl > 1) {
     const int st = negf_team::lead_adjoint_launch(*p, smem, grid, cl, s);
     if (st != NEGF_OK) return st;

@@ -29,7 +29,9 @@ size_t negf_rgf_scratch_bytes(const NegfRgfProblem* p) {
   return negf::RGF_SCRATCH_HEADER + (size_t)p->n_slots * negf::rgf_slot_elems(*p) * sizeof(double2);
 }
 
-int negf_rgf_run(const NegfRgfProblem* p, void* stream) {
+int negf_rgf_run(const NegfRgfProblem* p, void* stream) { return negf_rgf_run_ctas(p, 0, stream); }
+
+int negf_rgf_run_ctas(const NegfRgfProblem* p, int32_t ctas, void* stream) {
   if (!p || !p->blocks || !p->devices || !p->items || !p->hs || !p->status || !p->scratch) return NEGF_ERR_ARGUMENT;
   if (p->n_items <= 0) return NEGF_OK;
   if (p->max_n <= 0 || p->n_slots <= 0) return NEGF_ERR_ARGUMENT;
@@ -67,15 +69,21 @@ int negf_rgf_run(const NegfRgfProblem* p, void* stream) {
   const size_t smem = negf::rgf_smem_bytes(p->max_n, mixed);
   const int feat = (p->flags & NEGF_ADJOINT) ? negf::FEAT_ADJOINT
                    : (p->flags & (NEGF_LESSER | NEGF_GREATER)) ? negf::FEAT_LESSER : negf::FEAT_RETARDED;
-  if (cudaMemsetAsync(p->scratch, 0, negf::RGF_SCRATCH_HEADER, s) != cudaSuccess) return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
-  if (!mixed) {
+  int cl = 1;
+  if (mixed) {
+    if (ctas != 0 && ctas != 1) return NEGF_ERR_ARGUMENT;
+  } else {
     // The pivoted inverse of a block above 64 runs on one CTA, with outer updates of inv_ob columns that a
     // cluster could not split: a problem that asks for it throughout takes one CTA per item.
     const bool pivoted = p->inv_mode == 0 && p->max_n > 64;
-    const int cl =
-        pivoted ? 1 : negf::team_ctas(p->max_n, grid, [&](int c) { return negf_team::rgf_team_fit(feat, smem, c); });
-    if (cl > 1) return negf_team::rgf_launch_team(feat, *p, smem, grid, cl, s);
+    cl = negf::team_choice(ctas == 0 && pivoted ? 1 : ctas, p->max_n, grid,
+                           [&](int c) { return negf_team::rgf_team_fit(feat, smem, c); });
+    if (cl < 0) return NEGF_ERR_ARGUMENT;
+  }
+  if (cudaMemsetAsync(p->scratch, 0, negf::RGF_SCRATCH_HEADER, s) != cudaSuccess) return NEGF_ERR_CUDA;
+  if (cl > 1) return negf_team::rgf_launch_team(feat, *p, smem, grid, cl, s);
+  if (!mixed) {
     // more slots than SMs are asked for only where three small CTAs share one (negf_rgf_slots_per_sm)
     if (p->max_n <= 32 && grid > negf_sm_count()) return negf_small::rgf_launch_small(feat, *p, grid, s);
     return negf::rgf_launch_fp64(feat, *p, smem, grid, s);

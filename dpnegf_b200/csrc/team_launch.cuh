@@ -20,6 +20,15 @@ inline int team_ctas(int n, int slots, Fit fit) {
   return 1;
 }
 
+// The same for a caller's choice: 0 the rule above, 1, 2, 4 or 8 CTAs per slot whatever the slots (clusters
+// that do not fit together wait for each other); -1 when the GPU cannot run it.
+template <class Fit>
+inline int team_choice(int ctas, int n, int slots, Fit fit) {
+  if (ctas == 0) return team_ctas(n, slots, fit);
+  if (ctas == 1) return 1;
+  return (ctas == 2 || ctas == 4 || ctas == 8) && fit(ctas) > 0 ? ctas : -1;
+}
+
 inline void team_config(cudaLaunchConfig_t& c, cudaLaunchAttribute& a, size_t smem, int slots, int cl, cudaStream_t s) {
   a.id = cudaLaunchAttributeClusterDimension;
   a.val.clusterDim.x = (unsigned)cl;

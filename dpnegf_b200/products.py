@@ -117,14 +117,15 @@ def coupling_sigma(g: torch.Tensor, hdl: torch.Tensor, sdl: torch.Tensor, energi
 
 @_lib.on_given_stream
 def lead_adjoint(hL, hLL, sL, sLL, hDL, sDL, E, eta, gs, gsig, form, tol=LEADADJ_TOL, max_iter=LEADADJ_MAX_ITER,
-                 stream=None, info=None):
+                 stream=None, info=None, ctas=0):
     """dL/d(hL, hLL, sL, sLL, hDL, sDL) through Sigma(E) of one lead (PyTorch's complex convention).
 
     ``E`` [B] complex (energy + E_ref), ``gs`` [B, n, n] the converged surface Green's functions at
     E + i eta, ``gsig`` [B, nc, nc] (form 0) or [B, n, n] (forms 1, 2) the incoming gradient of
     Sigma.  form 0: Sigma = (E S_DL - H_DL) g[:b,:b] (E S_DL^H - H_DL^H); 1: Sigma = g^-1;
     2: Sigma = E S - H - g^-1.  Returns six tensors (None for hDL/sDL when not given); a dict
-    passed as ``info`` receives the doubling steps per energy under "iters"."""
+    passed as ``info`` receives the doubling steps per energy under "iters".  ``ctas``: CTAs per work
+    slot (0 lets few energies use the whole GPU, 1 keeps one SM per energy; see ``rgf_plan.run``)."""
     if form not in (0, 1, 2):
         raise ValueError(f"form must be 0, 1 or 2, not {form!r}")
     if form == 0 and hDL is None:
@@ -174,7 +175,8 @@ def lead_adjoint(hL, hLL, sL, sLL, hDL, sDL, E, eta, gs, gsig, form, tol=LEADADJ
     need = lib.negf_lead_adjoint_scratch_bytes(ctypes.byref(p))
     scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
     p.scratch, p.scratch_bytes = scratch.data_ptr(), scratch.numel()
-    _lib.check(lib.negf_lead_adjoint_run(ctypes.byref(p), _lib.stream_handle(stream)), "negf_lead_adjoint_run")
+    _lib.check(lib.negf_lead_adjoint_run_ctas(ctypes.byref(p), int(ctas), _lib.stream_handle(stream)),
+               "negf_lead_adjoint_run")
     st = status.cpu().numpy()
     if info is not None:
         info["iters"] = iters.cpu().numpy()

@@ -203,12 +203,13 @@ class RgfPlan:
     keep: list
     n_items: int
     result: "RgfResult"
+    ctas: int = 0
 
     def launch(self, stream=None):
         """Enqueue the sweep on ``stream`` (default: the current stream).  No host synchronisation and
         no allocation, so the call can be captured in a CUDA graph once the plan has run eagerly."""
         if self.n_items:
-            _lib.check(_lib.load().negf_rgf_run(ctypes.byref(self.prob), _lib.stream_handle(stream)),
+            _lib.check(_lib.load().negf_rgf_run_ctas(ctypes.byref(self.prob), self.ctas, _lib.stream_handle(stream)),
                        "negf_rgf_run")
 
     def check(self):
@@ -256,7 +257,8 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
         s_in: Optional[List[List[Optional[torch.Tensor]]]] = None,
         s_out: Optional[List[List[Optional[torch.Tensor]]]] = None,
         n_slots=None, check=True, stream=None, phase=False, events=None, adjoint_w=None, adjoint_w_dos=None,
-        precision="fp64", refine=False, refine_steps=1, defer=False, inv_ob=None, inverse=None, checkpoint=0):
+        precision="fp64", refine=False, refine_steps=1, defer=False, inv_ob=None, inverse=None, checkpoint=0,
+        ctas=0):
     """Run the batched sweep.
 
     ``energies[d]`` is a 1-D tensor of B_d energies for device d; ``se_l[d]``
@@ -296,6 +298,9 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     checkpoint when the backward sweep and the adjoint pass reach it (``"sqrt"``: s = ceil(sqrt(K))),
     so the g storage per slot is (ceil(K/s) + s) max_n^2 instead of sum n_q^2 (twice that with
     ``adjoint_w_dos``, whose z-tangents are checkpointed alike); results are identical.
+    ``ctas``: CTAs per work slot.  0 lets a launch of few items use clusters of 2, 4 or 8 CTAs and with
+    them the whole GPU; 1 keeps one SM per item, for launches on several streams that should run side by
+    side; 2, 4 or 8 forces clusters of that size (``precision="fp64"`` only).
     ``defer=True`` builds everything but launches nothing and returns an
     ``RgfPlan``: its ``launch()`` re-runs the sweep on the same descriptors,
     scratch and output tensors (a queue reset and one kernel, so it can be
@@ -587,7 +592,7 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     if not defer:
         if events is not None:
             events[0].record(stream)
-        _lib.check(lib.negf_rgf_run(ctypes.byref(prob), _lib.stream_handle(stream)), "negf_rgf_run")
+        _lib.check(lib.negf_rgf_run_ctas(ctypes.byref(prob), int(ctas), _lib.stream_handle(stream)), "negf_rgf_run")
         if events is not None:
             events[1].record(stream)
 
@@ -603,7 +608,7 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
                 dd[tag] = [out_t[off:off + B * s[0] * s[1]].view(B, *s) for off, s, B in v]
         res_blocks.append(dd)
     if defer:
-        return RgfPlan(prob=prob, keep=keep, n_items=n_items, result=RgfResult(
+        return RgfPlan(prob=prob, keep=keep, n_items=n_items, ctas=int(ctas), result=RgfResult(
             trans=trans_t[:item_cursor] if trans else None, orb_dos=orb_t[:orb_cursor] if orb_dos else None,
             dos=dos_t[:item_cursor] if dos else None, status=status_t[:item_cursor], blocks=res_blocks,
             phase_cycles=phase_t, orb_g=orbg_t[:orb_cursor] if orb_g else None,

@@ -100,12 +100,13 @@ class LeadArena:
 
 @_lib.on_given_stream
 def self_energies(arena: LeadArena, lead_index: Sequence[int], energies, eta, E_ref=0.0, want_gs=False,
-                  want_sigma=True, tol=LS_TOL, max_iter=LS_MAX_ITER, check=True, n_slots=None, stream=None):
+                  want_sigma=True, tol=LS_TOL, max_iter=LS_MAX_ITER, check=True, n_slots=None, stream=None, ctas=0):
     """Decimate every (lead_index[i], energies[i]) pair in one launch.
 
     ``energies`` are complex (E relative to ``E_ref``); the decimation uses
     z = E + E_ref + i*eta and the self-energy product E + E_ref (reference
-    :65-86).  ``eta`` is a scalar or per item.  Returns a DecimationResult.
+    :65-86).  ``eta`` is a scalar or per item.  ``ctas``: CTAs per work slot (0 lets few items use the
+    whole GPU, 1 keeps one SM per item; see ``rgf_plan.run``).  Returns a DecimationResult.
     """
     _lib.require_cuda()
     lib = _lib.load()
@@ -146,7 +147,8 @@ def self_energies(arena: LeadArena, lead_index: Sequence[int], energies, eta, E_
     need = lib.negf_lopez_sancho_scratch_bytes(ctypes.byref(p))
     scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
     p.scratch, p.scratch_bytes = scratch.data_ptr(), scratch.numel()
-    _lib.check(lib.negf_lopez_sancho_run(ctypes.byref(p), _lib.stream_handle(stream)), "negf_lopez_sancho_run")
+    _lib.check(lib.negf_lopez_sancho_run_ctas(ctypes.byref(p), int(ctas), _lib.stream_handle(stream)),
+               "negf_lopez_sancho_run")
     st = status.cpu().numpy()
     res = DecimationResult(
         sigma=[sig_buf[sig_off[i]:sig_off[i + 1]].view(sig_sizes[i], sig_sizes[i]) for i in range(B)]

@@ -246,7 +246,7 @@ typedef struct NegfLsProblem {
 /* Bytes of scratch negf_lopez_sancho_run needs for p->n_slots and p->max_n. */
 size_t negf_lopez_sancho_scratch_bytes(const NegfLsProblem* p);
 
-/* Batched Lopez-Sancho decimation over (lead, energy) items, one CTA per item.
+/* Batched Lopez-Sancho decimation over (lead, energy) items, a CTA or a cluster of CTAs per item.
  * Replaces _surface_green_numba_core (negf/surface_green.py:102-159) and the
  * self-energy product of selfEnergy (:9-91):
  *   alpha = h10 - z s10, beta = h01 - z s01, eps = eps_s = H;
@@ -306,7 +306,7 @@ typedef struct NegfLeadAdjProblem {
   double eta;
   double tol;                   /* doubling stops once max|P| max|Q| < tol */
   int32_t max_iter;             /* doubling steps at most */
-  int32_t n_slots;              /* CTAs; energies go to them round-robin */
+  int32_t n_slots;              /* work slots (a CTA or a cluster each); energies go to them round-robin */
   double* grad;                 /* complex128 out: dL/dH, dL/dH01, dL/dS, dL/dS01 [n x n] each, then
                                    dL/dH_DL, dL/dS_DL [nc x b] each for form 0; summed over energies */
   int32_t* status;              /* [n_items] NEGF_OK, NEGF_ERR_SINGULAR, NEGF_ERR_NONFINITE */
@@ -329,6 +329,16 @@ size_t negf_rgf_scratch_bytes(const NegfRgfProblem* p);
  * diagonal (:408-470) are reduced inside the sweep.  Returns a call-level
  * status; per-item status in p->status. */
 int negf_rgf_run(const NegfRgfProblem* p, void* cuda_stream);
+
+/* The same with the CTAs per work slot chosen by the caller, for the three entry points that choose them by
+ * themselves.  ctas = 0 is that choice: clusters of 2, 4 or 8 CTAs when the slots in use leave SMs free, so
+ * that one launch takes the whole GPU; the speed-up is less than the number of CTAs.  1 keeps one CTA (one
+ * SM) per slot: for a caller whose launches on several streams should share the GPU.  2, 4 or 8 forces
+ * clusters of that size (NEGF_ERR_ARGUMENT with NEGF_MIXED, for other values, or where the GPU has no room
+ * for one).  Sweep results agree to rounding, lead results are the same. */
+int negf_rgf_run_ctas(const NegfRgfProblem* p, int32_t ctas, void* cuda_stream);
+int negf_lopez_sancho_run_ctas(const NegfLsProblem* p, int32_t ctas, void* cuda_stream);
+int negf_lead_adjoint_run_ctas(const NegfLeadAdjProblem* p, int32_t ctas, void* cuda_stream);
 
 /* negf_rgf_run for callers that cannot allocate device memory (no counterpart
  * in the reference, which allocates through torch on every call).  A host code
