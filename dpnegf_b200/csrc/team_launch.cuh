@@ -2,25 +2,21 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "../../include/negf_b200.h"
+#include "team_rule.cuh"
 
 namespace negf {
 
-// CTAs per work slot.  A launch with fewer slots than half the SMs leaves the others idle, so each
-// slot gets a cluster of 2, 4 or 8 CTAs while all slots still run at once (fit(c): clusters of c
-// that fit the GPU together) and an n x n product has a 32 x 64 output piece for every CTA.
+// team_rule on the current GPU.
 template <class Fit>
 inline int team_ctas(int n, int slots, Fit fit) {
   int dev = 0, sms = 0;
   if (n <= 32 || cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return 1;
-  const int pieces = ((n + 31) / 32) * ((n + 63) / 64);
-  for (int cl = 8; cl > 1; cl /= 2)
-    if (cl <= pieces && slots * cl <= sms && fit(cl) >= slots) return cl;
-  return 1;
+  return team_rule(n, slots, sms, fit);
 }
 
-// The same for a caller's choice: 0 the rule above, 1, 2, 4 or 8 CTAs per slot whatever the slots (clusters
+// The same for a caller's choice: 0 the rule, 1, 2, 4 or 8 CTAs per slot whatever the slots (clusters
 // that do not fit together wait for each other); -1 when the GPU cannot run it.
 template <class Fit>
 inline int team_choice(int ctas, int n, int slots, Fit fit) {
