@@ -110,7 +110,10 @@ NEGF_DEV void lu_laswp(const LuCtx& c, cplx* col0, int64_t ld, int ncols, int ka
 // rank-1 update writes one place to the left, so that no register index depends on the column.  The
 // multipliers go to shared memory, where the row swaps reach them.  Two barriers per column, for
 // the pivot candidates of the warps and for the two rows that trade places (with the panel in shared
-// memory and every operand read from it, a column took 3000-3400 cycles; now 2300-2700).
+// memory and every operand read from it, a column took 3000-3400 cycles; now 2300-2700).  WID is the
+// number of entries that a step updates: at least the columns left, in classes of 8, NB / 2 and NB, as
+// the latency of a step grows with it (decimation at n = 8 x 148 energies: 390 us with 32 entries for
+// every panel, 311 with 8; 375 with the panel in shared memory).
 template <int NB, int RT, int WID>
 NEGF_DEV void lu_panel_steps(const LuCtx& c, cplx (&x)[RT][NB], cplx* P, cplx* rows, int r0, int m, int j0, int j1) {
   constexpr int PP = LuLayout<NB>::PP;
@@ -206,8 +209,14 @@ NEGF_DEV void lu_panel(const LuCtx& c, int r0, int w) {
     for (int k = 0; k < NB; ++k) x[a][k] = r < m ? P[r * PP + k] : cmk(0.0, 0.0);
   }
   __syncthreads();
-  lu_panel_steps<NB, RT, NB>(c, x, P, rows, r0, m, 0, min(w, NB / 2));
-  lu_panel_steps<NB, RT, NB / 2>(c, x, P, rows, r0, m, NB / 2, w);
+  if (w <= 8) {
+    lu_panel_steps<NB, RT, 8>(c, x, P, rows, r0, m, 0, w);
+  } else if (w <= NB / 2) {
+    lu_panel_steps<NB, RT, NB / 2>(c, x, P, rows, r0, m, 0, w);
+  } else {
+    lu_panel_steps<NB, RT, NB>(c, x, P, rows, r0, m, 0, NB / 2);
+    lu_panel_steps<NB, RT, NB / 2>(c, x, P, rows, r0, m, NB / 2, w);
+  }
   __syncthreads();
   for (int e = team_rank() == 0 ? tid : m * NB; e < m * NB; e += CTA_THREADS) {
     const int r = e / NB, k = e % NB;
