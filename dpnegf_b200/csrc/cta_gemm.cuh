@@ -360,7 +360,7 @@ NEGF_DEV void gemm_body(const GemmArgs& g, const Epi& epi) {
           frag8_load<CA, CB, G3>(f, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
           cp_async_wait<GT_STAGES - 2>();
           __syncthreads();
-          if (k0 + GT_K - 8 < g.K) frag8_mma<G3>(acc, f);
+          frag8_mma<G3>(acc, f);
           st = st + 1 == GT_STAGES ? 0 : st + 1;
         }
         acc_foreach<G3>(acc, wm, wn, lane, [&](int r, int c, cplx v) {
@@ -423,7 +423,7 @@ NEGF_DEV void gemm_body(const GemmArgs& g, const Epi& epi) {
       frag8_load<CA, CB, G3, MI>(f, a, b, GT_K / 8 - 1, wm, wn, lane, AI(), BI());
       cp_async_wait<GT_STAGES - 2>();
       __syncthreads();
-      if (k0 + GT_K - 8 < g.K) frag8_mma<G3, MI>(acc, f);
+      frag8_mma<G3, MI>(acc, f);
       st = st + 1 == GT_STAGES ? 0 : st + 1;
     }
     if constexpr (EpiTraits<Epi>::two_phase) {
