@@ -111,9 +111,10 @@ NEGF_DEV void lu_laswp(const LuCtx& c, cplx* col0, int64_t ld, int ncols, int ka
 // multipliers go to shared memory, where the row swaps reach them.  Two barriers per column, for
 // the pivot candidates of the warps and for the two rows that trade places (with the panel in shared
 // memory and every operand read from it, a column took 3000-3400 cycles; now 2300-2700).  WID is the
-// number of entries that a step updates: at least the columns left, in classes of 8, NB / 2 and NB, as
-// the latency of a step grows with it (decimation at n = 8 x 148 energies: 390 us with 32 entries for
-// every panel, 311 with 8; 375 with the panel in shared memory).
+// number of entries that a step updates, at least the columns left.  The latency of a step grows with
+// it, so matrices of one narrow panel (SMALL, n <= NB / 2) take 8 or NB / 2: decimation at n = 8 x 148
+// energies 390 -> 311 us, against 375 with the panel in shared memory.  The same choice for the last
+// panel of a larger matrix cost 1 % at n = 256.
 template <int NB, int RT, int WID>
 NEGF_DEV void lu_panel_steps(const LuCtx& c, cplx (&x)[RT][NB], cplx* P, cplx* rows, int r0, int m, int j0, int j1) {
   constexpr int PP = LuLayout<NB>::PP;
@@ -186,7 +187,7 @@ NEGF_DEV void lu_panel_steps(const LuCtx& c, cplx (&x)[RT][NB], cplx* P, cplx* r
     }
   }
 }
-template <int NB>
+template <int NB, bool SMALL = false>
 NEGF_DEV void lu_panel(const LuCtx& c, int r0, int w) {
   constexpr int PP = LuLayout<NB>::PP, RT = NB == 32 ? 1 : 2;  // NB = 32 for n <= 256
   const int tid = threadIdx.x;
@@ -209,12 +210,11 @@ NEGF_DEV void lu_panel(const LuCtx& c, int r0, int w) {
     for (int k = 0; k < NB; ++k) x[a][k] = r < m ? P[r * PP + k] : cmk(0.0, 0.0);
   }
   __syncthreads();
-  if (w <= 8) {
-    lu_panel_steps<NB, RT, 8>(c, x, P, rows, r0, m, 0, w);
-  } else if (w <= NB / 2) {
-    lu_panel_steps<NB, RT, NB / 2>(c, x, P, rows, r0, m, 0, w);
+  if constexpr (SMALL) {
+    if (w <= 8) lu_panel_steps<NB, RT, 8>(c, x, P, rows, r0, m, 0, w);
+    else lu_panel_steps<NB, RT, NB / 2>(c, x, P, rows, r0, m, 0, w);
   } else {
-    lu_panel_steps<NB, RT, NB>(c, x, P, rows, r0, m, 0, NB / 2);
+    lu_panel_steps<NB, RT, NB>(c, x, P, rows, r0, m, 0, min(w, NB / 2));
     lu_panel_steps<NB, RT, NB / 2>(c, x, P, rows, r0, m, NB / 2, w);
   }
   __syncthreads();
@@ -365,13 +365,14 @@ NEGF_DEV LuCtx lu_ctx(cplx* W, int64_t ldw, int n, char* smem_raw, PhaseClock* p
 
 // P A = L U in place (W holds L below the diagonal, U on and above); the permutation is left in
 // shared memory for cta_lu_perm / cta_lu_trsolve.  Returns 0, or 1 if a zero or non-finite pivot
-// was met.  Uniform across the CTA; ends with __syncthreads().
-template <int NB>
+// was met.  Uniform across the CTA; ends with __syncthreads().  SMALL: n <= NB / 2.
+template <int NB, bool SMALL = false>
 __device__ __noinline__ int cta_lu_factor_nb(cplx* W, int64_t ldw, int n, char* smem_raw, PhaseClock* pc) {
   const LuCtx c = lu_ctx<NB>(W, ldw, n, smem_raw, pc);
   if (threadIdx.x == 0) *c.flag = 0;
   __syncthreads();
-  lu_rec<NB, 6>(c, 0, n);
+  if constexpr (SMALL) lu_panel<NB, true>(c, 0, n);
+  else lu_rec<NB, 6>(c, 0, n);
   if (threadIdx.x == 0) {  // compose the swaps into a row permutation
     for (int k = 0; k < n; ++k) c.perm[k] = k;
     for (int k = 0; k < n; ++k) {
@@ -401,6 +402,7 @@ __device__ __noinline__ void cta_lu_trsolve_nb(cplx* W, int64_t ldw, int n, cplx
 // cta_lu_trsolve.  pc: optional phase counters (panel / row swaps / GEMM updates / register
 // triangular solves).
 NEGF_DEV int cta_lu_factor(cplx* W, int64_t ldw, int n, char* smem_raw, PhaseClock* pc = nullptr) {
+  if (n <= 16) return cta_lu_factor_nb<32, true>(W, ldw, n, smem_raw, pc);
   if (n <= 256) return cta_lu_factor_nb<32>(W, ldw, n, smem_raw, pc);
   return cta_lu_factor_nb<16>(W, ldw, n, smem_raw, pc);
 }
