@@ -33,6 +33,12 @@ class DeviceBlocks:
         return [int(h.shape[-1]) for h in self.hd]
 
 
+# Fewest pieces that one pack launch beats copies for (it uploads the piece table and reads the flags back).  A
+# device of one block has 3: building the geometry takes 57-73 us with copies, 78-85 with the launch; 6 pieces 97
+# and 90-100, a device of two blocks (12) 167 and 105.
+PACK_MIN = 6
+
+
 def _packable(copies, device):
     """Whether the one-launch pack takes these (offset, tensor) pieces: it loads whole 16-byte entries, while
     complex128 memory that torch did not allocate (DLPack, ``__cuda_array_interface__``) may start at any
@@ -157,7 +163,7 @@ class Geometry:
         16-byte aligned addresses; returns the per-piece nonzero flags, or None when the blocks go one
         by one (also under stream capture, where the piece table cannot be uploaded)."""
         hs = self.hs
-        if torch.cuda.is_current_stream_capturing() or not _packable(copies, hs.device):
+        if len(copies) < PACK_MIN or torch.cuda.is_current_stream_capturing() or not _packable(copies, hs.device):
             return None
         tab = np.zeros(len(copies), dtype=_lib.PACK_DTYPE)
         tab["src"] = [t.data_ptr() for _, t in copies]

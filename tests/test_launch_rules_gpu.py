@@ -1,5 +1,4 @@
-"""How calls reach the kernels: packing under stream capture, empty problems, little
-memory."""
+"""How calls reach the kernels: packing, empty problems, little memory, the inverse's widths."""
 import pytest
 import torch
 
@@ -104,3 +103,18 @@ def test_outer_block_width_is_honoured_with_few_items():
     for x in grd[1:]:
         assert not torch.equal(x, grd[0])
         assert float((x - grd[0]).abs().max()) <= 1e-10 * float(grd[0].abs().max())
+
+
+@pytest.mark.parametrize("K,packs", [(1, 0), (2, 1), (5, 1)])
+def test_one_block_is_copied(K, packs, monkeypatch):
+    """A device of one block has three pieces, fewer than a pack launch pays for."""
+    from dpnegf_b200 import _lib, rgf_plan
+    lib, calls = _lib.load(), []
+    run = lib.negf_pack_run
+    monkeypatch.setattr(lib, "negf_pack_run", lambda *a: calls.append(a) or run(*a))
+    eye = torch.eye(7, dtype=torch.complex128, device="cuda")
+    geom = rgf_plan.Geometry([rgf_plan.DeviceBlocks([eye] * K, *([[2 * eye] * (K - 1)] * 2), [3 * eye] * K,
+                                                    *([[4 * eye] * (K - 1)] * 2))])
+    assert len(calls) == packs
+    for off, v in ((geom.blocks[0]["hd"], 1), (geom.blocks[K - 1]["sd"], 3)):
+        assert torch.equal(geom.hs[int(off):int(off) + 49].view(7, 7), v * eye)
