@@ -31,8 +31,7 @@ int negf_lopez_sancho_run_ctas(const NegfLsProblem* p, int32_t ctas, void* strea
   if ((reinterpret_cast<uintptr_t>(p->scratch) & 255) != 0) return NEGF_ERR_ARGUMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const size_t smem = negf::ls_smem_bytes(p->max_n);
-  if (cudaFuncSetAttribute(negf::ls_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return NEGF_ERR_CUDA;
+  if (!negf::allow_smem(negf::ls_kernel, smem)) return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
   const int cl = negf::team_choice(ctas, negf::ls_team_n(p->max_n), grid, [&](int c) { return negf_team::ls_fit(smem, c); });
   if (cl < 0) return NEGF_ERR_ARGUMENT;

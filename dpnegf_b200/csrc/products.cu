@@ -150,9 +150,7 @@ int negf_gamma_sum_run(const NegfGammaSum* p, void* stream) {
   negf::cplx* Tst = reinterpret_cast<negf::cplx*>(p->scratch);
   negf::cplx* Gst = reinterpret_cast<negf::cplx*>(reinterpret_cast<char*>(p->scratch) + negf::gamma_stack_bytes(*p));
   const int smem = negf::GEMM_SMEM_BYTES;
-  if (cudaFuncSetAttribute(negf::gamma_stack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaFuncSetAttribute(negf::gamma_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return NEGF_ERR_CUDA;
+  if (!negf::allow_smem(negf::gamma_stack_kernel, smem) || !negf::allow_smem(negf::gamma_reduce_kernel, smem)) return NEGF_ERR_CUDA;
   const int sms = negf::sm_count_or(148);
   const int grid1 = p->n_items < sms ? p->n_items : sms;
   negf::gamma_stack_kernel<<<grid1, negf::CTA_THREADS, smem, s>>>(*p, Tst, Gst);
@@ -191,9 +189,7 @@ int negf_lead_adjoint_run_ctas(const NegfLeadAdjProblem* p, int32_t ctas, void* 
     return cudaMemsetAsync(p->grad, 0, (size_t)negf::la_grad_elems(*p) * sizeof(double2), s) == cudaSuccess
                ? NEGF_OK : NEGF_ERR_CUDA;
   const size_t smem = negf::lead_smem_bytes(negf::la_max_n(ld));
-  if (cudaFuncSetAttribute(negf::lead_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return NEGF_ERR_CUDA;
+  if (!negf::allow_smem(negf::lead_adjoint_kernel, smem)) return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
   const int cl = negf::team_choice(ctas, ld.n, grid, [&](int c) { return negf_team::lead_adjoint_fit(smem, c); });
   if (cl < 0) return NEGF_ERR_ARGUMENT;

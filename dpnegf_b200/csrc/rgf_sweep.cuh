@@ -35,6 +35,7 @@
 #include "../../include/negf_b200.h"
 #include "cta_inverse.cuh"
 #include "cta_stream.cuh"
+#include "smem_limit.cuh"
 
 namespace NEGF_NS {
 
@@ -240,7 +241,7 @@ __device__ __noinline__ int cta_inverse_blk(cplx* W, int64_t ldw, int n, cplx* G
     const int h = ((n + 1) / 2 + 7) & ~7, m = n - h;
     cplx *W11 = W, *W12 = W + h, *W21 = W + (int64_t)h * ldw, *W22 = W21 + h;
     cplx *G11 = G, *G12 = G + h, *G21 = G + (int64_t)h * ldg, *G22 = G21 + h;
-    const cplx ONE = cmk(1.0, 0.0), MONE = cmk(-1.0, 0.0);
+    const cplx MONE = cmk(-1.0, 0.0);
     int bad = cta_inverse_blk<LV - 1, MX>(W11, ldw, h, G11, ldg, smem, pc, snap);             // X
     gemm<OP_N, OP_N, MX>(smem, m, h, h, W21, ldw, G11, ldg, G21, ldg);                         // U = A21 X
     gemm_schur<MX>(smem, m, m, h, G21, ldg, W12, ldw, W22, ldw, MONE, W22, ldw);         // S
@@ -256,7 +257,6 @@ __device__ __noinline__ int cta_inverse_blk(cplx* W, int64_t ldw, int n, cplx* G
     }
     team_sync();
     pc.mark(PH_INV_UPDATE);
-    (void)ONE;
     return bad;
   }
 }
@@ -1075,14 +1075,13 @@ int rgf_launch_team(int feat, const NegfRgfProblem& p, size_t smem, int slots, i
 // Teams of `cl` CTAs that fit the GPU at once; 0 when it cannot run them.
 int rgf_team_fit(int feat, size_t smem, int cl);
 #else
-// Set the shared-memory limit of one instantiation and launch it (grid CTAs).  The FP64 sweep
+// Allow one instantiation its shared memory and launch it (grid CTAs).  The FP64 sweep
 // is compiled per feature set (rgf.cu); the mixed-precision sweep is one instantiation with
 // every feature (rgf_mx.cu).
 template <bool MX, int FEAT>
 inline int rgf_launch_impl(const NegfRgfProblem& p, size_t smem, int grid, cudaStream_t s) {
   auto kern = rgf_kernel<MX, FEAT>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return NEGF_ERR_CUDA;
+  if (!negf::allow_smem(kern, smem)) return NEGF_ERR_CUDA;
   kern<<<grid, CTA_THREADS, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? NEGF_OK : NEGF_ERR_CUDA;
 }

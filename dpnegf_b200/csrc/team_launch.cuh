@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "../../include/negf_b200.h"
+#include "smem_limit.cuh"
 #include "team_rule.cuh"
 
 namespace negf {
@@ -45,8 +46,7 @@ inline int team_fit(void (*kernel)(const Problem), size_t smem, int cl) {
   cudaLaunchAttribute a;
   team_config(c, a, smem, 1, cl, nullptr);
   int n = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, kernel, &c) != cudaSuccess) {
+  if (!allow_smem(kernel, smem) || cudaOccupancyMaxActiveClusters(&n, kernel, &c) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -58,8 +58,7 @@ inline int team_launch(void (*kernel)(const Problem), const Problem& p, size_t s
   cudaLaunchConfig_t c;
   cudaLaunchAttribute a;
   team_config(c, a, smem, slots, cl, s);
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return NEGF_ERR_CUDA;
+  if (!allow_smem(kernel, smem)) return NEGF_ERR_CUDA;
   return cudaLaunchKernelEx(&c, kernel, p) == cudaSuccess ? NEGF_OK : NEGF_ERR_CUDA;
 }
 

@@ -1,4 +1,5 @@
-"""How calls reach the kernels: packing, empty problems, little memory, the inverse's widths."""
+"""How calls reach the kernels: packing, empty problems, little memory, the inverse's
+widths, threads."""
 import pytest
 import torch
 
@@ -118,3 +119,36 @@ def test_one_block_is_copied(K, packs, monkeypatch):
     assert len(calls) == packs
     for off, v in ((geom.blocks[0]["hd"], 1), (geom.blocks[K - 1]["sd"], 3)):
         assert torch.equal(geom.hs[int(off):int(off) + 49].view(7, 7), v * eye)
+
+
+@pytest.mark.parametrize("ctas", [0, 1])
+def test_threads_launch_problems_of_different_sizes(ctas):
+    """Two threads on two streams launch sweeps that need different amounts of shared memory: neither may take
+    the other's limit away between setting it and launching."""
+    import threading
+    from dpnegf_b200 import rgf_plan
+    plans = [rgf_plan.run(*_device(1, n, 1, 44 + n), eta=1e-3, outputs=(), trans=True, defer=True, ctas=ctas)
+             for n in (40, 256)]
+    for p in plans:
+        p.launch()
+    torch.cuda.synchronize()
+    want, errors = [p.result.trans.clone() for p in plans], []
+
+    def work(p):
+        s = torch.cuda.Stream()
+        try:
+            for k in range(3000):
+                p.launch(s)
+                if k % 64 == 0:
+                    s.synchronize()
+            s.synchronize()
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(p,)) for p in plans]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors, errors
+    for p, w in zip(plans, want):
+        p.check()
+        assert torch.equal(p.result.trans, w)
