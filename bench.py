@@ -79,9 +79,11 @@ def parse():
     return ap.parse_args()
 
 
-def flops_per_point(b, L):
-    """Algorithmic work of one retarded RGF energy point: 9 complex n^3 MACs per block (4M)."""
-    return 72.0 * b ** 3 * L
+def flops_per_point(b, L, macs=8):
+    """Work of one energy point's sweep: ``macs`` complex n^3 multiply-adds per block (counted 4M, 8 flop each).
+    T + DOS of a non-orthogonal basis takes 8 with L g kept from the forward sweep (two products, the inverse,
+    then g U, and G_{q+1,q}, G_{q,q+1}, G_qq, G_qN); the mixed kernel keeps none and forms 9."""
+    return 8.0 * macs * b ** 3 * L
 
 
 class Clocks:
@@ -418,7 +420,7 @@ def _uneven_inputs(torch, n_devices, seed, first=0):
         devs.append(rgf_plan.DeviceBlocks(dev.hd, dev.hu, dev.hl, dev.sd, dev.su, dev.sl))
         lb = lambda ld: LeadBlocks(ld.hL, ld.hLL, ld.sL, ld.sLL, ld.hDL, ld.sDL)
         leads.append((lb(dev.lead_L), lb(dev.lead_R)))
-        work += 72.0 * b ** 3 * L
+        work += flops_per_point(b, L)  # g U, G_{q+1,q}, G_qq, G_qN and the spectral diagonal's product
     kBT, mu_L, vL, vR = 0.025, 0.0, 0.15, -0.15
     oz = Ozaki(R=1e6, M_cut=64, n_gauss=256)
     fL = lambda x: 1.0 / (1.0 + torch.exp((x - (mu_L - vL)) / kBT))
@@ -526,7 +528,7 @@ def uneven_leg(torch, n_devices=128, seed=2024, precisions=("fp64", "mixed", "mi
     return dict(res, **{
             "note": "per chunk: one call each (lead decimation + persistent sweep + density reduction), CUDA "
                     "events, summed over chunks; item = (device, energy); lead_decimation = that phase timed "
-                    "alone; sweep_tflops counts 72 b^3 L per item over the FP64 time less the decimation's"})
+                    "alone; sweep_tflops counts 64 b^3 L per item over the FP64 time less the decimation's"})
 
 
 def scf_leg(torch, peak, nk=8, n_energies=37, iters=10, eta_lead=ETA_LEAD_SYNTH):
@@ -569,7 +571,8 @@ def scf_leg(torch, peak, nk=8, n_energies=37, iters=10, eta_lead=ETA_LEAD_SYNTH)
         loop.restore()
         del loop
     pts = nk * nE * iters  # one sweep over every (k, energy) item per replayed iteration
-    ach = 72.0 * b ** 3 * L * pts / (ms["fp64"] * 1e-3) / 1e12
+    # L g is not kept at this size (61 GB of scratch for 148 slots), so the sweep takes nine
+    ach = flops_per_point(b, L, 9) * pts / (ms["fp64"] * 1e-3) / 1e12
     rel = lambda x, y: float((x - y).abs().max() / max(float(y.abs().max()), 1e-300))
     return {"b": b, "L": L, "k_points": nk, "energies_per_k": nE, "iterations": iters,
             "lead_decimation": {"items": 2 * nk * nE, "seconds": t_lead * 1e-3, "n": b, "eta": eta_lead,
@@ -789,7 +792,7 @@ def main():
     tpp = traffic_per_point(b, L)
     roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
             "traffic": tpp * B if tpp else None, "kernel": "negf::rgf_kernel",
-            "algorithmic": f"72*b^3*L flop/energy point (9 complex n^3 MACs per block, 4M count; "
+            "algorithmic": f"64*b^3*L flop/energy point (8 complex n^3 MACs per block, 4M count; "
                            f"3M products not credited) x {B} points per launch",
             "peak_source": "FP64 cuBLAS DGEMM 8192^3 measured in this run (of measured; "
                            "MEASURED_PEAKS.json has no FP64 figure)"}
@@ -831,7 +834,7 @@ def main():
         rr, msr = leg(lambda s: mstep(s, refine=True, refine_steps=args.refine_steps))
         tf32 = measured_tf32_peak(torch)
         v_m, v_r = B / (msm * 1e-3), B / (msr * 1e-3)
-        ach_m = flops_per_point(b, L) * v_m / 1e12
+        ach_m = flops_per_point(b, L, 9) * v_m / 1e12
         mixed = {
             "value": v_m, "unit": UNIT, "speedup_vs_fp64": v_m / value,
             "t_abs_err_max": float((rm.trans.cpu() - T64).abs().max()),
@@ -843,7 +846,7 @@ def main():
                          "frac": ach_m / tf32,
                          "tensor_frac_executed": 3.0 * ach_m / tf32,
                          "peak_source": "cuBLAS TF32 GEMM 8192^3 measured in this run (of measured)",
-                         "note": "algorithmic 72*b^3*L flop per point as for FP64; the 3xTF32 split "
+                         "note": "72*b^3*L flop per point (nine products per block); the 3xTF32 split "
                                  "executes 3x that on the tensor cores"},
             "precision": "complex products as 3xTF32 split on tcgen05.mma kind::tf32 (FP32 accumulation "
                          "in TMEM); pivoting, panels and storage FP64; refined = FP64-residual steps on "
