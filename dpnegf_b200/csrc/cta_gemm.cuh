@@ -6,7 +6,12 @@
 // tile streams 16-wide k-slabs of op(A) and op(B) into padded shared-memory
 // tiles with cp.async (3-stage ring).  Each warp owns a 32x16 sub-tile and
 // forms every complex product with three real DMMA m16n8k8 (Gauss/3M):
-//   T1 = Ar*Br, T2 = Ai*Bi, T3 = (Ar+Ai)*(Br+Bi);  Re = T1-T2, Im = T3-T1-T2.
+//   T1 = Ar*Br, T2 = Ai*Bi, T3 = (Ar+Ai)*(Br+Bi);  Re = T1-T2, Im = T3-T1-T2,
+// or with four (4M) where an iteration amplifies the looser bound of 3M.  Other
+// forms of the same code: CTAs of two warps with 32x32 tiles (NEGF_SMALL),
+// clusters that deal the tiles round their CTAs (NEGF_TEAM), 32-row tiles of
+// 16x16 sub-tiles (MI = 1) for few rows or even shares, and a drifting ring for
+// ragged products (gemm_body).
 // Shared-memory pitches are chosen so the DMMA fragment reads (one 16-byte
 // complex per lane) are bank-conflict free for every operand orientation.
 #pragma once

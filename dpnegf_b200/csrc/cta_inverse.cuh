@@ -1,5 +1,7 @@
 // CTA-wide complex128 matrix inverse: two-level blocked Gauss-Jordan with
-// partial pivoting on FP64 tensor cores.
+// partial pivoting on FP64 tensor cores, and for FP64 blocks of up to 64 the same
+// transform held in registers (cta_inverse_reg, described there).  The rest of this
+// comment is about the first.
 //
 // The matrix W (n x n, row stride ldw) is a work buffer in global memory and
 // is destroyed; the inverse is written to G.  Pivoting is implicit: rows never

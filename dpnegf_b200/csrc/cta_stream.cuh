@@ -4,8 +4,8 @@
 // form passes of the first kernel version were load-latency bound at
 // ~25 GB/s per SM).  Here every thread stages its elements of 2048-element
 // chunks with cp.async, two chunks in flight (128 KB per SM), and consumes
-// exactly the elements it staged, so no barrier is needed inside the loop (the
-// reads are ordered behind the wait by lds_after_wait).
+// exactly the elements it staged, so no barrier is needed inside the loop (a
+// thread's own copies are complete behind its wait).
 #pragma once
 #include "negf_common.cuh"
 

@@ -97,7 +97,9 @@ NEGF_DEV cplx* smem_cplx() { return reinterpret_cast<cplx*>(negf_smem); }
 // ---------------------------------------------------------------------------
 // cp.async (16-byte, L2-only) with zero fill when the source is out of range.  The copy writes
 // shared memory behind the compiler's back: the memory clobbers here and on the wait keep reads of
-// the staged entries between them, also where a thread consumes its own copies without a barrier.
+// the staged entries between them, also where a thread consumes its own copies without a barrier
+// (which wait_group orders; without the clobbers some instantiations of the sweep had their reads
+// moved ahead of the wait and returned wrong, varying blocks).
 NEGF_DEV void cp_async16(void* smem_dst, const void* gmem_src, bool valid) {
   unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
   int n = valid ? 16 : 0;
@@ -110,9 +112,8 @@ NEGF_DEV cplx ldg_early(const cplx* p) {
   asm volatile("ld.global.cg.v2.f64 {%0,%1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
   return v;
 }
-// Shared-memory read that stays behind the wait for a copy of the same thread.  A plain load is not
-// ordered against cp.async.wait_group without a barrier in between: some instantiations of the sweep
-// read the streamed entries before they had arrived.
+// Shared-memory read of an entry that this thread staged itself, kept in program order with the wait
+// and the next copies as they are (volatile).
 NEGF_DEV cplx lds_after_wait(const cplx* p) {
   cplx v;
   asm volatile("ld.shared.v2.f64 {%0,%1}, [%2];\n"

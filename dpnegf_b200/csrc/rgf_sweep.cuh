@@ -202,9 +202,9 @@ NEGF_DEV void gemm_epi(const GemmArgs& g, cplx* smem, const Epi& e) {
 }
 
 // The Schur complement of the block inverse: conventional 4M in FP64.  It is inverted next, which
-// amplifies the looser componentwise error of Gauss/3M; at b = 96 the noise of a finite difference of
-// T and DOS fell from 0.59 to 0.41 of its test's tolerance (0.39 with all six products in 4M, which
-// costs 4 % of the sweep instead of 1 %).
+// amplifies the looser componentwise error of Gauss/3M: at b = 96 the noise in a finite difference of
+// T and DOS is 0.41 of 1e-5 of the largest gradient, 0.59 with this product in 3M, 0.39 with all six
+// in 4M.  Costs 0.6 % of the b = 256 sweep (all six 4 %).
 template <bool MX>
 NEGF_DEV void gemm_schur(cplx* smem, int M, int N, int K, const cplx* A, int64_t lda, const cplx* B, int64_t ldb, cplx* C,
                     int64_t ldc, cplx alpha = cmk(1.0, 0.0), const cplx* D = nullptr, int64_t ldd = 0) {

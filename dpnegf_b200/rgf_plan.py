@@ -203,8 +203,7 @@ def check_status(status: torch.Tensor):
 @dataclass
 class RgfPlan:
     """A prepared sweep (``run(..., defer=True)``): descriptors, scratch and outputs stay allocated.  Of the
-    scratch, what only makes the sweep faster is at most a 1/PLAN_EXTRA of the GPU's memory twice (extra
-    slots, kept L g)."""
+    scratch, what only makes the sweep faster (extra slots, kept L g) is bounded by ``_plan_takes``."""
     prob: object
     keep: list
     n_items: int
@@ -236,8 +235,17 @@ class RgfResult:
     grads: Optional[dict] = None            # adjoint: block gradients and per-energy dT/dSigma
 
 
-# Bound on each optional part of a deferred plan's scratch: memory / 256, 0.7 GB of a B200.
-PLAN_EXTRA = 256
+def _plan_takes(extra, dev, memory):
+    """Whether a deferred plan takes ``extra`` bytes of scratch for speed alone.  It holds them for its life,
+    beside other plans and tensors: at most a 64th of the GPU's memory (2.9 GB), and more than 180 MB only of
+    its first half (asking for the free memory takes 0.2 ms)."""
+    if extra <= memory // 1024:
+        return True
+    if extra > memory // 64:
+        return False
+    free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+    return free - extra >= memory // 2
+
 
 _FAMILY = {  # output tag -> (flag, block field, shape fn (n_q, n_next, n_last))
     "grd": (_lib.OUT_GRD, "o_grd", lambda n, nn, nl: (n, n), False),
@@ -507,7 +515,7 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
     orbar_t = torch.zeros(max(orb_cursor, 1), dtype=torch.float64, device=dev) if orb_ar else None
     status_t = torch.empty(max(item_cursor, 1), dtype=torch.int32, device=dev)
     # Memory for speed alone, extra slots for small blocks and a kept L g: a call gives it back when it
-    # returns; a deferred plan holds it beside other plans and tensors, so it takes little.
+    # returns; a deferred plan does not, so it takes little.
     memory = torch.cuda.get_device_properties(dev).total_memory
     sms = lib.negf_sm_count()
     if n_slots is None:
@@ -515,9 +523,8 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
         # small blocks: several slots per SM, while their scratch stays a sixteenth of the GPU's memory
         per_sm = lib.negf_rgf_slots_per_sm(geom.max_n) if precision == "fp64" and not adjoint else 1
         slot_bytes = 16 * (20 * geom.max_n ** 2 + 4 * geom.max_g_slab)
-        fits = (per_sm - 1) * sms * slot_bytes <= memory // PLAN_EXTRA if defer else \
-            per_sm * sms * slot_bytes <= memory // 16
-        if per_sm > 1 and fits:
+        if per_sm > 1 and (_plan_takes((per_sm - 1) * sms * slot_bytes, dev, memory) if defer
+                           else per_sm * sms * slot_bytes <= memory // 16):
             n_slots = max(1, min(n_items, per_sm * sms))
     prob = _lib.NegfRgfProblem()
     prob.blocks = blocks_t.data_ptr()
@@ -563,7 +570,7 @@ def run(geom: Geometry, energies: List[torch.Tensor], se_l: List[Optional[torch.
         need = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
         prob.flags = flags | _lib.KEEP_LG
         kept = lib.negf_rgf_scratch_bytes(ctypes.byref(prob))
-        if kept - need > memory // PLAN_EXTRA if defer else kept > memory // 4:
+        if not (_plan_takes(kept - need, dev, memory) if defer else kept <= memory // 4):
             prob.flags = flags
     # the gradient accumulators first: only what is left is there for the kept L g and the extra slots
     grad_t = None

@@ -75,23 +75,36 @@ def test_gradient_fits_where_only_the_kept_products_do_not():
         assert float((x - y).abs().max()) <= 1e-10 * float(y.abs().max())
 
 
-@pytest.mark.parametrize("K,n,keeps", [(4, 64, True), (96, 64, False)])
+@pytest.mark.parametrize("K,n,keeps", [(4, 64, True), (320, 64, False)])
 def test_deferred_plan_keeps_little(K, n, keeps):
     """A deferred plan holds its scratch for its life: L g is kept where it is small, and only there."""
     from dpnegf_b200 import _lib, rgf_plan
     sms = _lib.load().negf_sm_count()
     plan = rgf_plan.run(*_device(K, n, sms, 41), eta=1e-3, outputs=(), trans=True, dos=True, defer=True)
     kept = sms * K * n * n * 16
-    assert (kept <= torch.cuda.get_device_properties(0).total_memory // rgf_plan.PLAN_EXTRA) == keeps
+    assert (kept <= torch.cuda.get_device_properties(0).total_memory // 64) == keeps
     assert bool(plan.prob.flags & _lib.KEEP_LG) == keeps
 
 
-@pytest.mark.parametrize("K,n,many", [(4, 8, True), (64, 32, False)])
+@pytest.mark.parametrize("K,n,many", [(4, 8, True), (256, 32, False)])
 def test_deferred_plan_takes_extra_slots_where_they_are_small(K, n, many):
     from dpnegf_b200 import _lib, rgf_plan
     sms = _lib.load().negf_sm_count()
     plan = rgf_plan.run(*_device(K, n, 3 * sms, 42), eta=1e-3, outputs=(), trans=True, dos=True, defer=True)
     assert plan.prob.n_slots == (3 * sms if many else sms)
+
+
+def test_deferred_plan_takes_nothing_large_of_a_half_full_gpu():
+    from dpnegf_b200 import _lib, rgf_plan
+    sms = _lib.load().negf_sm_count()
+    args = _device(96, 32, 3 * sms, 43)
+    build = lambda: rgf_plan.run(*args, eta=1e-3, outputs=(), trans=True, dos=True, defer=True)
+    full = torch.empty(int(0.52 * torch.cuda.get_device_properties(0).total_memory), dtype=torch.uint8, device="cuda")
+    plan = build()
+    del full
+    assert plan.prob.n_slots == sms and not plan.prob.flags & _lib.KEEP_LG
+    plan = build()
+    assert plan.prob.n_slots == 3 * sms and plan.prob.flags & _lib.KEEP_LG
 
 
 def test_outer_block_width_is_honoured_with_few_items():
