@@ -20,6 +20,54 @@ namespace NEGF_NS {
 // Energies go to the CTAs round-robin; each CTA sums its energies' contributions in its own slot,
 // and a second kernel sums the slots in slot order.
 
+// The product of one tile and one k = 8 step (the leads of up to 8, a few dozen products per energy): no
+// ring, and no MMAs for the empty half of the 16-deep slab, which is half of them.  The drifting form's
+// larger start-up had made the lead adjoint of such leads 3-8 % slower than the form before it.  Lead
+// adjoint, 148 energies: n = 1 201 -> 143 us, n = 8 245 -> 176 (191 and 232 before the drifting form).
+// Skipping the empty half inside the tile GEMM's loop instead cost the large products 1-3 %, and the same
+// choice in the decimation 5 % of its steps at n = 33..64.
+template <int OPA, int OPB, bool G3>
+__device__ __noinline__ void cta_gemm_thin(const GemmArgs& gr) {
+  const GemmArgs g = gr;
+  cplx *sA = smem_cplx(), *sB = sA + GT_TILE;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = (warp >> 2) * 32, wn = ((warp + 2 * (warp >> 2)) & 3) * 16;  // as the drifting form
+  typedef typename std::conditional<OPA == OP_C, AIdxOpC, AIdxOp0>::type AI;
+  typedef typename std::conditional<OPB == OP_C, BIdxOpC, BIdxOp0>::type BI;
+  if (team_rank() == 0) {
+    __syncthreads();  // whatever used this memory before is done with it
+    load_a_tile<OPA>(sA, g, 0, 0, tid);
+    load_b_tile<OPB>(sB, g, 0, 0, tid);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    if (wm < g.M && wn < g.N) {
+      Acc3M acc;
+      acc.zero();
+      warp_mma_3m<(OPA != OP_N), (OPB != OP_N), G3>(acc, sA, sB, 1, wm, wn, lane, AI(), BI());
+      const EpiStore epi{g};
+      acc_foreach<G3>(acc, wm, wn, lane, [&](int m, int n, cplx v) {
+        if (m < g.M && n < g.N) epi(m, n, v);
+      });
+    }
+  }
+  team_sync();
+}
+
+// gemm_ls with Gauss/3M products, thin where it can be.
+template <int OPA, int OPB>
+NEGF_DEV void gemm_la(cplx* smem, int M, int N, int K, const cplx* A, int64_t lda, const cplx* B, int64_t ldb, cplx* C,
+                      int64_t ldc, const cplx* D = nullptr, int64_t ldd = 0, cplx alpha = cmk(1.0, 0.0)) {
+  if (K > 8 || M > GT_M || N > GT_N) {
+    gemm_ls<OPA, OPB, true>(smem, M, N, K, A, lda, B, ldb, C, ldc, D, ldd, alpha);
+    return;
+  }
+  GemmArgs g = gemm_args(M, N, K, A, lda, B, ldb, C, ldc);
+  g.alpha = alpha;
+  if (D) { g.D = D; g.ldd = ldd; g.beta = cmk(1.0, 0.0); g.use_d = true; }
+  cta_gemm_thin<OPA, OPB, true>(g);
+}
+
 constexpr int LA_NACC = 6, LA_NWORK = 12;
 
 __host__ __device__ inline int la_max_n(const NegfLead& ld) { return ld.nc > ld.n ? ld.nc : ld.n; }
@@ -66,11 +114,11 @@ NEGF_DEV void la_item(const NegfLeadAdjProblem& P, int idx, cplx* slot, char* sm
     for (int e = team_tid(); e < nc * b; e += team_threads()) Lm[e] = csub(cmul(E, sdl[e]), hdl[e]);
     team_sync();
     form_eS_minus_h_herm(Rm, hdl, sdl, E, b, nc);                       // b x nc
-    gemm_ls<OP_C, OP_N, true>(smem, b, nc, nc, Lm, b, Gs, nc, T1, nc);        // L^H Gs       (b x nc)
-    gemm_ls<OP_N, OP_C, true>(smem, b, b, nc, T1, nc, Rm, nc, lam, n);        // V[:b,:b]
-    gemm_ls<OP_N, OP_C, true>(smem, nc, b, nc, Gs, nc, Rm, nc, T2, b);        // Gs R^H       (nc x b)
-    gemm_ls<OP_N, OP_C, true>(smem, nc, b, b, T2, b, g, n, gL, b);            // dL/dL        (nc x b)
-    gemm_ls<OP_C, OP_N, true>(smem, b, nc, b, g, n, T1, nc, gR, nc);          // dL/dR        (b x nc)
+    gemm_la<OP_C, OP_N>(smem, b, nc, nc, Lm, b, Gs, nc, T1, nc);        // L^H Gs       (b x nc)
+    gemm_la<OP_N, OP_C>(smem, b, b, nc, T1, nc, Rm, nc, lam, n);        // V[:b,:b]
+    gemm_la<OP_N, OP_C>(smem, nc, b, nc, Gs, nc, Rm, nc, T2, b);        // Gs R^H       (nc x b)
+    gemm_la<OP_N, OP_C>(smem, nc, b, b, T2, b, g, n, gL, b);            // dL/dL        (nc x b)
+    gemm_la<OP_C, OP_N>(smem, b, nc, b, g, n, T1, nc, gR, nc);          // dL/dR        (b x nc)
     const cplx Ec = cconj(E);
     for (int e = team_tid(); e < nc * b; e += team_threads()) {
       const int i = e / b, j = e % b;
@@ -83,8 +131,8 @@ NEGF_DEV void la_item(const NegfLeadAdjProblem& P, int idx, cplx* slot, char* sm
     for (int64_t e = team_tid(); e < n2; e += team_threads()) F[e] = g[e];
     team_sync();
     bad |= cta_lu_inverse(F, W, n, smem_raw);                           // W = g^-1
-    gemm_ls<OP_C, OP_N, true>(smem, n, n, n, W, n, Gs, n, T1, n);             // g^-H Gs
-    gemm_ls<OP_N, OP_C, true>(smem, n, n, n, T1, n, W, n, lam, n, nullptr, 0, P.form == 1 ? MONE : ONE);
+    gemm_la<OP_C, OP_N>(smem, n, n, n, W, n, Gs, n, T1, n);             // g^-H Gs
+    gemm_la<OP_N, OP_C>(smem, n, n, n, T1, n, W, n, lam, n, nullptr, 0, P.form == 1 ? MONE : ONE);
     if (P.form == 2) {
       const cplx Ec = cconj(E);
       for (int64_t e = team_tid(); e < n2; e += team_threads()) {
@@ -98,16 +146,16 @@ NEGF_DEV void la_item(const NegfLeadAdjProblem& P, int idx, cplx* slot, char* sm
   // ---- Lambda by doubling
   cta_shift_form<true>(tau, H01, S01, z, MONE, (int)n2, smem);                // z S01 - H01
   form_eS_minus_h_herm(taup, H01, S01, z, n, n);                        // z S01^H - H01^H
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, g, n, tau, n, Pm, n);              // P = g tau
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, taup, n, g, n, Qm, n);             // Q = tau' g
+  gemm_la<OP_N, OP_N>(smem, n, n, n, g, n, tau, n, Pm, n);              // P = g tau
+  gemm_la<OP_N, OP_N>(smem, n, n, n, taup, n, g, n, Qm, n);             // Q = tau' g
   int steps = 0;
   bool finite = true;
   for (int s = 0; s < P.max_iter; ++s) {
     steps = s + 1;
-    gemm_ls<OP_C, OP_N, true>(smem, n, n, n, Pm, n, lam, n, T1, n);           // P^H Lambda
-    gemm_ls<OP_N, OP_C, true>(smem, n, n, n, T1, n, Qm, n, lam, n, lam, n);   // Lambda += ... Q^H
-    gemm_ls<OP_N, OP_N, true>(smem, n, n, n, Pm, n, Pm, n, P2, n);
-    gemm_ls<OP_N, OP_N, true>(smem, n, n, n, Qm, n, Qm, n, Q2, n);
+    gemm_la<OP_C, OP_N>(smem, n, n, n, Pm, n, lam, n, T1, n);           // P^H Lambda
+    gemm_la<OP_N, OP_C>(smem, n, n, n, T1, n, Qm, n, lam, n, lam, n);   // Lambda += ... Q^H
+    gemm_la<OP_N, OP_N>(smem, n, n, n, Pm, n, Pm, n, P2, n);
+    gemm_la<OP_N, OP_N>(smem, n, n, n, Qm, n, Qm, n, Q2, n);
     cplx* t = Pm; Pm = P2; P2 = t;
     t = Qm; Qm = Q2; Q2 = t;
     double mp = 0.0, mq = 0.0;
@@ -123,16 +171,16 @@ NEGF_DEV void la_item(const NegfLeadAdjProblem& P, int idx, cplx* slot, char* sm
   }
 
   // ---- F = (zS - H - tau g tau')^-1 and the parameter gradients
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, g, n, taup, n, Y1, n);             // g tau'
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, tau, n, Y1, n, W, n);              // tau g tau'
+  gemm_la<OP_N, OP_N>(smem, n, n, n, g, n, taup, n, Y1, n);             // g tau'
+  gemm_la<OP_N, OP_N>(smem, n, n, n, tau, n, Y1, n, W, n);              // tau g tau'
   for (int64_t e = team_tid(); e < n2; e += team_threads()) W[e] = csub(csub(cmul(z, S[e]), H[e]), W[e]);
   team_sync();
   bad |= cta_lu_inverse(W, F, n, smem_raw);
-  gemm_ls<OP_C, OP_N, true>(smem, n, n, n, F, n, lam, n, T1, n);              // F^H Lambda
-  gemm_ls<OP_N, OP_C, true>(smem, n, n, n, T1, n, F, n, gW, n, nullptr, 0, MONE);  // dW
-  gemm_ls<OP_N, OP_C, true>(smem, n, n, n, gW, n, Y1, n, T1, n, nullptr, 0, MONE);  // dtau = -dW (g tau')^H
-  gemm_ls<OP_N, OP_N, true>(smem, n, n, n, tau, n, g, n, Pm, n);              // tau g
-  gemm_ls<OP_C, OP_N, true>(smem, n, n, n, Pm, n, gW, n, Qm, n, nullptr, 0, MONE);  // dtau' = -(tau g)^H dW
+  gemm_la<OP_C, OP_N>(smem, n, n, n, F, n, lam, n, T1, n);              // F^H Lambda
+  gemm_la<OP_N, OP_C>(smem, n, n, n, T1, n, F, n, gW, n, nullptr, 0, MONE);  // dW
+  gemm_la<OP_N, OP_C>(smem, n, n, n, gW, n, Y1, n, T1, n, nullptr, 0, MONE);  // dtau = -dW (g tau')^H
+  gemm_la<OP_N, OP_N>(smem, n, n, n, tau, n, g, n, Pm, n);              // tau g
+  gemm_la<OP_C, OP_N>(smem, n, n, n, Pm, n, gW, n, Qm, n, nullptr, 0, MONE);  // dtau' = -(tau g)^H dW
   const cplx zc = cconj(z);
   for (int64_t e = team_tid(); e < n2; e += team_threads()) {
     const int64_t i = e / n, j = e % n;

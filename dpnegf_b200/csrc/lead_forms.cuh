@@ -29,39 +29,6 @@ NEGF_DEV void form_eS_minus_h_herm(cplx* out, const cplx* H, const cplx* S, cplx
   team_sync();
 }
 
-// The product of one tile and one k = 8 step (the leads of up to 8, a few dozen products per energy): no
-// ring, and no MMAs for the empty half of the 16-deep slab, which is half of them.  The drifting form's
-// larger start-up had made the lead adjoint of such leads 3-8 % slower than the form before it.  Lead
-// adjoint, 148 energies: n = 1 201 -> 143 us, n = 8 245 -> 176 (191 and 232 before the drifting form).
-// Skipping the empty half inside the tile GEMM's loop instead cost the large products 1-3 %.
-template <int OPA, int OPB, bool G3>
-__device__ __noinline__ void cta_gemm_thin(const GemmArgs& gr) {
-  const GemmArgs g = gr;
-  cplx *sA = smem_cplx(), *sB = sA + GT_TILE;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp >> 2) * 32, wn = ((warp + 2 * (warp >> 2)) & 3) * 16;  // as the drifting form
-  typedef typename std::conditional<OPA == OP_C, AIdxOpC, AIdxOp0>::type AI;
-  typedef typename std::conditional<OPB == OP_C, BIdxOpC, BIdxOp0>::type BI;
-  if (team_rank() == 0) {
-    __syncthreads();  // whatever used this memory before is done with it
-    load_a_tile<OPA>(sA, g, 0, 0, tid);
-    load_b_tile<OPB>(sB, g, 0, 0, tid);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    if (wm < g.M && wn < g.N) {
-      Acc3M acc;
-      acc.zero();
-      warp_mma_3m<(OPA != OP_N), (OPB != OP_N), G3>(acc, sA, sB, 1, wm, wn, lane, AI(), BI());
-      const EpiStore epi{g};
-      acc_foreach<G3>(acc, wm, wn, lane, [&](int m, int n, cplx v) {
-        if (m < g.M && n < g.N) epi(m, n, v);
-      });
-    }
-  }
-  team_sync();
-}
-
 // C = alpha op(A) op(B) (+ beta D when D is given).  By default conventional 4M complex products
 // (see warp_mma_3m): the decimation squares and accumulates products, which amplifies the looser
 // componentwise error of Gauss/3M products; G3 = true selects Gauss/3M where no iteration feeds
@@ -73,8 +40,7 @@ NEGF_DEV void gemm_ls(cplx* smem, int M, int N, int K, const cplx* A, int64_t ld
   GemmArgs g = gemm_args(M, N, K, A, lda, B, ldb, C, ldc);
   g.alpha = alpha;
   if (D) { g.D = D; g.ldd = ldd; g.beta = beta; g.use_d = true; }
-  if (K <= 8 && M <= GT_M && N <= GT_N) cta_gemm_thin<OPA, OPB, G3>(g);
-  else cta_gemm<OPA, OPB, G3>(g);
+  cta_gemm<OPA, OPB, G3>(g);
 }
 
 // out = W^-1 (n x n, row stride n) by the LU solve against I (numpy.linalg.inv's route); W is
