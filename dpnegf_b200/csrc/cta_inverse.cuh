@@ -31,7 +31,6 @@
 // produced.  Two barriers per column.
 #pragma once
 #include "cta_gemm_tc.cuh"
-#include "item_status.cuh"
 
 namespace NEGF_NS {
 
@@ -388,6 +387,8 @@ __device__ __noinline__ int cta_inverse_nb(cplx* W, int64_t ldw, int n, cplx* G,
   return flag;
 }
 
+static __shared__ int inv_lost;  // a panel of an in-register inverse of this item never came
+
 NEGF_DEV void mbar_init(unsigned long long* b, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(b)), "r"(count) : "memory");
 }
@@ -426,8 +427,8 @@ NEGF_DEV void static_groups(F f) {
 //     x[i][j] = (i a pivot of the panel ? 0 : x[i][j]) + sum_s P[i][s] v_s,   v_s = x[p_s][j],
 // where the pivot rows' entries are exchanged inside the warp.  Every panel has its own slot in
 // shared memory, so the warps need not be in step.  The pivot is the row whose |re| + |im| has the
-// largest leading 32 bits (within 2^-20 of the largest), the lowest lane among equals.  Returns the
-// flags of item_status.cuh.
+// largest leading 32 bits (within 2^-20 of the largest), the lowest lane among equals.  Returns 1
+// after a singular pivot or an expired wait, which also sets inv_lost.
 // Bound by the latency of the panel chain (per column a reduction, a reciprocal and a rank-1 step
 // of PW columns).  Against the blocked form with 8-wide panels in shared memory, every SM inverting
 // its own matrices: n = 16 22.7 -> 7.4 us, 32 47 -> 17, 64 108 -> 57; the block inverse built on it
@@ -596,7 +597,7 @@ __device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, c
   };
   if (warp == 0) factor(G0);
   for (int w0 = 0; w0 < NW; ++w0) static_groups<NSUB>([&](auto g_c) { panel(g_c, w0); });
-  if (lost) flag[1] = 1;
+  if (lost) flag[1] = inv_lost = 1;
   __syncthreads();
   // G[i][j] = W[p(i)][p^-1(j)] (every CTA of a team holds the same result; one stores it)
   if (!flag[1] && team_rank() == 0) {
@@ -608,7 +609,7 @@ __device__ __noinline__ int cta_inverse_reg(const cplx* W, int64_t ldw, int n, c
         if (i < n && c < n) G[(int64_t)pinv[i] * ldg + piv[c]] = x[a][j];
       }
   }
-  const int f = (flag[0] ? INV_SINGULAR : 0) | (flag[1] ? INV_LOST : 0);
+  const int f = flag[0] | flag[1];
   if (tid < NPAN) mbar_inval(bar + tid);
   team_sync();
   return f;

@@ -8,15 +8,11 @@
 #define NEGF_HD
 #endif
 
-// Flags of a block inverse; an item collects those of its blocks.
-constexpr int INV_SINGULAR = 1;  // a zero or non-finite pivot
-constexpr int INV_LOST = 2;      // a bounded wait for a panel expired: the inverse was not stored
-
-// `inv`: the collected flags; tc_lost: a bounded tensor-core wait expired; finite: T and DOS are.
-// A lost inverse leaves arbitrary numbers behind it, so it goes before the pivots met in them.
-NEGF_HD inline int item_status(int inv, bool tc_lost, bool finite) {
-  if (inv & INV_LOST) return NEGF_ERR_TIMEOUT;
-  if (inv) return NEGF_ERR_SINGULAR;
+// inv_bad: a block inverse failed; inv_lost: one of them because a bounded wait for a panel expired, so that it
+// was not stored (the numbers behind it are arbitrary, so this goes before the pivots met in them); tc_lost: a
+// bounded tensor-core wait expired; finite: T and DOS are.
+NEGF_HD inline int item_status(bool inv_bad, bool inv_lost, bool tc_lost, bool finite) {
+  if (inv_bad) return inv_lost ? NEGF_ERR_TIMEOUT : NEGF_ERR_SINGULAR;
   if (tc_lost) return NEGF_ERR_TIMEOUT;
   return finite ? NEGF_OK : NEGF_ERR_NONFINITE;
 }

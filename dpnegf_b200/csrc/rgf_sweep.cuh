@@ -34,6 +34,7 @@
 #include <cstdio>
 #include "../../include/negf_b200.h"
 #include "cta_inverse.cuh"
+#include "item_status.cuh"
 #include "cta_stream.cuh"
 #include "smem_limit.cuh"
 
@@ -353,7 +354,7 @@ struct EpiGrad {
 // (null for q = 0), and with dgq its z-tangent dg_q from dgprev.  Uses the slot's W, T1, Lz, Uz
 // and tA..tE; leaves L_{q-1}, U_{q-1} in Lz, Uz for the lesser and greater steps, and
 // L_{q-1} g_{q-1} in lg (T1 when null; the tangent reads it from T1).  Inlined into the sweep; the checkpointed adjoint recomputes its segments
-// through the non-inlined copy below.  Returns the flags of the inverse (item_status.cuh).
+// through the non-inlined copy below.  Returns the failure flag of the inverse.
 template <bool MX>
 NEGF_DEV int forward_block_body(const NegfRgfProblem& P, const NegfItem& it, const SlotBufs& sb,
                                 char* smem_raw, double* red, PhaseClock& pc, int q,
@@ -396,6 +397,8 @@ NEGF_DEV int forward_block_body(const NegfRgfProblem& P, const NegfItem& it, con
     bb = team_max((double)bb, red) != 0.0;  // one decision for the team, whatever a CTA met
 #endif
     if (bb || !inv_probe(sb.tD, gq, nq, MX ? 1e-4 : 1e-10, smem, red, sb.tE)) {
+      if constexpr (!MX)
+        if (threadIdx.x == 0) inv_lost = 0;  // the inverse that replaces it decides
       copy_mat(sb.W, sb.tD, nq, nq, smem);
       gj = true;
     }
@@ -1023,9 +1026,10 @@ NEGF_DEV void rgf_item(const NegfRgfProblem& P, const NegfItem& it, const SlotBu
   if (team_tid() == 0) {
     if (fl & NEGF_TRANS) P.trans[it.out] = tval;
     if (fl & NEGF_DOS) P.dos[it.out] = dos_total;
-    bool tc_lost = false;
+    bool lost = false, tc_lost = false;  // (flags in shared memory: two values of `bad` cost the sweep 0.6 %)
     if constexpr (MX) tc_lost = tc_err != 0;
-    P.status[it.out] = item_status(bad, tc_lost, isfinite(tval) && isfinite(dos_total));
+    else lost = inv_lost != 0;
+    P.status[it.out] = item_status(bad, lost, tc_lost, isfinite(tval) && isfinite(dos_total));
   }
   team_sync();
   pc.mark(PH_TRANS);
@@ -1053,6 +1057,8 @@ __global__ void __launch_bounds__(CTA_THREADS, MIN_CTAS) rgf_kernel(const NegfRg
     pc.mark(PH_OTHER);
     if (idx >= P.n_items) break;
     const NegfItem it = P.items[idx];
+    if constexpr (!MX)
+      if (threadIdx.x == 0) inv_lost = 0;
     rgf_item<MX, FEAT>(P, it, sb, smem, red, pc);
   }
   if constexpr (MX) tc_tmem_free();

@@ -10,9 +10,8 @@ SRC = """
 #include <cstdio>
 #include "item_status.cuh"
 int main() {
-  for (int inv = 0; inv < 4; ++inv)
-    for (int lost = 0; lost < 2; ++lost)
-      for (int fin = 0; fin < 2; ++fin) std::printf("%d %d %d %d\\n", inv, lost, fin, item_status(inv, lost, fin));
+  for (int i = 0; i < 16; ++i)
+    std::printf("%d %d %d %d %d\\n", i & 1, i >> 1 & 1, i >> 2 & 1, i >> 3 & 1, item_status(i & 1, i >> 1 & 1, i >> 2 & 1, i >> 3 & 1));
 }
 """
 
@@ -23,17 +22,19 @@ def test_an_expired_wait_is_not_reported_as_a_singular_block(tmp_path):
     (tmp_path / "s.cpp").write_text(SRC)
     subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "dpnegf_b200", "csrc"), "s.cpp", "-o", "s"],
                    cwd=tmp_path, check=True)
-    got = {}
-    for line in subprocess.run([str(tmp_path / "s")], check=True, capture_output=True, text=True).stdout.splitlines():
-        inv, lost, fin, st = map(int, line.split())
-        got[inv, lost, fin] = st
-    singular, expired = 1, 2
-    for lost in (0, 1):
-        for fin in (0, 1):
-            assert got[expired, lost, fin] == got[expired | singular, lost, fin] == _lib.NEGF_ERR_TIMEOUT
-            assert got[singular, lost, fin] == _lib.NEGF_ERR_SINGULAR
-            assert lost == 0 or got[0, 1, fin] == _lib.NEGF_ERR_TIMEOUT
-    assert got[0, 0, 1] == _lib.NEGF_OK and got[0, 0, 0] == _lib.NEGF_ERR_NONFINITE
+    out = subprocess.run([str(tmp_path / "s")], check=True, capture_output=True, text=True).stdout
+    seen = 0
+    for line in out.splitlines():
+        bad, inv_lost, tc_lost, finite, status = map(int, line.split())
+        if bad:
+            want = _lib.NEGF_ERR_TIMEOUT if inv_lost else _lib.NEGF_ERR_SINGULAR
+        elif tc_lost:
+            want = _lib.NEGF_ERR_TIMEOUT
+        else:
+            want = _lib.NEGF_OK if finite else _lib.NEGF_ERR_NONFINITE
+        assert status == want, line
+        seen += 1
+    assert seen == 16
 
 
 def test_the_exception_of_an_expired_wait():
