@@ -4,20 +4,17 @@
 
 namespace negf {
 
-// Allow `smem` bytes.  The limit belongs to the kernel, not to a launch, so it is only ever set to all that
-// the GPU has beside the kernel's static shared memory: a thread that sets it to what its own problem needs
-// takes it from another thread's larger one, between that one's setting it and launching.
+// What every kernel is allowed: 227 KB of a CTA less 4 KB for its static shared memory; the largest need is
+// 221 KB (the Gauss-Jordan panels at n = 256).
+constexpr size_t SMEM_LIMIT = 223 * 1024;
+
+// Allow `smem` bytes.  The limit belongs to the kernel, not to a launch, so it is only ever set to the same
+// value: a thread that sets it to what its own problem needs takes it from another thread's larger one,
+// between that one's setting it and launching.
 template <class Kernel>
 inline bool allow_smem(Kernel* kernel, size_t smem) {
-  cudaFuncAttributes a;
-  int dev = 0, most = 0;
-  if (cudaFuncGetAttributes(&a, kernel) != cudaSuccess) return false;
-  if ((size_t)a.maxDynamicSharedSizeBytes >= smem) return true;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
-    return false;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes) ==
-         cudaSuccess;
+  return smem <= SMEM_LIMIT &&
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT) == cudaSuccess;
 }
 
 }  // namespace negf
