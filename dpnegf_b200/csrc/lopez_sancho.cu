@@ -33,7 +33,8 @@ int negf_lopez_sancho_run_ctas(const NegfLsProblem* p, int32_t ctas, void* strea
   const size_t smem = negf::ls_smem_bytes(p->max_n);
   if (!negf::allow_smem(negf::ls_kernel, smem)) return NEGF_ERR_CUDA;
   const int grid = p->n_slots < p->n_items ? p->n_slots : p->n_items;
-  const int cl = negf::team_choice(ctas, negf::ls_team_n(p->max_n), grid, [&](int c) { return negf_team::ls_fit(smem, c); });
+  const int cl =
+      negf::team_choice(ctas, negf::ls_team_n(p->max_n), grid, [&](int c) { return negf_team::ls_fit(smem, c); });
   if (cl < 0) return NEGF_ERR_ARGUMENT;
   if (cudaMemsetAsync(p->scratch, 0, negf::LS_SCRATCH_HEADER, s) != cudaSuccess) return NEGF_ERR_CUDA;
   if (cl > 1) return negf_team::ls_launch(*p, smem, grid, cl, s);

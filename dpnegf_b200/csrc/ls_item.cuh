@@ -1,7 +1,7 @@
 // Batched Lopez-Sancho decimation for lead surface Green's functions and
 // self-energies (sm_100a, FP64 tensor cores).
 //
-// Persistent kernel: one CTA per work slot pulls (lead, energy) items from an
+// Persistent kernel: one CTA (or a cluster of CTAs) per work slot pulls (lead, energy) items from an
 // atomic queue and runs the whole decimation for that item in a private
 // scratch slot, with the same CTA tile GEMM and blocked Gauss-Jordan inverse
 // as the RGF sweep.  Follows _surface_green_numba_core

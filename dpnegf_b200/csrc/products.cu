@@ -150,7 +150,8 @@ int negf_gamma_sum_run(const NegfGammaSum* p, void* stream) {
   negf::cplx* Tst = reinterpret_cast<negf::cplx*>(p->scratch);
   negf::cplx* Gst = reinterpret_cast<negf::cplx*>(reinterpret_cast<char*>(p->scratch) + negf::gamma_stack_bytes(*p));
   const int smem = negf::GEMM_SMEM_BYTES;
-  if (!negf::allow_smem(negf::gamma_stack_kernel, smem) || !negf::allow_smem(negf::gamma_reduce_kernel, smem)) return NEGF_ERR_CUDA;
+  if (!negf::allow_smem(negf::gamma_stack_kernel, smem) || !negf::allow_smem(negf::gamma_reduce_kernel, smem))
+    return NEGF_ERR_CUDA;
   const int sms = negf::sm_count_or(148);
   const int grid1 = p->n_items < sms ? p->n_items : sms;
   negf::gamma_stack_kernel<<<grid1, negf::CTA_THREADS, smem, s>>>(*p, Tst, Gst);

@@ -1,6 +1,6 @@
 // Batched block-tridiagonal recursive Green's function (RGF) sweep, sm_100a.
 //
-// Persistent kernel: one CTA per work slot pulls (device, energy) items from
+// Persistent kernel: one CTA (or a cluster of CTAs) per work slot pulls (device, energy) items from
 // an atomic queue and runs the whole sweep for that item -- forward
 // left-connected inverses, backward retarded blocks, optional lesser blocks,
 // and the T(E) / per-orbital DOS reductions -- keeping its intermediates in a
